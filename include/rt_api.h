@@ -593,8 +593,9 @@ typedef struct RtTuning {
      * scene never reaches).  Lower values exist to exercise the error paths:
      * a render call whose wavefront has not drained after max_iterations
      * iterations returns RT_ERR_TIMEOUT; a traversal that needs more than
-     * stack_limit stack entries stops and the call returns RT_ERR_CAPACITY.
-     * rt_get_tuning reports the stack entries in force (7 per tree level). */
+     * stack_limit stack entries (the pending children of one node each) stops
+     * and the call returns RT_ERR_CAPACITY.  rt_get_tuning reports the stack
+     * entries in force (7 per tree level; a traversal needs at most one). */
     uint32_t max_iterations;       /* 0 or ≥ 1 */
     uint32_t stack_limit;          /* 0 or 1 .. the built-in capacity */
     /* Traversal stack entries kept in a per-thread ring (local memory) before the
@@ -602,10 +603,13 @@ typedef struct RtTuning {
      * results never depend on it; small rings make every traversal take the
      * spill path. */
     uint32_t stack_ring;
-    /* Node layout the traversal reads: RT_NODES_FULL (0, the default), the
-     * reference's 224-byte float layout (bvh.rs:25-32); RT_NODES_QUANTISED
-     * (1, when the scene's extents allow it), 128-byte nodes whose child boxes
-     * are 8-bit offsets rounded outward; RT_NODES_WIDE4 (2, scenes whose tree
+    /* Node layout the traversal reads (every layout keeps a node's children
+     * next to each other in octant order, with one header): RT_NODES_FULL (0,
+     * the default), the reference's float boxes (bvh.rs:25-32), 208 bytes per
+     * node — or, where it measured faster (trees far beyond the L1, caller-given
+     * rays), the quantised copy when the scene has one; RT_NODES_QUANTISED (1,
+     * when the scene's extents allow it), 80-byte nodes whose child boxes are
+     * 8-bit offsets rounded outward; RT_NODES_WIDE4 (2, scenes whose tree
      * was built on the device), 4-wide nodes of 112 bytes over the same binary
      * SAH tree — the reference's BVH width choice (bvh.rs:10-14).  The hits do
      * not depend on it. */

@@ -4,8 +4,8 @@ renderer runs a fixed rayon row loop, renderer.rs:684).
 The knobs are rt_set_tuning's: the path-pool capacity (how many paths are in
 flight; memory, and how long the final drain runs on a partial wavefront),
 the grids of the persistent traversal kernels and of the shading kernels, and
-the node layout the traversal reads: the reference's 224-byte 8-wide float
-nodes, their 8-bit quantised 128-byte copy, or 4-wide 112-byte nodes over the
+the node layout the traversal reads: 8-wide nodes with the reference's float
+boxes, their 8-bit quantised copy, or 4-wide nodes over the
 same binary tree — the BVH width the reference picks by target
 (bvh.rs:10-14).
 Every path draws its random numbers from (pixel, sample), so the knobs change

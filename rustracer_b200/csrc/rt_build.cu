@@ -1,5 +1,6 @@
 // rt_build.cu — the BVH built on the device: the binary SAH tree, then its
-// collapse to 8-wide nodes (full and quantised copies).
+// collapse to 8-wide nodes, and the packed node arrays the traversal reads
+// (full, quantised and 4-wide).
 //
 // The same tree as the host builder (SahBuilder in rt_host.cu), which restates
 // BvhTree::sah_partition (bvh.rs:290-323): at every node the centroid bounds,
@@ -536,18 +537,187 @@ __global__ void k_fix_leaf_refs(float4* nodes, int64_t n_nodes, const int32_t* _
         *ch = RT_LEAF_BIT | (t << 28) | (uint32_t)scans[(size_t)t * n + slot];
     }
 }
-// the quantised copy of every node, as encode_qnode does on the host: the
-// directed-rounding subtractions are the exact ones the host forms from
-// TwoSum; a node whose extent needs a step beyond 2^60 sets *fail
-__global__ void k_encode_qnodes(const float4* __restrict__ nodes, int64_t n_nodes, float4* qnodes, int* fail) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_nodes; i += (int64_t)gridDim.x * blockDim.x) {
-        const float4* N = nodes + (size_t)i * 14;
+// ── packed nodes: what the traversal reads (rt_trace.cu) ────────────────────
+// From a tree in the reference layout (preorder, child references): every
+// child gets a slot by octant (bit 0, 1, 2 of the slot: the upper side of x, y,
+// z), so a ray finds its children roughly front to back as slot XOR octant
+// without keeping distances; the inner children of a node become neighbours in
+// slot order, so a node index, a slot mask and a population count name a child
+// (a header instead of 8 references), and a visit's pending children are one
+// 8-byte stack entry.  The leaves of a node are neighbours too, in their own
+// copy of the triangle records (for other primitives only the reference), so a
+// leaf's triangle is found from the header without a reference in between; the
+// leaves' float boxes are a second array.
+//
+// Slots of one node's children, 4 bits per child: greedily the (child, free
+// slot) pair with the largest projection of the child's offset from the node
+// centre onto the slot's diagonal.
+template <int W>
+__device__ uint32_t octant_slots(const float* f, const uint32_t* ch) {
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int c = 0; c < W; c++) {
+        if (ch[c] == RT_EMPTY_REF) continue;
+        for (int a = 0; a < 3; a++) { lo[a] = fminf(lo[a], f[a * W + c]); hi[a] = fmaxf(hi[a], f[3 * W + a * W + c]); }
+    }
+    uint32_t slots = 0, free_slots = (1u << W) - 1u, todo = 0;
+    for (int c = 0; c < W; c++) todo |= (ch[c] != RT_EMPTY_REF ? 1u : 0u) << c;
+    while (todo) {
+        float best = -INFINITY;
+        int bc = __ffs(todo) - 1, bs = __ffs(free_slots) - 1;
+        for (int c = 0; c < W; c++) {
+            if (!((todo >> c) & 1u)) continue;
+            float off[3];
+            for (int a = 0; a < 3; a++) off[a] = (f[a * W + c] + f[3 * W + a * W + c]) - (lo[a] + hi[a]);
+            for (int q = 0; q < W; q++) {
+                if (!((free_slots >> q) & 1u)) continue;
+                float v = ((q & 1) ? off[0] : -off[0]) + ((q & 2) ? off[1] : -off[1]);
+                if (W == 8) v += (q & 4) ? off[2] : -off[2];
+                if (v > best) { best = v; bc = c; bs = q; }
+            }
+        }
+        slots |= (uint32_t)bs << (4 * bc);
+        todo &= ~(1u << bc);
+        free_slots &= ~(1u << bs);
+    }
+    return slots;
+}
+template <int W>
+__device__ void load_ref_node(const float4* __restrict__ in, int64_t i, float* f, uint32_t* ch) {
+    constexpr int F4 = W == 8 ? 14 : 7;
+    const float4* N = in + (size_t)i * F4;
+    for (int q = 0; q < F4; q++) {
+        float4 v = N[q];
+        f[q * 4] = v.x; f[q * 4 + 1] = v.y; f[q * 4 + 2] = v.z; f[q * 4 + 3] = v.w;
+    }
+    for (int c = 0; c < W; c++) ch[c] = __float_as_uint(f[6 * W + c]);
+}
+template <int W>
+__global__ void k_pack_slots(const float4* __restrict__ in, int32_t n, uint32_t* slots, uint64_t* cnt) {
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        float f[7 * W];
+        uint32_t ch[W];
+        load_ref_node<W>(in, i, f, ch);
+        slots[i] = octant_slots<W>(f, ch);
+        // inner children (low word) and leaves (high word) of the node
+        uint64_t k = 0;
+        for (int c = 0; c < W; c++)
+            if (ch[c] != RT_EMPTY_REF) k += (ch[c] & RT_LEAF_BIT) ? 1ull << 32 : 1ull;
+        cnt[i] = k;
+    }
+}
+// slots of a node's inner children
+template <int W>
+__device__ uint32_t inner_slots(const uint32_t* ch, uint32_t slots) {
+    uint32_t m = 0;
+    for (int c = 0; c < W; c++)
+        if (ch[c] != RT_EMPTY_REF && !(ch[c] & RT_LEAF_BIT)) m |= 1u << ((slots >> (4 * c)) & 7u);
+    return m;
+}
+// packed index of every node: 1 + the inner children of the nodes before its
+// parent + its rank among its siblings' slots (the root is 0)
+template <int W>
+__global__ void k_pack_index(const float4* __restrict__ in, int32_t n, const uint32_t* __restrict__ slots,
+                             const uint64_t* __restrict__ base, int32_t* index) {
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t* ch = reinterpret_cast<const uint32_t*>(in + (size_t)i * (W == 8 ? 14 : 7) + (W == 8 ? 12 : 6));
+        uint32_t r[W];
+        for (int c = 0; c < W; c++) r[c] = ch[c];
+        uint32_t im = inner_slots<W>(r, slots[i]);
+        for (int c = 0; c < W; c++) {
+            if (r[c] == RT_EMPTY_REF || (r[c] & RT_LEAF_BIT)) continue;
+            uint32_t q = (slots[i] >> (4 * c)) & 7u;
+            index[r[c]] = 1 + (int32_t)base[i] + __popc(im & ((1u << q) - 1u));
+        }
+        if (i == 0) index[0] = 0;
+    }
+}
+// a leaf reference (RT_LEAF_BIT, type, typed index) as the hit record it yields
+__device__ uint32_t leaf_hit_ref(const rtd::DevScene& S, uint32_t v) {
+    uint32_t type = (v >> 28) & 3u, idx = v & 0x07FFFFFFu;
+    float m = type == RT_PRIM_TRI ? S.tri[(size_t)idx * 3 + 2].z
+            : type == RT_PRIM_QUAD ? S.quad[(size_t)idx * 5 + 4].y
+            : type == RT_PRIM_SPHERE ? S.sphere[(size_t)idx * 2 + 1].y : S.cvx[(size_t)idx * 2].z;
+    return RT_HIT_MAKE(v, S.mat_code[__float_as_int(m)]);
+}
+// the record of a leaf: a triangle's (v0, e1, e2, canonical id) with its
+// reference in place of the material; of another primitive (-, -, (-, id, reference, -))
+__device__ void write_leaf(const rtd::DevScene& S, uint32_t v, float4* rec) {
+    uint32_t type = (v >> 28) & 3u, idx = v & 0x07FFFFFFu;
+    float ref = __uint_as_float(leaf_hit_ref(S, v));
+    if (type == RT_PRIM_TRI) {
+        const float4* g = S.tri + (size_t)idx * 3;
+        rec[0] = g[0];
+        rec[1] = g[1];
+        rec[2] = make_float4(g[2].x, g[2].y, ref, 0.f);
+    } else {
+        float gid = type == RT_PRIM_QUAD ? S.quad[(size_t)idx * 5 + 4].x
+                  : type == RT_PRIM_SPHERE ? S.sphere[(size_t)idx * 2 + 1].x : S.cvx[(size_t)idx * 2 + 1].x;
+        rec[0] = rec[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        rec[2] = make_float4(0.f, gid, ref, 0.f);
+    }
+}
+// the packed node's header; its leaves go to `LS` (rec null: they are written already)
+template <int W>
+__device__ float4 pack_head(const rtd::DevScene& S, const float* f, const uint32_t* ch, uint32_t slots, uint64_t base,
+                            rtd::LeafSet LS) {
+    uint32_t lm = 0, first = (uint32_t)(base >> 32);
+    for (int c = 0; c < W; c++)
+        if (ch[c] != RT_EMPTY_REF && (ch[c] & RT_LEAF_BIT)) lm |= 1u << ((slots >> (4 * c)) & 7u);
+    for (int c = 0; LS.rec && c < W; c++) {
+        if (ch[c] == RT_EMPTY_REF || !(ch[c] & RT_LEAF_BIT)) continue;
+        uint32_t q = (slots >> (4 * c)) & 7u;
+        size_t k = first + __popc(lm & ((1u << q) - 1u));
+        write_leaf(S, ch[c], const_cast<float4*>(LS.rec) + k * 3);
+        float4* r = const_cast<float4*>(LS.box) + k * 2;
+        r[0] = make_float4(f[c], f[W + c], f[2 * W + c], 0.f);
+        r[1] = make_float4(f[3 * W + c], f[4 * W + c], f[5 * W + c], 0.f);
+    }
+    return make_float4(__uint_as_float(1u + (uint32_t)base), __uint_as_float(inner_slots<W>(ch, slots) | lm << 8),
+                       __uint_as_float(first), 0.f);
+}
+// full nodes: RT_NODE_F4 (8-wide) or RT_NODE4_F4 (4-wide) float4
+template <int W>
+__global__ void k_pack_nodes(rtd::DevScene S, const float4* __restrict__ in, int32_t n,
+                             const uint32_t* __restrict__ slots, const uint64_t* __restrict__ base,
+                             const int32_t* __restrict__ index, float4* out, rtd::LeafSet LS) {
+    constexpr int F4 = W == 8 ? RT_NODE_F4 : RT_NODE4_F4, BOX4 = W == 8 ? 12 : 6;
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        float f[7 * W], g[6 * W];
+        uint32_t ch[W];
+        load_ref_node<W>(in, i, f, ch);
+        // slots without a child hold inverted boxes: their slab test fails
+        for (int a = 0; a < 3; a++)
+            for (int q = 0; q < W; q++) { g[a * W + q] = INFINITY; g[3 * W + a * W + q] = -INFINITY; }
+        for (int c = 0; c < W; c++) {
+            if (ch[c] == RT_EMPTY_REF) continue;
+            int q = (slots[i] >> (4 * c)) & 7u;
+            for (int a = 0; a < 3; a++) { g[a * W + q] = f[a * W + c]; g[3 * W + a * W + q] = f[3 * W + a * W + c]; }
+        }
+        float4* N = out + (size_t)index[i] * F4;
+        for (int q = 0; q < BOX4; q++) N[q] = make_float4(g[q * 4], g[q * 4 + 1], g[q * 4 + 2], g[q * 4 + 3]);
+        N[BOX4] = pack_head<W>(S, f, ch, slots[i], base[i], LS);
+    }
+}
+// Quantised nodes (RT_QNODE_F4 float4): the child boxes as 8-bit offsets from
+// the node's lower corner p in steps of s = 2^e per axis, rounded outward so
+// that the real planes p + q·s contain the exact child box (Ylitie et al. 2017
+// store child boxes this way; the rounding here is made conservative so the
+// hits stay the brute-force ones).  Words: 0: p.x, p.y, p.z, (e_x + 127) << 23 |
+// (e_y + 127) << 15 | (e_z + 127) << 7; 1-3: per axis the bytes q_lo, q_hi of
+// slots 0-7 in turn; 4: header.
+// A node whose extent needs a step beyond 2^60 sets *fail (steps are kept in
+// [2^-60, 2^60], so with |1/d| in [2^-60, 2^60] every s/d is a normal float).
+__global__ void k_pack_qnodes(rtd::DevScene S, const float4* __restrict__ nodes, int32_t n_nodes,
+                              const uint32_t* __restrict__ slots, const uint64_t* __restrict__ base,
+                              const int32_t* __restrict__ index, float4* qnodes, int* fail) {
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x) {
         float f[56];
-        for (int q = 0; q < 14; q++) { float4 v = N[q]; f[q * 4] = v.x; f[q * 4 + 1] = v.y; f[q * 4 + 2] = v.z; f[q * 4 + 3] = v.w; }
+        uint32_t ch[8];
+        load_ref_node<8>(nodes, i, f, ch);
         uint32_t valid = 0;
         float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
         for (int c = 0; c < 8; c++) {
-            if (__float_as_uint(f[48 + c]) == RT_EMPTY_REF) continue;
+            if (ch[c] == RT_EMPTY_REF) continue;
             valid |= 1u << c;
             for (int a = 0; a < 3; a++) { lo[a] = fminf(lo[a], f[a * 8 + c]); hi[a] = fmaxf(hi[a], f[24 + a * 8 + c]); }
         }
@@ -572,29 +742,26 @@ __global__ void k_encode_qnodes(const float4* __restrict__ nodes, int64_t n_node
             if (e[a] > 60) ok = false;
         }
         if (!ok) { atomicExch(fail, 1); continue; }
-        uint32_t w[3][4] = {};
+        uint32_t w[3][4];
         for (int a = 0; a < 3; a++) {
             float sa = ldexpf(1.0f, e[a]);
+            w[a][0] = w[a][1] = w[a][2] = w[a][3] = 0x00FF00FFu;   // slots without a child: lo 255, hi 0
             for (int c = 0; c < 8; c++) {
-                uint32_t ql = 255, qh = 0;
-                if ((valid >> c) & 1u) {
-                    float dl = __fsub_rd(f[a * 8 + c], lo[a]), dh = __fsub_ru(f[24 + a * 8 + c], lo[a]);
-                    ql = (uint32_t)fminf(fmaxf(floorf(dl / sa), 0.0f), 255.0f);
-                    qh = (uint32_t)fminf(fmaxf(ceilf(dh / sa), 0.0f), 255.0f);
-                }
-                w[a][c >> 2] |= ql << (8 * (c & 3));
-                w[a][2 + (c >> 2)] |= qh << (8 * (c & 3));
+                if (!((valid >> c) & 1u)) continue;
+                uint32_t q = (slots[i] >> (4 * c)) & 7u, sh = 16 * (q & 1u);
+                float dl = __fsub_rd(f[a * 8 + c], lo[a]), dh = __fsub_ru(f[24 + a * 8 + c], lo[a]);
+                uint32_t ql = (uint32_t)fminf(fmaxf(floorf(dl / sa), 0.0f), 255.0f);
+                uint32_t qh = (uint32_t)fminf(fmaxf(ceilf(dh / sa), 0.0f), 255.0f);
+                w[a][q >> 1] = (w[a][q >> 1] & ~(0xFFFFu << sh)) | (ql | qh << 8) << sh;
             }
         }
-        uint32_t meta = (uint32_t)(e[0] + 127) | (uint32_t)(e[1] + 127) << 8 | (uint32_t)(e[2] + 127) << 16 | valid << 24;
-        float4* Q = qnodes + (size_t)i * 8;
+        uint32_t meta = (uint32_t)(e[0] + 127) << 23 | (uint32_t)(e[1] + 127) << 15 | (uint32_t)(e[2] + 127) << 7;
+        float4* Q = qnodes + (size_t)index[i] * RT_QNODE_F4;
         Q[0] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(meta));
         for (int a = 0; a < 3; a++)
             Q[1 + a] = make_float4(__uint_as_float(w[a][0]), __uint_as_float(w[a][1]), __uint_as_float(w[a][2]),
                                    __uint_as_float(w[a][3]));
-        Q[4] = N[12];
-        Q[5] = N[13];
-        Q[6] = Q[7] = make_float4(0.f, 0.f, 0.f, 0.f);
+        Q[4] = pack_head<8>(S, f, ch, slots[i], base[i], rtd::LeafSet{nullptr, nullptr});
     }
 }
 
@@ -609,7 +776,6 @@ static cudaError_t collapse_wide(const int32_t* bl, const int32_t* br, const flo
     const int32_t nn = n - 1;
     int32_t *kids = nullptr, *nk = nullptr, *order = nullptr, *cnt = nullptr, *pos = nullptr;
     int32_t *S = nullptr, *L = nullptr, *P = nullptr, *LB = nullptr, *leaf_gid = nullptr, *flags = nullptr, *scans = nullptr;
-    int* fail = nullptr;
     void* tmp = nullptr;
     size_t tmp_bytes = 0;
     cudaError_t e = cudaSuccess;
@@ -631,7 +797,6 @@ static cudaError_t collapse_wide(const int32_t* bl, const int32_t* br, const flo
     ok(cudaMalloc(&S, (size_t)nn * 4)); ok(cudaMalloc(&L, (size_t)nn * 4));
     ok(cudaMalloc(&P, (size_t)nn * 4)); ok(cudaMalloc(&LB, (size_t)nn * 4));
     ok(cudaMalloc(&leaf_gid, (size_t)n * 4)); ok(cudaMalloc(&flags, (size_t)n * 16)); ok(cudaMalloc(&scans, (size_t)n * 16));
-    ok(cudaMalloc(&fail, 4));
     int grid = sms * 8;
     std::vector<int32_t> lvl_off;
     // the wide nodes of one width: each binary node's opening, the wide roots
@@ -681,7 +846,6 @@ static cudaError_t collapse_wide(const int32_t* bl, const int32_t* br, const flo
     if (e == cudaSuccess) W->n_nodes = plan(8, &W->max_depth);
     if (e == cudaSuccess) {
         ok(cudaMalloc(&W->nodes, (size_t)W->n_nodes * 14 * 16));
-        ok(cudaMalloc(&W->qnodes, (size_t)W->n_nodes * 8 * 16));
         ok(cudaMalloc(&W->export_ch, (size_t)W->n_nodes * 8 * 4));
     }
     if (e == cudaSuccess) {
@@ -692,14 +856,9 @@ static cudaError_t collapse_wide(const int32_t* bl, const int32_t* br, const flo
         for (int t = 0; t < 4; t++) scan(flags + (size_t)t * n, scans + (size_t)t * n, n);
         k_fix_leaf_refs<<<grid, 256, 0, st>>>(W->nodes, W->n_nodes, leaf_gid, n, W->type_end[0], W->type_end[1],
                                              W->type_end[2], scans);
-        ok(cudaMemsetAsync(fail, 0, 4, st));
-        k_encode_qnodes<<<grid, 128, 0, st>>>(W->nodes, W->n_nodes, W->qnodes, fail);
-        int hfail = 0;
         ok(cudaMemcpyAsync(W->leaf_gids_h, leaf_gid, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
-        ok(cudaMemcpyAsync(&hfail, fail, 4, cudaMemcpyDeviceToHost, st));
         ok(cudaStreamSynchronize(st));
         ok(cudaGetLastError());
-        if (e == cudaSuccess && hfail) { cudaFree(W->qnodes); W->qnodes = nullptr; }
     }
     // the 4-wide tree over the same binary tree (RT_NODES_WIDE4), its leaves
     // referring to the primitive records in the 8-wide leaf order
@@ -717,13 +876,67 @@ static cudaError_t collapse_wide(const int32_t* bl, const int32_t* br, const flo
             ok(cudaGetLastError());
         }
     }
-    void* all[] = {kids, nk, order, cnt, pos, S, L, P, LB, leaf_gid, flags, scans, fail, tmp};
+    void* all[] = {kids, nk, order, cnt, pos, S, L, P, LB, leaf_gid, flags, scans, tmp};
     for (void* p : all) if (p) cudaFree(p);
     if (e != cudaSuccess) {
-        void* outs[] = {W->nodes, W->qnodes, W->export_ch, W->nodes4};
+        void* outs[] = {W->nodes, W->export_ch, W->nodes4};
         for (void* p : outs) if (p) cudaFree(p);
-        W->nodes = W->qnodes = W->nodes4 = nullptr;
+        W->nodes = W->nodes4 = nullptr;
         W->export_ch = nullptr;
+    }
+    return e;
+}
+
+// Packs the n nodes of a reference-layout tree (width 8 or 4) with n_leaves
+// leaves: *out gets the packed nodes, *lout the leaves, and for width 8
+// *qout the quantised nodes (left null when an extent is beyond their range).  Needs the scene's primitive records and
+// material codes on the device.
+cudaError_t pack_nodes(const rtd::DevScene& S, const float4* in, int64_t n_nodes, int64_t n_leaves, int width,
+                       float4** out, rtd::LeafSet* lout, float4** qout, int sms, cudaStream_t st) {
+    const int32_t n = (int32_t)n_nodes;
+    uint32_t* slots = nullptr;
+    uint64_t *cnt = nullptr, *base = nullptr;
+    int32_t* index = nullptr;
+    int* fail = nullptr;
+    void* tmp = nullptr;
+    size_t need = 0;
+    cudaError_t e = cudaSuccess;
+    auto ok = [&](cudaError_t r) { if (e == cudaSuccess && r != cudaSuccess) e = r; return e == cudaSuccess; };
+    cub::DeviceScan::ExclusiveSum(nullptr, need, cnt, base, n, st);
+    ok(cudaMalloc(&slots, (size_t)n * 4)); ok(cudaMalloc(&cnt, (size_t)n * 8)); ok(cudaMalloc(&base, (size_t)n * 8));
+    ok(cudaMalloc((void**)&lout->rec, (size_t)n_leaves * 48)); ok(cudaMalloc((void**)&lout->box, (size_t)n_leaves * 32));
+    ok(cudaMalloc(&index, (size_t)n * 4)); ok(cudaMalloc(&fail, 4)); ok(cudaMalloc(&tmp, std::max<size_t>(need, 16)));
+    ok(cudaMalloc(out, (size_t)n * (width == 8 ? RT_NODE_F4 : RT_NODE4_F4) * 16));
+    if (qout) ok(cudaMalloc(qout, (size_t)n * RT_QNODE_F4 * 16));
+    if (e == cudaSuccess) {
+        const int g = std::max(1, std::min((n + 127) / 128, sms * 8));
+        ok(cudaMemsetAsync(fail, 0, 4, st));
+        if (width == 8) k_pack_slots<8><<<g, 128, 0, st>>>(in, n, slots, cnt);
+        else            k_pack_slots<4><<<g, 128, 0, st>>>(in, n, slots, cnt);
+        ok(cub::DeviceScan::ExclusiveSum(tmp, need, cnt, base, n, st));
+        if (width == 8) {
+            k_pack_index<8><<<g, 128, 0, st>>>(in, n, slots, base, index);
+            k_pack_nodes<8><<<g, 128, 0, st>>>(S, in, n, slots, base, index, *out, *lout);
+        } else {
+            k_pack_index<4><<<g, 128, 0, st>>>(in, n, slots, base, index);
+            k_pack_nodes<4><<<g, 128, 0, st>>>(S, in, n, slots, base, index, *out, *lout);
+        }
+        if (qout) k_pack_qnodes<<<g, 128, 0, st>>>(S, in, n, slots, base, index, *qout, fail);
+        int hfail = 0;
+        ok(cudaMemcpyAsync(&hfail, fail, 4, cudaMemcpyDeviceToHost, st));
+        ok(cudaStreamSynchronize(st));
+        ok(cudaGetLastError());
+        if (e == cudaSuccess && hfail && qout) { cudaFree(*qout); *qout = nullptr; }
+    }
+    void* all[] = {slots, cnt, base, index, fail, tmp};
+    for (void* p : all) if (p) cudaFree(p);
+    if (e != cudaSuccess) {
+        if (*out) cudaFree(*out);
+        if (lout->rec) cudaFree((void*)lout->rec);
+        if (lout->box) cudaFree((void*)lout->box);
+        *out = nullptr;
+        *lout = rtd::LeafSet{nullptr, nullptr};
+        if (qout && *qout) { cudaFree(*qout); *qout = nullptr; }
     }
     return e;
 }

@@ -2,11 +2,13 @@
 // traversal (rt_trace.cu) and shading (rt_shade.cu) kernels.
 //
 // HBM layout (all arrays 16-byte aligned, read through the read-only path):
-//   nodes  : 8-wide BVH nodes, 14 float4 = 224 B each, the reference layout of
-//            src/bvh.rs:25-32 (min[3][8], max[3][8], children[8]) so one node is
-//            fetched with 14 128-bit loads.  child ≥ 0 → inner node, child with
-//            the top bit set → leaf (type in bits 28-30, index in bits 0-27),
-//            0xFFFFFFFF → empty slot.
+//   nodes  : packed 8-wide BVH nodes, RT_NODE_F4 float4 each: the boxes of the
+//            reference layout (min[3][8], max[3][8], src/bvh.rs:25-32) and a
+//            header (first inner child, slots of the inner children and of the
+//            leaves, first leaf).  208 bytes: an odd number of 16-byte
+//            words, so the same word of 8 different nodes falls into 8 different
+//            bank groups of the L1 (224 bytes: 4).
+//   leaves : the leaves of the tree, those of a node in a row (LeafSet).
 //   tri    : 3 float4 per triangle, leaf order: (v0.xyz, e1.x) (e1.yz, e2.xy)
 //            (e2.z, gid, mat, has_normals).  e1 = v1 - v0 and e2 = v2 - v0 are
 //            the exact f32 differences the reference forms per hit
@@ -21,6 +23,9 @@
 #define RT_HD __host__ __device__ __forceinline__
 #define RT_D __device__ __forceinline__
 
+#define RT_NODE_F4    13
+#define RT_QNODE_F4   5
+#define RT_NODE4_F4   7
 #define RT_LEAF_BIT   0x80000000u
 #define RT_EMPTY_REF  0xFFFFFFFFu
 #define RT_MISS_REF   0xFFFFFFFFu
@@ -103,15 +108,24 @@ struct DevTexture {
     const int32_t* perm;         // 3 × 256 permutations
 };
 
+// The leaves of a packed tree, in the order its nodes' headers name them: per
+// leaf 3 float4 (v0.xyz, e1.x) (e1.yz, e2.xy) (e2.z, gid, reference, -) of a
+// triangle — of another primitive only gid and reference are set; the reference
+// is the hit record (RT_HIT_MAKE) — and 2 float4 with the leaf's float box.
+struct LeafSet { const float4 *rec, *box; };
+
 struct DevScene {
     const float4* nodes;
-    // the same nodes with 8-bit child boxes, 8 float4 each (see encode_qnode),
+    // the same nodes with 8-bit child boxes, RT_QNODE_F4 float4 each (k_pack_qnodes),
     // and which copy the traversal reads (RT_NODES_*)
     const float4* qnodes;
-    // 4-wide nodes of the same binary tree, 7 float4 each (lower x, y, z and
-    // upper x, y, z planes of 4 children, then their references)
+    LeafSet leaves;
+    // 4-wide nodes of the same binary tree, RT_NODE4_F4 float4 each (lower x, y, z
+    // and upper x, y, z planes of 4 children, header), and their leaves
     const float4* nodes4;
-    int node_format;
+    LeafSet leaves4;
+    int node_format;            // as set by rt_set_tuning (RT_NODES_FULL: the launch picks, see trace_format)
+    uint32_t n_nodes;           // 8-wide nodes
     const float4* tri;
     const float4* tri_n;
     const float4* quad;
@@ -137,9 +151,9 @@ struct DevScene {
     const float4* shape_par;
     int n_analytic;             // convex solids + shapes (the traversal compiles their tests in only if > 0)
     int trace_per_sm, shade_per_sm;   // launch tuning (host side; 0 = the built-in grids)
-    // traversal stack beyond the shared-memory ring: entry e ≥ RT_SHORT_STACK
-    // of global thread g at stack_spill[(e − RT_SHORT_STACK) · threads + g];
-    // stack_cap entries in all (7 per tree level; lowered only by rt_set_tuning)
+    // traversal stack beyond the ring: the words of entry e ≥ RT_SHORT_STACK of
+    // global thread g at stack_spill[(2(e − RT_SHORT_STACK) + 0, 1) · threads + g];
+    // at most stack_cap entries (lowered only by rt_set_tuning)
     uint32_t* stack_spill;
     int stack_cap;
     int stack_ring;             // shared-memory ring slots: RT_SHORT_STACK unless tuned (a power of two)

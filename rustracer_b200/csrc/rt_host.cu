@@ -173,82 +173,6 @@ static inline float area(const Box& b) {
 // Reference-layout node (bvh.rs:25-32).
 struct RefNode { float mn[3][8], mx[3][8]; int32_t ch[8]; };
 
-// ── quantised node (128 B): the child boxes as 8-bit offsets from the node's
-// lower corner p in steps of s = 2^e per axis, rounded outward so that the
-// real planes p + q·s contain the exact child box (Ylitie et al. 2017 store
-// child boxes this way; the rounding here is made conservative so the hits
-// stay the brute-force ones).  Layout (float4 words):
-//   0: p.x, p.y, p.z, (e_x + 127) | (e_y + 127) << 8 | (e_z + 127) << 16 | valid-slot mask << 24
-//   1-3: per axis x, y, z: q_lo of slots 0-3, 4-7, then q_hi of slots 0-3, 4-7 (a byte each)
-//   4-5: the 8 child references (as in the full node); 6-7: unused
-// x − y rounded down / up, exactly (TwoSum gives the rounding error of x − y)
-static inline float sub_dir(float x, float y, bool up) {
-    float a = x, b = -y;
-    float sm = a + b, bb = sm - a;
-    float err = (a - (sm - bb)) + (b - bb);
-    if (up) return err > 0.0f ? std::nextafter(sm, INFINITY) : sm;
-    return err < 0.0f ? std::nextafter(sm, -INFINITY) : sm;
-}
-// quantise one node; false when an extent needs a step beyond 2^60 (steps are
-// kept in [2^-60, 2^60], so with |1/d| in [2^-60, 2^60] every s/d is a normal float)
-static bool encode_qnode(const RefNode& r, const float4* full, float4* out) {
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    uint32_t valid = 0;
-    for (int c = 0; c < 8; c++) {
-        if (r.ch[c] == INT32_MIN) continue;
-        valid |= 1u << c;
-        for (int a = 0; a < 3; a++) { lo[a] = std::fmin(lo[a], r.mn[a][c]); hi[a] = std::fmax(hi[a], r.mx[a][c]); }
-    }
-    if (!valid) for (int a = 0; a < 3; a++) lo[a] = hi[a] = 0.0f;
-    int e[3];
-    bool flat[3];
-    int e_any = -60;
-    for (int a = 0; a < 3; a++) {
-        float ext = sub_dir(hi[a], lo[a], true);
-        flat[a] = !(ext > 0.0f);
-        if (flat[a]) continue;
-        int ex;
-        std::frexp(ext / 255.0f, &ex);              // ext/255 < 2^ex
-        while (ex > -60 && std::ldexp(255.0f, ex - 1) >= ext) ex--;
-        while (std::ldexp(255.0f, ex) < ext) ex++;
-        e[a] = std::max(ex, -60);                    // steps of at least 2^-60
-        e_any = std::max(e_any, e[a]);
-    }
-    for (int a = 0; a < 3; a++) {
-        if (flat[a]) e[a] = e_any;
-        if (e[a] > 60) return false;
-    }
-    uint8_t qlo[3][8], qhi[3][8];
-    for (int a = 0; a < 3; a++) {
-        float sa = std::ldexp(1.0f, e[a]);
-        for (int c = 0; c < 8; c++) {
-            if (!((valid >> c) & 1u)) { qlo[a][c] = 255; qhi[a][c] = 0; continue; }
-            float dl = sub_dir(r.mn[a][c], lo[a], false), dh = sub_dir(r.mx[a][c], lo[a], true);
-            float ql = std::floor(dl / sa), qh = std::ceil(dh / sa);
-            qlo[a][c] = (uint8_t)std::min(std::max(ql, 0.0f), 255.0f);
-            qhi[a][c] = (uint8_t)std::min(std::max(qh, 0.0f), 255.0f);
-        }
-    }
-    uint32_t meta = (uint32_t)(e[0] + 127) | (uint32_t)(e[1] + 127) << 8 | (uint32_t)(e[2] + 127) << 16 | valid << 24;
-    float fm;
-    memcpy(&fm, &meta, 4);
-    out[0] = make_float4(lo[0], lo[1], lo[2], fm);
-    for (int a = 0; a < 3; a++) {
-        uint32_t w[4] = {0, 0, 0, 0};
-        for (int c = 0; c < 8; c++) {
-            w[c >> 2] |= (uint32_t)qlo[a][c] << (8 * (c & 3));
-            w[2 + (c >> 2)] |= (uint32_t)qhi[a][c] << (8 * (c & 3));
-        }
-        float f[4];
-        memcpy(f, w, 16);
-        out[1 + a] = make_float4(f[0], f[1], f[2], f[3]);
-    }
-    out[4] = full[12];
-    out[5] = full[13];
-    out[6] = out[7] = make_float4(0.f, 0.f, 0.f, 0.f);
-    return true;
-}
-
 // ── binned-SAH 8-wide builder (cost model of bvh.rs:52-174) ─────────────────
 // In place on an index array: each partition reorders idx[lo, hi) by a stable
 // counting sort on bucket id, which is what the reference's stable
@@ -593,6 +517,7 @@ struct RtScene {
     // the device collapse it is made from the device nodes on first use
     mutable std::vector<RefNode> ref_nodes;
     mutable bool ref_ready = false;
+    const float4* d_ref_nodes = nullptr;    // the nodes in the reference layout (14 float4 each)
     const int32_t* d_export_ch = nullptr;   // device collapse: children in export form, 8 per node
     std::vector<int32_t> leaf_gids;
     bool empty = true;
@@ -748,7 +673,7 @@ static int ensure_ref_nodes(const RtScene* s) {
         std::vector<float4> nodes((size_t)s->n_nodes * 14);
         std::vector<int32_t> ch((size_t)s->n_nodes * 8);
         if (cudaSetDevice(s->device) != cudaSuccess ||
-            cudaMemcpy(nodes.data(), s->S.nodes, nodes.size() * 16, cudaMemcpyDeviceToHost) != cudaSuccess ||
+            cudaMemcpy(nodes.data(), s->d_ref_nodes, nodes.size() * 16, cudaMemcpyDeviceToHost) != cudaSuccess ||
             cudaMemcpy(ch.data(), s->d_export_ch, ch.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
             return RT_ERR_CUDA;
         s->ref_nodes.assign((size_t)s->n_nodes, RefNode{});
@@ -1033,6 +958,8 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
 
     // ── BVH ─────────────────────────────────────────────────────────────────
     std::vector<float4> gnodes;
+    const float4* d_ref4 = nullptr;      // the 4-wide tree in reference-like layout, and its node count
+    int64_t n_ref4 = 0;
     std::vector<float4> gtri, gtri_n, gquad, gsph, gtri_uv, gtri_tan;
     if (n > 0) {
         SahBuilder B(boxes);
@@ -1052,7 +979,7 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
             int brc = rth::gpu_build_binary(bx.data(), (int32_t)n, nullptr, nullptr, nullptr, nullptr, &root, s->sms,
                                             s->stream, &W);
             if (brc) return bail(fail(s, RT_ERR_CUDA, std::string("device BVH build: ") + cudaGetErrorString((cudaError_t)brc)));
-            void* owned_ptrs[] = {W.nodes, W.qnodes, W.export_ch, W.nodes4};
+            void* owned_ptrs[] = {W.nodes, W.export_ch, W.nodes4};
             for (void* p : owned_ptrs) if (p) s->owned.push_back(DevBuf{p, 0});
             B.max_depth = W.max_depth;
         } else {
@@ -1061,20 +988,21 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
         }
         s->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tb).count();
         s->max_depth = B.max_depth;
-        // traversal stack: a visit of a node at depth k leaves at most 7 entries
-        // per level above it, so 7 · (depth + 1) entries always suffice; the
-        // ones beyond the shared-memory ring spill to a column per persistent
+        // traversal stack: at most one 8-byte entry (a node's pending children)
+        // per tree level, so the capacity of 7 · (depth + 1) entries always
+        // suffices; entries beyond the ring spill to a column per persistent
         // traversal thread (grid ≤ SMs × RT_TRACE_MINB blocks)
         if (B.max_depth > 4096) return bail(fail(s, RT_ERR_CAPACITY, "BVH deeper than 4096 levels"));
         s->stack_cap_built = 7 * (B.max_depth + 1) + 8;
-        // the 4-wide tree is deeper; a visit there pushes at most 3 entries
+        // the 4-wide tree is deeper
         if (dev_wide) s->stack_cap_built = std::max(s->stack_cap_built, 3 * (W.max_depth4 + 1) + 8);
         s->S.stack_cap = s->stack_cap_built;
         s->S.stack_ring = RT_SHORT_STACK;
-        size_t spill_entries = (size_t)s->stack_cap_built;   // also room for a ring shrunk by rt_set_tuning
+        // also room for a ring shrunk by rt_set_tuning
+        size_t spill_words = 2 * (size_t)(std::max(B.max_depth, dev_wide ? W.max_depth4 : 0) + 2);
         size_t spill_threads = (size_t)s->sms * RT_TRACE_MINB * RT_TRACE_BLOCK;
         void* sp_buf = nullptr;
-        if (int rc = dalloc(s, &sp_buf, std::max<size_t>(spill_entries, 1) * spill_threads * sizeof(uint32_t)))
+        if (int rc = dalloc(s, &sp_buf, spill_words * spill_threads * sizeof(uint32_t)))
             return bail(rc);
         s->S.stack_spill = (uint32_t*)sp_buf;
         s->ref_nodes = std::move(B.nodes);
@@ -1228,25 +1156,13 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
         if ((rc = upload(s, gcvx.data(), gcvx.size(), &s->S.cvx))) return bail(rc);
         if ((rc = upload(s, wpl.data(), wpl.size(), &s->S.cvx_planes))) return bail(rc);
         if ((rc = upload(s, wsh.data(), wsh.size(), &s->S.cvx_shade))) return bail(rc);
+        s->S.node_format = RT_NODES_FULL;
         if (dev_wide) {
-            s->S.nodes = W.nodes;
-            s->S.qnodes = W.qnodes;
-            s->qnodes_ok = W.qnodes != nullptr;
-            s->S.nodes4 = W.nodes4;
-            s->wide4_ok = W.nodes4 != nullptr;
-            s->S.node_format = RT_NODES_FULL;
-        } else if ((rc = upload(s, gnodes.data(), gnodes.size(), &s->S.nodes))) {
+            s->d_ref_nodes = W.nodes;
+            d_ref4 = W.nodes4;
+            n_ref4 = W.n_nodes4;
+        } else if ((rc = upload(s, gnodes.data(), gnodes.size(), &s->d_ref_nodes))) {
             return bail(rc);
-        } else {   // the quantised copy of the nodes (rt_set_tuning node_format RT_NODES_QUANTISED)
-            std::vector<float4> qn((size_t)s->n_nodes * 8);
-            bool qok = true;
-            for (int64_t k = 0; k < s->n_nodes && qok; k++)
-                qok = encode_qnode(s->ref_nodes[k], &gnodes[(size_t)k * 14], &qn[(size_t)k * 8]);
-            if (qok) {
-                if ((rc = upload(s, qn.data(), qn.size(), &s->S.qnodes))) return bail(rc);
-                s->qnodes_ok = true;
-            }
-            s->S.node_format = RT_NODES_FULL;
         }
         if ((rc = upload(s, gtri.data(), gtri.size(), &s->S.tri))) return bail(rc);
         if ((rc = upload(s, gtri_n.data(), gtri_n.size(), &s->S.tri_n))) return bail(rc);
@@ -1369,6 +1285,21 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
                  : t == RT_MAT_PBR ? 4 : 1;
     }
     if ((rc = upload(s, codes.data(), codes.size(), &s->S.mat_code))) return bail(rc);
+    // the node arrays the traversal reads (their leaf references carry the class codes)
+    if (n > 0) {
+        float4 *pk = nullptr, *qk = nullptr, *pk4 = nullptr;
+        LeafSet lk{nullptr, nullptr}, lk4{nullptr, nullptr};
+        cudaError_t pe = rth::pack_nodes(s->S, s->d_ref_nodes, s->n_nodes, s->n_leaves, 8, &pk, &lk, &qk, s->sms, s->stream);
+        if (pe == cudaSuccess && d_ref4)
+            pe = rth::pack_nodes(s->S, d_ref4, n_ref4, s->n_leaves, 4, &pk4, &lk4, nullptr, s->sms, s->stream);
+        for (const float4* p : {(const float4*)pk, lk.rec, lk.box, (const float4*)qk, (const float4*)pk4, lk4.rec, lk4.box})
+            if (p) s->owned.push_back(DevBuf{(void*)p, 0});
+        if (pe != cudaSuccess) return bail(fail(s, RT_ERR_CUDA, std::string("packing the BVH nodes: ") + cudaGetErrorString(pe)));
+        s->S.nodes = pk; s->S.leaves = lk; s->S.qnodes = qk; s->S.nodes4 = pk4; s->S.leaves4 = lk4;
+        s->S.n_nodes = (uint32_t)s->n_nodes;
+        s->qnodes_ok = qk != nullptr;
+        s->wide4_ok = pk4 != nullptr;
+    }
     // shading classes the scene can produce: a miss always, a hit's class from
     // its material's code (launches of the other classes' kernels are skipped)
     s->S.class_mask = 1u << CLS_MISS;

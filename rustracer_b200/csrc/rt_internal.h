@@ -10,13 +10,9 @@
 
 #define RT_TRACE_BLOCK 128
 #define RT_TRACE_BLOCKS_PER_SM 8
-// resident blocks per SM of the persistent traversal kernels (their launch
-// bound and the most blocks per SM a traversal grid has): 6 blocks of 128
-// threads cap the kernels at 80 registers (measured faster than 5 blocks at
-// 96 registers and than 8 blocks at 64)
-#ifndef RT_TRACE_MINB
-#define RT_TRACE_MINB 6
-#endif
+// the most resident blocks per SM a persistent traversal kernel is compiled for
+// (the spill columns hold that many; see trace_minb in rt_trace.cu)
+#define RT_TRACE_MINB 8
 // the traversal stack's ring in local memory (1) or shared memory (0): a
 // shared ring reserves 8 KB per block of the SM's L1 / shared storage, and the
 // node fetches lose more to the smaller L1 than the stack gains (measured on
@@ -24,10 +20,11 @@
 #ifndef RT_STACK_LOCAL
 #define RT_STACK_LOCAL 1
 #endif
-// traversal stack: RT_SHORT_STACK entries per thread in a ring (local or
-// shared memory), deeper entries spilled to a per-thread column of global memory
-// sized from the tree depth at scene creation (7 per level: a visit pushes
-// at most 7 of its 8 children), so a traversal never runs out of stack
+// traversal stack: RT_SHORT_STACK entries (the pending children of one node, 8
+// bytes) per thread in a ring (local or shared memory), deeper entries spilled
+// to a per-thread column of global memory sized from the tree depth at scene
+// creation (a traversal holds at most one entry per level), so it never runs
+// out of stack
 #define RT_SHORT_STACK 16
 #define RT_SHADE_BLOCK 128
 #define RT_SHADE_BLOCKS_PER_SM 8
@@ -263,14 +260,13 @@ void launch_photon_gather_paths(const PhotonMapDev& map, const PendTargets& T, c
 void launch_accumulate(const float* scratch, uint32_t nsamp, uint32_t npix, float* acc, float* m2, uint32_t* cnt,
                        const uint8_t* conv, float clamp, uint32_t min_samples, float floor_, cudaStream_t st);
 // The 8-wide tree collapsed on the device from the binary tree (the host
-// collapse's greedy rule and preorder numbering): full and quantised node
-// arrays in device memory (the caller owns them), the leaf order, the node
+// collapse's greedy rule and preorder numbering): the nodes in the reference
+// layout in device memory (the caller owns them), the leaf order, the node
 // count and depth, and per node the children in the reference's export form
 // (≥ 0 node, −(leaf slot + 1), INT32_MIN empty) for rt_scene_bvh_export.
 struct WideOut {
     int64_t type_end[3];          // canonical ids below [0] are triangles, below [1] quads, below [2] spheres
     float4* nodes = nullptr;      // 14 float4 per node
-    float4* qnodes = nullptr;     // 8 float4 per node (null when an extent is beyond the quantised range)
     int32_t* export_ch = nullptr; // 8 per node
     int64_t n_nodes = 0;
     int32_t max_depth = 0;
@@ -283,6 +279,11 @@ struct WideOut {
 // or (wide != null) the device collapse into *wide
 int gpu_build_binary(const float* boxes_h, int32_t n, int32_t* idx_h, int32_t* bl_h, int32_t* br_h, float* bbox_h,
                      int32_t* root_h, int sms, cudaStream_t st, WideOut* wide = nullptr);
+// the packed nodes the traversal reads, from a reference-layout tree of n
+// nodes of `width` 8 or 4 and its leaves (see rt_build.cu); qout: the
+// quantised copy too (8-wide)
+cudaError_t pack_nodes(const rtd::DevScene& S, const float4* in, int64_t n, int64_t n_leaves, int width, float4** out,
+                       rtd::LeafSet* lout, float4** qout, int sms, cudaStream_t st);
 // guide mixture of every path in the diffuse queue (before its shading kernel)
 void launch_guide_infer(const rtd::DevScene& S, const PathState& A, const RenderLaunch& R, const uint32_t* queue,
                         const uint32_t* count, int sms, cudaStream_t st);

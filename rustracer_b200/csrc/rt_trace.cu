@@ -8,11 +8,13 @@
 // slab test :326-364): one ray per lane in persistent warps; lanes that finish
 // pull new rays as soon as enough of the warp is idle (lane refill), which keeps
 // SIMD lanes busy across very uneven ray costs.
-// Per node the thread issues 14 128-bit loads (224 B, the reference node),
-// tests all 8 child boxes, intersects hit leaves immediately (closest-t
-// first-wins, ties → smaller canonical id), then sorts the hit inner children
-// by entry distance with a 19-comparator network on packed (t | slot) keys and
-// continues with the nearest while the others go on a per-thread stack.
+// Per visited node the thread tests all 8 child boxes, intersects the hit leaves
+// at once (closest t, ties → smaller canonical id) and is left with a mask of
+// hit inner children.  The children of a node are neighbours in memory and sit
+// in slots by octant (pack_slots in rt_build.cu), so that mask and the index of
+// the first child are the whole to-do list of the visit (a "group", 8 bytes):
+// the next child is the slot nearest along the ray's octant, no distances are
+// kept or sorted, and a visit pushes at most one stack entry.
 #include <algorithm>
 
 #include <cub/block/block_scan.cuh>
@@ -24,69 +26,426 @@ using namespace rtd;
 
 namespace {
 
-struct Best { float t, b1, b2; uint32_t ref, gid, mat; };
+struct Best { float t, b1, b2; uint32_t ref, gid; };
 
 RT_D uint32_t f2u(float f) { return __float_as_uint(f); }
 
-// Leaf test for one reference; updates `best` and returns nothing.
+// convex_test (rt_device.cuh) of one ray by the whole warp: a brilliant has 97
+// planes and a step cut up to several hundred, one lane's serial loop over
+// them idles the other 31, and the loop's result — the entry is the largest
+// crossing of the planes facing the ray, the exit the smallest of the others,
+// the first plane of equal ones — does not depend on the order.  Lane l takes
+// planes l, l + 32, …; a −0 crossing counts as 0 in the comparison, as it does
+// there.  Every lane calls it with the same arguments; all get the result.
+RT_D uint32_t order_key(float t) {                  // monotone in t
+    uint32_t u = __float_as_uint(t + 0.0f);
+    return (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+RT_D bool warp_convex(const float4* pl, int n, float3 o, float3 d, float tmin, float tmax, float* t_out, int* plane) {
+    const uint32_t FULL = 0xFFFFFFFFu;
+    float te = tmin, tx = tmax;
+    int ie = -1, ix = -1;
+    bool out = false;
+    for (int i = threadIdx.x & 31u; i < n; i += 32) {
+        float4 q = __ldg(pl + i);
+        float nd = q.x * d.x + q.y * d.y + q.z * d.z;
+        float no = q.x * o.x + q.y * o.y + q.z * o.z;
+        float tf = (q.w - no) / nd;
+        if (fabsf(nd) < 1e-8f) out = out || no > q.w;
+        else if (nd < 0.0f) { if (tf > te) { te = tf; ie = i; } }
+        else if (tf < tx || (ix < 0 && tf == tx)) { tx = tf; ix = i; }
+    }
+    if (__any_sync(FULL, out)) return false;
+    // the entry: the largest key, then its first plane (none: t_min); the exit likewise
+    uint32_t ke = ie >= 0 ? order_key(te) : 0u, me = __reduce_max_sync(FULL, ke);
+    uint32_t pe = __reduce_min_sync(FULL, ie >= 0 && ke == me ? (uint32_t)ie : 0xFFFFFFFFu);
+    uint32_t kx = ix >= 0 ? order_key(tx) : 0xFFFFFFFFu, mx = __reduce_min_sync(FULL, kx);
+    uint32_t px = __reduce_min_sync(FULL, ix >= 0 && kx == mx ? (uint32_t)ix : 0xFFFFFFFFu);
+    const bool entry = pe != 0xFFFFFFFFu, exit = px != 0xFFFFFFFFu;
+    float t_enter = tmin, t_exit = tmax;
+    if (entry) t_enter = __shfl_sync(FULL, te, __ffs(__ballot_sync(FULL, ie == (int)pe)) - 1);
+    if (exit) t_exit = __shfl_sync(FULL, tx, __ffs(__ballot_sync(FULL, ix == (int)px)) - 1);
+    if (t_enter > t_exit) return false;
+    if (t_enter == t_exit && t_enter < tmax) return false;
+    if (entry) { *t_out = t_enter; *plane = (int)pe; return true; }
+    if (!exit || t_exit > tmax) return false;
+    *t_out = t_exit; *plane = (int)px;
+    return true;
+}
+
+// three-input min / max (sm_100)
+RT_D float fmax3f(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+RT_D float fmin3f(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// Per-ray slab constants.  Fast path (every |1/d| in [2^-60, 2^60], o/d finite,
+// t_min ≥ 0): the near and far planes of each axis are chosen once per ray from
+// the sign of the direction, and a plane distance is one FMA, b·inv + c with
+// c = −o·inv moved outward by 2^-22·|o·inv| (more than the rounding of o·inv):
+// a near distance is then at most the exact one and a far distance at least
+// the exact one, but for the 3 relative roundings of inv and the FMA, which
+// the exit widened by 2^-15 covers many times over.  So the culling is
+// conservative and any layout returns the brute-force answer.
+// General path (all other rays): both planes with min/max, a NaN slab (ray
+// lying in a face plane) spanning the whole line, and the exit widened.
+struct RayC {
+    float3 o, inv, cn, cf;
+    int nx, ny, nz;          // float4 offsets of the near-plane arrays in a full node
+    uint32_t ord;            // per slot bit 2, 1, 0 (bytes 0, 1, 2): the slots nearer along the ray
+    bool general;
+};
+constexpr float EXIT_WIDEN = 1.000031471252441f;      // 1 + 2^-15 + 2^-20
+
+RT_D bool inv_in_range(float x) {
+    float a = fabsf(x);
+    return a >= 8.673617379884035e-19f && a <= 1.152921504606846976e18f;   // 2^-60 .. 2^60
+}
+RT_D void axis_consts(float o, float inv, float* cn, float* cf) {
+    float oi = o * inv, m = fabsf(oi) * 2.384185791015625e-07f;           // 2^-22
+    *cn = __fsub_rd(-oi, m);
+    *cf = __fadd_ru(-oi, m);
+}
+
+RT_D RayC make_rayc(float3 o, float3 d, float tmin) {
+    RayC r;
+    r.o = o;
+    r.inv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+    axis_consts(o.x, r.inv.x, &r.cn.x, &r.cf.x);
+    axis_consts(o.y, r.inv.y, &r.cn.y, &r.cf.y);
+    axis_consts(o.z, r.inv.z, &r.cn.z, &r.cf.z);
+    r.general = !(tmin >= 0.0f) || !inv_in_range(r.inv.x) || !inv_in_range(r.inv.y) || !inv_in_range(r.inv.z) ||
+                !isfinite(r.cn.x + r.cn.y + r.cn.z);
+    bool sx = signbit(r.inv.x), sy = signbit(r.inv.y), sz = signbit(r.inv.z);
+    r.nx = sx ? 6 : 0;
+    r.ny = sy ? 8 : 2;
+    r.nz = sz ? 10 : 4;
+    // slot bit 0, 1, 2 set = the child lies on the upper side of x, y, z
+    r.ord = (sz ? 0xF0u : 0x0Fu) | (sy ? 0xCC00u : 0x3300u) | (sx ? 0xAA0000u : 0x550000u);
+    return r;
+}
+
+// Header of a node: the index of its first inner child, the slots of its inner
+// children (bits 0-7) and of its leaves (bits 8-15), and the index of its first
+// leaf record; the children of a node and its leaves follow one another in slot
+// order.
+struct NodeHead { uint32_t child, masks, leaf; };
+RT_D NodeHead load_head(const float4* p) {
+    uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+    return NodeHead{v.x, v.y, v.z};
+}
+
+__device__ __noinline__ uint32_t node_test_general(const float4* N, float3 o, float3 inv, float tmin, float tmax) {
+    uint32_t mask = 0;
+    float4 q[12];
+#pragma unroll
+    for (int i = 0; i < 12; i++) q[i] = __ldg(N + i);
+    const float* f = reinterpret_cast<const float*>(q);
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+        float dax = (f[0 + c] - o.x) * inv.x, dbx = (f[24 + c] - o.x) * inv.x;
+        float day = (f[8 + c] - o.y) * inv.y, dby = (f[32 + c] - o.y) * inv.y;
+        float daz = (f[16 + c] - o.z) * inv.z, dbz = (f[40 + c] - o.z) * inv.z;
+        float lx = fminf(dax, dbx), hx = fmaxf(dax, dbx);
+        float ly = fminf(day, dby), hy = fmaxf(day, dby);
+        float lz = fminf(daz, dbz), hz = fmaxf(daz, dbz);
+        if (isnan(dax) || isnan(dbx)) { lx = -INFINITY; hx = INFINITY; }
+        if (isnan(day) || isnan(dby)) { ly = -INFINITY; hy = INFINITY; }
+        if (isnan(daz) || isnan(dbz)) { lz = -INFINITY; hz = INFINITY; }
+        float t0 = fmaxf(fmaxf(fmaxf(tmin, lx), ly), lz);
+        float t1 = fminf(fminf(fminf(tmax, hx), hy), hz);
+        float t1w = t1 + fabsf(t1) * SLAB_WIDEN;
+        if (t0 <= t1w) mask |= 1u << c;
+    }
+    return mask;
+}
+
+// Slots of node `ni` whose box meets [tmin, tmax] along the ray (slots without
+// a child may be among them: the header's masks clear those).  The sign of
+// exit·widen − entry is shifted into the mask (a funnel shift per child)
+// instead of a compare and a select.
+RT_D uint32_t node_test(const DevScene& S, uint32_t ni, const RayC& R, float tmin, float tmax, NodeHead& h) {
+    const float4* N = S.nodes + (size_t)ni * RT_NODE_F4;
+    h = load_head(N + 12);
+    if (R.general) return node_test_general(N, R.o, R.inv, tmin, tmax);
+    float4 q[12];
+    q[0] = __ldg(N + R.nx); q[1] = __ldg(N + R.nx + 1);
+    q[2] = __ldg(N + R.ny); q[3] = __ldg(N + R.ny + 1);
+    q[4] = __ldg(N + R.nz); q[5] = __ldg(N + R.nz + 1);
+    q[6] = __ldg(N + 6 - R.nx); q[7] = __ldg(N + 7 - R.nx);
+    q[8] = __ldg(N + 10 - R.ny); q[9] = __ldg(N + 11 - R.ny);
+    q[10] = __ldg(N + 14 - R.nz); q[11] = __ldg(N + 15 - R.nz);
+    const float* f = reinterpret_cast<const float*>(q);
+    uint32_t miss = 0;
+#pragma unroll
+    for (int c = 7; c >= 0; c--) {
+        float nx = __fmaf_rn(f[0 + c], R.inv.x, R.cn.x), fx = __fmaf_rn(f[24 + c], R.inv.x, R.cf.x);
+        float ny = __fmaf_rn(f[8 + c], R.inv.y, R.cn.y), fy = __fmaf_rn(f[32 + c], R.inv.y, R.cf.y);
+        float nz = __fmaf_rn(f[16 + c], R.inv.z, R.cn.z), fz = __fmaf_rn(f[40 + c], R.inv.z, R.cf.z);
+        float t0 = fmax3f(fmaxf(tmin, nx), ny, nz);
+        float t1 = fmin3f(fminf(tmax, fx), fy, fz);
+        miss = __funnelshift_l(__float_as_uint(__fmaf_rn(t1, EXIT_WIDEN, -t0)), miss, 1);
+    }
+    return ~miss;
+}
+
+// ── quantised nodes (5 float4: see k_pack_qnodes in rt_build.cu) ─────────────
+// Child planes are the real numbers p + q·s (s = 2^e per axis), which contain
+// the exact child boxes.  Per ray and node S = s/d is exact, and with the ray's
+// slab constants (c moved outward by more than the rounding of o/d)
+// A = fma(p, 1/d, c), rounded down for the near planes and up for the far ones,
+// bounds (p − o)/d.  The byte q enters as the float 2^15 + q (one byte permute,
+// its unit 2^8 above the last mantissa bit), with 2^15·S taken off A rounded the
+// same way: that loses at most 2^-8 steps (2^23 + q would lose a whole one), so
+// q·S + A stays on the conservative side but for the last FMA's own rounding,
+// which the widened exit covers: the hits are the brute-force ones.  The kernel
+// is bound by issue here (73 % of the slots, ALU pipe 56 %), so the decode is
+// what counts; packed two-wide FMAs save 14 % of the instructions and lose it
+// again to the register pairs their constants need (spills; icosphere extend
+// 50.2 against 49.7 ms).
+RT_D float qbyte(uint32_t w, uint32_t sel) { return __uint_as_float(__byte_perm(w, 0x47000000u, sel)); }
+
+__device__ __noinline__ uint32_t qnode_test_general(const float4* N, float3 o, float3 inv, float tmin, float tmax);
+
+RT_D uint32_t qnode_test(const DevScene& S, uint32_t ni, const RayC& R, float tmin, float tmax, NodeHead& hd) {
+    const float4* N = S.qnodes + (size_t)ni * RT_QNODE_F4;
+    float4 h = __ldg(N);
+    uint4 bq[3] = {__ldg(reinterpret_cast<const uint4*>(N + 1)), __ldg(reinterpret_cast<const uint4*>(N + 2)),
+                   __ldg(reinterpret_cast<const uint4*>(N + 3))};
+    hd = load_head(N + 4);
+    if (R.general) return qnode_test_general(N, R.o, R.inv, tmin, tmax);
+    const uint32_t meta = __float_as_uint(h.w);
+    const float P[3] = {h.x, h.y, h.z}, I[3] = {R.inv.x, R.inv.y, R.inv.z};
+    const float CN[3] = {R.cn.x, R.cn.y, R.cn.z}, CF[3] = {R.cf.x, R.cf.y, R.cf.z};
+    float Sa[3], An[3], Af[3];
+    uint32_t sn[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        // exponent fields of x, y, z: bits 30-23, 22-15, 14-7
+        Sa[a] = __uint_as_float((meta << (8 * a)) & 0x7F800000u) * I[a];
+        An[a] = __fmaf_rd(-32768.0f, Sa[a], __fmaf_rd(P[a], I[a], CN[a]));
+        Af[a] = __fmaf_ru(-32768.0f, Sa[a], __fmaf_ru(P[a], I[a], CF[a]));
+        // the bytes of a child are (lower, upper): the near one is the lower for a positive direction
+        sn[a] = I[a] < 0.0f ? 0x7414u : 0x7404u;
+    }
+    uint32_t miss = 0;
+#pragma unroll
+    for (int c = 7; c >= 0; c--) {
+        float n[3], f[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const uint32_t w = c < 2 ? bq[a].x : c < 4 ? bq[a].y : c < 6 ? bq[a].z : bq[a].w;
+            const uint32_t sel = sn[a] + ((c & 1) ? 0x20u : 0u);
+            n[a] = __fmaf_rn(qbyte(w, sel), Sa[a], An[a]);
+            f[a] = __fmaf_rn(qbyte(w, sel ^ 0x10u), Sa[a], Af[a]);
+        }
+        float t0 = fmax3f(fmaxf(tmin, n[0]), n[1], n[2]);
+        float t1 = fmin3f(fminf(tmax, f[0]), f[1], f[2]);
+        miss = __funnelshift_l(__float_as_uint(__fmaf_rn(t1, EXIT_WIDEN, -t0)), miss, 1);
+    }
+    return ~miss;
+}
+
+// General rays (a zero, denormal or extreme direction component, or t_min < 0):
+// the planes decoded with outward rounding, then the general slab test.
+__device__ __noinline__ uint32_t qnode_test_general(const float4* N, float3 o, float3 inv, float tmin, float tmax) {
+    float4 h = __ldg(N);
+    const uint32_t meta = __float_as_uint(h.w);
+    const float P[3] = {h.x, h.y, h.z};
+    float lo[3][8], hi[3][8];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        uint4 b = __ldg(reinterpret_cast<const uint4*>(N + 1 + a));
+        float sa = __uint_as_float((meta << (8 * a)) & 0x7F800000u);
+        const uint32_t w[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            uint32_t v = w[c >> 1] >> (16 * (c & 1));
+            float ql = (float)(v & 0xFFu), qh = (float)((v >> 8) & 0xFFu);
+            lo[a][c] = __fmaf_rd(ql, sa, P[a]);
+            hi[a][c] = __fmaf_ru(qh, sa, P[a]);
+        }
+    }
+    uint32_t mask = 0;
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+        float dax = (lo[0][c] - o.x) * inv.x, dbx = (hi[0][c] - o.x) * inv.x;
+        float day = (lo[1][c] - o.y) * inv.y, dby = (hi[1][c] - o.y) * inv.y;
+        float daz = (lo[2][c] - o.z) * inv.z, dbz = (hi[2][c] - o.z) * inv.z;
+        float lx = fminf(dax, dbx), hx = fmaxf(dax, dbx);
+        float ly = fminf(day, dby), hy = fmaxf(day, dby);
+        float lz = fminf(daz, dbz), hz = fmaxf(daz, dbz);
+        if (isnan(dax) || isnan(dbx)) { lx = -INFINITY; hx = INFINITY; }
+        if (isnan(day) || isnan(dby)) { ly = -INFINITY; hy = INFINITY; }
+        if (isnan(daz) || isnan(dbz)) { lz = -INFINITY; hz = INFINITY; }
+        float t0 = fmaxf(fmaxf(fmaxf(tmin, lx), ly), lz);
+        float t1 = fminf(fminf(fminf(tmax, hx), hy), hz);
+        float t1w = t1 + fabsf(t1) * SLAB_WIDEN;
+        if (t0 <= t1w) mask |= 1u << c;
+    }
+    return mask;
+}
+
+// ── 4-wide nodes (7 float4: lower x, y, z, upper x, y, z, header) ───────────
+__device__ __noinline__ uint32_t node4_test_general(const float4* N, float3 o, float3 inv, float tmin, float tmax) {
+    float4 q[6];
+#pragma unroll
+    for (int i = 0; i < 6; i++) q[i] = __ldg(N + i);
+    const float* f = reinterpret_cast<const float*>(q);
+    uint32_t mask = 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        float dax = (f[0 + c] - o.x) * inv.x, dbx = (f[12 + c] - o.x) * inv.x;
+        float day = (f[4 + c] - o.y) * inv.y, dby = (f[16 + c] - o.y) * inv.y;
+        float daz = (f[8 + c] - o.z) * inv.z, dbz = (f[20 + c] - o.z) * inv.z;
+        float lx = fminf(dax, dbx), hx = fmaxf(dax, dbx);
+        float ly = fminf(day, dby), hy = fmaxf(day, dby);
+        float lz = fminf(daz, dbz), hz = fmaxf(daz, dbz);
+        if (isnan(dax) || isnan(dbx)) { lx = -INFINITY; hx = INFINITY; }
+        if (isnan(day) || isnan(dby)) { ly = -INFINITY; hy = INFINITY; }
+        if (isnan(daz) || isnan(dbz)) { lz = -INFINITY; hz = INFINITY; }
+        float t0 = fmaxf(fmaxf(fmaxf(tmin, lx), ly), lz);
+        float t1 = fminf(fminf(fminf(tmax, hx), hy), hz);
+        float t1w = t1 + fabsf(t1) * SLAB_WIDEN;
+        if (t0 <= t1w) mask |= 1u << c;
+    }
+    return mask;
+}
+
+RT_D uint32_t node4_test(const DevScene& S, uint32_t ni, const RayC& R, float tmin, float tmax, NodeHead& h) {
+    const float4* N = S.nodes4 + (size_t)ni * RT_NODE4_F4;
+    h = load_head(N + 6);
+    if (R.general) return node4_test_general(N, R.o, R.inv, tmin, tmax);
+    // the near planes of an axis are the lower ones for a positive direction
+    // (R.nx / 2 is 0 or 3, R.ny / 2 is 1 or 4, R.nz / 2 is 2 or 5)
+    float4 q[6];
+    q[0] = __ldg(N + R.nx / 2); q[1] = __ldg(N + R.ny / 2); q[2] = __ldg(N + R.nz / 2);
+    q[3] = __ldg(N + 3 - R.nx / 2); q[4] = __ldg(N + 5 - R.ny / 2); q[5] = __ldg(N + 7 - R.nz / 2);
+    const float* f = reinterpret_cast<const float*>(q);
+    uint32_t miss = 0;
+#pragma unroll
+    for (int c = 3; c >= 0; c--) {
+        float nx = __fmaf_rn(f[0 + c], R.inv.x, R.cn.x), fx = __fmaf_rn(f[12 + c], R.inv.x, R.cf.x);
+        float ny = __fmaf_rn(f[4 + c], R.inv.y, R.cn.y), fy = __fmaf_rn(f[16 + c], R.inv.y, R.cf.y);
+        float nz = __fmaf_rn(f[8 + c], R.inv.z, R.cn.z), fz = __fmaf_rn(f[20 + c], R.inv.z, R.cf.z);
+        float t0 = fmax3f(fmaxf(tmin, nx), ny, nz);
+        float t1 = fmin3f(fminf(tmax, fx), fy, fz);
+        miss = __funnelshift_l(__float_as_uint(__fmaf_rn(t1, EXIT_WIDEN, -t0)), miss, 1);
+    }
+    return ~miss;
+}
+
+// the node test of node `ni` in the layout NF (RT_NODES_FULL,
+// RT_NODES_QUANTISED, RT_NODES_WIDE4) and the leaves of its tree
+template <int NF>
+RT_D uint32_t node_test_any(const DevScene& S, uint32_t ni, const RayC& R, float tmin, float tmax, NodeHead& h) {
+    if constexpr (NF == RT_NODES_QUANTISED) return qnode_test(S, ni, R, tmin, tmax, h);
+    else if constexpr (NF == RT_NODES_WIDE4) return node4_test(S, ni, R, tmin, tmax, h);
+    else return node_test(S, ni, R, tmin, tmax, h);
+}
+template <int NF>
+RT_D const LeafSet& leaf_set(const DevScene& S) { return NF == RT_NODES_WIDE4 ? S.leaves4 : S.leaves; }
+
+// The node tests let every leaf through that this test accepts; a primitive's
+// hit counts only if the leaf's own float box is met too, in the arithmetic of the
+// reference-layout slab test: planes (b − o)·inv, the exit widened by 2^-15,
+// the bound by 2^-16 (rays with a zero direction component or t_min < 0: both
+// planes with min / max, a NaN slab spanning the whole line).  A triangle seen
+// edge-on at its box's corner can have a t far off its box, so without this the
+// layout and the looseness of the node tests would show in a hit (one in 10^8
+// camera rays of the icosphere).  Asked for accepted hits only: ahead of every
+// primitive test it cost 12 % of the closest-hit kernel (48.3 → 54.0 ms).
+__device__ __noinline__ bool leaf_box_general(float4 lo, float4 hi, float3 o, float3 inv, float tmin, float tmax) {
+    const float W = 1.000030517578125f;   // 1 + 2^-15
+    const float L[3] = {lo.x, lo.y, lo.z}, H[3] = {hi.x, hi.y, hi.z}, O[3] = {o.x, o.y, o.z}, I[3] = {inv.x, inv.y, inv.z};
+    const bool general = isinf(inv.x) || isinf(inv.y) || isinf(inv.z) || !(tmin >= 0.0f);
+    float t0 = tmin, t1 = general ? tmax : tmax + fabsf(tmax) * SLAB_WIDEN;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        if (general) {
+            float da = (L[a] - O[a]) * I[a], db = (H[a] - O[a]) * I[a];
+            float l = fminf(da, db), h = fmaxf(da, db);
+            if (isnan(da) || isnan(db)) { l = -INFINITY; h = INFINITY; }
+            t0 = fmaxf(t0, l);
+            t1 = fminf(t1, h);
+        } else {
+            bool neg = signbit(I[a]);
+            t0 = fmaxf(t0, ((neg ? H[a] : L[a]) - O[a]) * I[a]);
+            t1 = fminf(t1, ((neg ? L[a] : H[a]) - O[a]) * (I[a] * W));
+        }
+    }
+    return t0 <= (general ? t1 + fabsf(t1) * SLAB_WIDEN : t1);
+}
+RT_D bool leaf_box(const float4* box, const RayC& R, float tmin, float tmax) {
+    const float4 lo = __ldg(box), hi = __ldg(box + 1);
+    if (R.general) return leaf_box_general(lo, hi, R.o, R.inv, tmin, tmax);
+    const float W = 1.000030517578125f;
+    bool sx = R.inv.x < 0.0f, sy = R.inv.y < 0.0f, sz = R.inv.z < 0.0f;
+    float nx = ((sx ? hi.x : lo.x) - R.o.x) * R.inv.x, fx = ((sx ? lo.x : hi.x) - R.o.x) * (R.inv.x * W);
+    float ny = ((sy ? hi.y : lo.y) - R.o.y) * R.inv.y, fy = ((sy ? lo.y : hi.y) - R.o.y) * (R.inv.y * W);
+    float nz = ((sz ? hi.z : lo.z) - R.o.z) * R.inv.z, fz = ((sz ? lo.z : hi.z) - R.o.z) * (R.inv.z * W);
+    return fmax3f(fmaxf(tmin, nx), ny, nz) <= fmin3f(fminf(tmax + fabsf(tmax) * SLAB_WIDEN, fx), fy, fz);
+}
+
+// Test of leaf `k` (its index in the set's order); updates `best`.  Returns true
+// for a convex solid, which is not tested here.  The leaf's triangle is its own
+// record, found from the node's header alone: one round trip to the L2 where a
+// reference and then the primitive would be two (icosphere extend 52.9 ms that
+// way, 51.3 this way; gem 10.4 and 9.3).  The reference is a hit record already (RT_HIT_MAKE).
 // ANA: the scene has convex solids or shapes; without them the type-3 branch
 // is compiled out, so triangle scenes keep a lean traversal kernel.
 template <bool ANA>
-RT_D void leaf_closest(const DevScene& S, uint32_t ref, float3 o, float3 d, float tmin, Best& best) {
-    uint32_t type = (ref >> 28) & 7u, idx = ref & 0x0FFFFFFFu;
+RT_D bool leaf_closest(const DevScene& S, const LeafSet& LS, uint32_t k, const RayC& R, float3 d, float tmin, Best& best) {
+    const float3 o = R.o;
+    const float4* rec = LS.rec + (size_t)k * 3;
+    float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
+    const uint32_t ref = f2u(c.z), type = RT_HIT_TYPE(ref), idx = RT_HIT_INDEX(ref);
     float t, b1, b2;
-    uint32_t gid, mat;
+    uint32_t gid = f2u(c.y);
     bool h;
     if (type == RT_PRIM_TRI) {
-        const float4* g = S.tri + (size_t)idx * 3;
-        float4 a = __ldg(g), b = __ldg(g + 1), c = __ldg(g + 2);
         h = tri_test(a, b, c, o, d, tmin, best.t, &t, &b1, &b2);
-        gid = f2u(c.y);
-        mat = f2u(c.z);
     } else if (type == RT_PRIM_QUAD) {
         const float4* g = S.quad + (size_t)idx * 5;
         float4 gg[4] = {__ldg(g), __ldg(g + 1), __ldg(g + 2), __ldg(g + 3)};
         h = quad_test(gg, o, d, tmin, best.t, &t, &b1, &b2);
-        float4 gm = h ? __ldg(g + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-        gid = f2u(gm.x);
-        mat = f2u(gm.y);
     } else if (type == RT_PRIM_SPHERE) {
         const float4* g = S.sphere + (size_t)idx * 2;
         h = sphere_test(__ldg(g), o, d, tmin, best.t, &t);
         b1 = b2 = 0.0f;
-        float4 gm = h ? __ldg(g + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
-        gid = f2u(gm.x);
-        mat = f2u(gm.y);
     } else if (!ANA) {
-        return;
-    } else {                                        // convex solid or shape; b1 carries the plane / surface
+        return false;
+    } else {                                        // a shape; b1 carries the surface
         float4 c0 = __ldg(S.cvx + (size_t)idx * 2);
         int pi = -1, cnt = __float_as_int(c0.y);
-        if (cnt > 0) {
-            h = convex_test(S.cvx_planes + __float_as_int(c0.x), cnt, o, d, tmin, best.t, &t, &pi);
-        } else {
-            const float4* P = S.shape_par + __float_as_int(c0.x);
-            float3 lo, ld;
-            shape_local(P, o, d, &lo, &ld);
-            h = shape_test(-1 - cnt, P, lo, ld, tmin, best.t, &t, &pi);
-        }
+        if (cnt > 0) return true;                   // a convex solid: left to the warp (warp_convex)
+        const float4* P = S.shape_par + __float_as_int(c0.x);
+        float3 lo, ld;
+        shape_local(P, o, d, &lo, &ld);
+        h = shape_test(-1 - cnt, P, lo, ld, tmin, best.t, &t, &pi);
         b1 = __int_as_float(pi);
         b2 = 0.0f;
-        gid = h ? f2u(__ldg(S.cvx + (size_t)idx * 2 + 1).x) : 0u;
-        mat = f2u(c0.z);
     }
-    if (h && (t < best.t || best.ref == RT_MISS_REF || gid < best.gid)) {
-        best.t = t; best.b1 = b1; best.b2 = b2; best.ref = ref; best.gid = gid; best.mat = mat;
+    if (h && (t < best.t || best.ref == RT_MISS_REF || gid < best.gid) &&
+        leaf_box(LS.box + (size_t)k * 2, R, tmin, best.t)) {
+        best.t = t; best.b1 = b1; best.b2 = b2; best.ref = ref; best.gid = gid;
     }
+    return false;
 }
 
 template <bool ANA>
-RT_D bool leaf_any(const DevScene& S, uint32_t ref, float3 o, float3 d, float tmin, float tmax) {
-    uint32_t type = (ref >> 28) & 7u, idx = ref & 0x0FFFFFFFu;
+RT_D bool leaf_any_test(const DevScene& S, const float4* rec, float3 o, float3 d, float tmin, float tmax, bool* convex) {
+    float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
+    const uint32_t ref = f2u(c.z), type = RT_HIT_TYPE(ref), idx = RT_HIT_INDEX(ref);
     float t, b1, b2;
     if (type == RT_PRIM_TRI) {
-        const float4* g = S.tri + (size_t)idx * 3;
-        return tri_test(__ldg(g), __ldg(g + 1), __ldg(g + 2), o, d, tmin, tmax, &t, &b1, &b2);
+        return tri_test(a, b, c, o, d, tmin, tmax, &t, &b1, &b2);
     } else if (type == RT_PRIM_QUAD) {
         const float4* g = S.quad + (size_t)idx * 5;
         float4 gg[4] = {__ldg(g), __ldg(g + 1), __ldg(g + 2), __ldg(g + 3)};
@@ -96,520 +455,201 @@ RT_D bool leaf_any(const DevScene& S, uint32_t ref, float3 o, float3 d, float tm
     if (!ANA) return false;
     float4 c0 = __ldg(S.cvx + (size_t)idx * 2);
     int pi, cnt = __float_as_int(c0.y);
-    if (cnt > 0) return convex_test(S.cvx_planes + __float_as_int(c0.x), cnt, o, d, tmin, tmax, &t, &pi);
+    if (cnt > 0) { *convex = true; return false; }  // left to the warp (warp_convex)
     const float4* P = S.shape_par + __float_as_int(c0.x);
     float3 lo, ld;
     shape_local(P, o, d, &lo, &ld);
     return shape_test(-1 - cnt, P, lo, ld, tmin, tmax, &t, &pi);
 }
-
-#ifndef RT_MNMX3
-#define RT_MNMX3 1
-#endif
-#ifndef RT_EMPTY_INVERTED
-#define RT_EMPTY_INVERTED 1
-#endif
-// three-input min / max (sm_100)
-RT_D float fmax3f(float a, float b, float c) {
-#if RT_MNMX3
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-#else
-    return fmaxf(fmaxf(a, b), c);
-#endif
+template <bool ANA>
+RT_D bool leaf_any(const DevScene& S, const LeafSet& LS, uint32_t k, const RayC& R, float3 d, float tmin, float tmax,
+                   bool* convex) {
+    return leaf_any_test<ANA>(S, LS.rec + (size_t)k * 3, R.o, d, tmin, tmax, convex) &&
+           leaf_box(LS.box + (size_t)k * 2, R, tmin, tmax);
 }
-RT_D float fmin3f(float a, float b, float c) {
-#if RT_MNMX3
-    float d;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-#else
-    return fminf(fminf(a, b), c);
-#endif
-}
-
-#define CAS(a, b) { uint32_t lo_ = min(k[a], k[b]); uint32_t hi_ = max(k[a], k[b]); k[a] = lo_; k[b] = hi_; }
-
-// Per-ray slab constants.  Fast path (every direction component non-zero and
-// t_min ≥ 0): the near and far planes of each axis are chosen once per ray from
-// the sign of the direction, so a child costs 6 FSUB + 6 FMUL + 6 FMNMX.  The
-// far-plane reciprocal is widened by 2^-15, which after the two roundings of
-// (b − o)·inv still exceeds the exact exit distance by ≥ 2^-16 relative — the
-// culling stays conservative, so any layout returns the brute-force answer.
-// General path (a zero or denormal component, or t_min < 0): both planes with
-// min/max, a NaN slab (ray lying in a face plane) spanning the whole line, and
-// the exit widened explicitly.
-struct RayC {
-    float3 o, inv, invf;
-    int nx, ny, nz;          // float4 offsets of the near-plane arrays in a node
-    bool general;
-    bool qgeneral;           // quantised nodes: also any |1/d| outside [2^-60, 2^60]
-};
-
-RT_D bool inv_in_range(float x) {
-    float a = fabsf(x);
-    return a >= 8.673617379884035e-19f && a <= 1.152921504606846976e18f;   // 2^-60 .. 2^60
-}
-
-RT_D RayC make_rayc(float3 o, float3 d, float tmin) {
-    RayC r;
-    r.o = o;
-    r.inv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
-    const float W = 1.000030517578125f;   // 1 + 2^-15
-    r.invf = mk(r.inv.x * W, r.inv.y * W, r.inv.z * W);
-    r.general = isinf(r.inv.x) || isinf(r.inv.y) || isinf(r.inv.z) || !(tmin >= 0.0f);
-    r.qgeneral = r.general || !inv_in_range(r.inv.x) || !inv_in_range(r.inv.y) || !inv_in_range(r.inv.z);
-    r.nx = signbit(r.inv.x) ? 6 : 0;
-    r.ny = signbit(r.inv.y) ? 8 : 2;
-    r.nz = signbit(r.inv.z) ? 10 : 4;
-    return r;
-}
-
-__device__ __noinline__ uint32_t node_test_general(const DevScene& S, uint32_t ni, const RayC& R, float tmin,
-                                                   float tmax, float* tn);
-
-// Slab test of the 8 children of node `ni` against [tmin, tmax]; returns the
-// hit mask and the entry distances.
-RT_D uint32_t node_test(const DevScene& S, uint32_t ni, const RayC& R, float tmin, float tmax, float tn[8],
-                        uint32_t ch[8]) {
-    const float4* N = S.nodes + (size_t)ni * 14;
-    uint32_t mask = 0;
-    float4 c0 = __ldg(N + 12), c1 = __ldg(N + 13);
-    const uint32_t cc[8] = {__float_as_uint(c0.x), __float_as_uint(c0.y), __float_as_uint(c0.z), __float_as_uint(c0.w),
-                            __float_as_uint(c1.x), __float_as_uint(c1.y), __float_as_uint(c1.z), __float_as_uint(c1.w)};
-#pragma unroll
-    for (int c = 0; c < 8; c++) ch[c] = cc[c];
-    if (!R.general) {
-        float4 q[12];
-        q[0] = __ldg(N + R.nx); q[1] = __ldg(N + R.nx + 1);
-        q[2] = __ldg(N + R.ny); q[3] = __ldg(N + R.ny + 1);
-        q[4] = __ldg(N + R.nz); q[5] = __ldg(N + R.nz + 1);
-        q[6] = __ldg(N + 6 - R.nx); q[7] = __ldg(N + 7 - R.nx);
-        q[8] = __ldg(N + 10 - R.ny); q[9] = __ldg(N + 11 - R.ny);
-        q[10] = __ldg(N + 14 - R.nz); q[11] = __ldg(N + 15 - R.nz);
-        const float* f = reinterpret_cast<const float*>(q);
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            float nx = (f[0 + c] - R.o.x) * R.inv.x, fx = (f[24 + c] - R.o.x) * R.invf.x;
-            float ny = (f[8 + c] - R.o.y) * R.inv.y, fy = (f[32 + c] - R.o.y) * R.invf.y;
-            float nz = (f[16 + c] - R.o.z) * R.inv.z, fz = (f[40 + c] - R.o.z) * R.invf.z;
-            float t0 = fmax3f(fmaxf(tmin, nx), ny, nz);
-            float t1 = fmin3f(fminf(tmax, fx), fy, fz);
-            tn[c] = t0;
-#if RT_EMPTY_INVERTED
-            if (t0 <= t1) mask |= 1u << c;     // empty slots hold inverted boxes
-#else
-            if (t0 <= t1 && ch[c] != RT_EMPTY_REF) mask |= 1u << c;
-#endif
-        }
-        return mask;
-    }
-    float tg[8];
-    mask = node_test_general(S, ni, R, tmin, tmax, tg);
-#pragma unroll
-    for (int c = 0; c < 8; c++) tn[c] = tg[c];
-    return mask;
-}
-
-__device__ __noinline__ uint32_t node_test_general(const DevScene& S, uint32_t ni, const RayC& R, float tmin,
-                                                   float tmax, float* tn) {
-    const float4* N = S.nodes + (size_t)ni * 14;
-    uint32_t mask = 0;
-    float4 q[14];
-#pragma unroll
-    for (int i = 0; i < 14; i++) q[i] = __ldg(N + i);
-    const float* f = reinterpret_cast<const float*>(q);
-    const uint32_t* ch = reinterpret_cast<const uint32_t*>(f + 48);
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-        float dax = (f[0 + c] - R.o.x) * R.inv.x, dbx = (f[24 + c] - R.o.x) * R.inv.x;
-        float day = (f[8 + c] - R.o.y) * R.inv.y, dby = (f[32 + c] - R.o.y) * R.inv.y;
-        float daz = (f[16 + c] - R.o.z) * R.inv.z, dbz = (f[40 + c] - R.o.z) * R.inv.z;
-        float lx = fminf(dax, dbx), hx = fmaxf(dax, dbx);
-        float ly = fminf(day, dby), hy = fmaxf(day, dby);
-        float lz = fminf(daz, dbz), hz = fmaxf(daz, dbz);
-        if (isnan(dax) || isnan(dbx)) { lx = -INFINITY; hx = INFINITY; }
-        if (isnan(day) || isnan(dby)) { ly = -INFINITY; hy = INFINITY; }
-        if (isnan(daz) || isnan(dbz)) { lz = -INFINITY; hz = INFINITY; }
-        float t0 = fmaxf(fmaxf(fmaxf(tmin, lx), ly), lz);
-        float t1 = fminf(fminf(fminf(tmax, hx), hy), hz);
-        float t1w = t1 + fabsf(t1) * SLAB_WIDEN;
-        tn[c] = t0;
-        if (t0 <= t1w && ch[c] != RT_EMPTY_REF) mask |= 1u << c;
-    }
-    return mask;
-}
-
-// ── quantised nodes (8 float4: see encode_qnode in rt_host.cu) ───────────────
-// Child planes are the real numbers p + q·s (s = 2^e per axis), which contain
-// the exact child boxes.  Per ray and node, S = s/d is exact and
-// A = (p − o)/d is computed with two roundings; q·S + A then differs from the
-// exact plane distance by at most u·(255|S| + 3.02|A|) (u = 2^-24), so with
-// err = 2^-20·(|A| + 256|S|) the near distance fma(2^23 + q, S, A − err − 2^23·S)
-// rounded down is below it and the far one rounded up is above it: the
-// culling stays conservative and the hits are the brute-force ones.  The
-// byte q enters as the float 2^23 + q (one byte permute), its 2^23 folded
-// into the per-node constant.
-RT_D float qbyte(uint32_t w, uint32_t sel) { return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)); }
-
-__device__ __noinline__ uint32_t qnode_test_general(const DevScene& S, uint32_t ni, const RayC& R, float tmin,
-                                                    float tmax, float* tn);
-
-RT_D uint32_t qnode_test(const DevScene& S, uint32_t ni, const RayC& R, float tmin, float tmax, float tn[8],
-                         uint32_t ch[8]) {
-    const float4* N = S.qnodes + (size_t)ni * 8;
-    float4 h = __ldg(N);
-    uint4 bq[3] = {__ldg(reinterpret_cast<const uint4*>(N + 1)), __ldg(reinterpret_cast<const uint4*>(N + 2)),
-                   __ldg(reinterpret_cast<const uint4*>(N + 3))};
-    float4 c0 = __ldg(N + 4), c1 = __ldg(N + 5);
-    const uint32_t cc[8] = {__float_as_uint(c0.x), __float_as_uint(c0.y), __float_as_uint(c0.z), __float_as_uint(c0.w),
-                            __float_as_uint(c1.x), __float_as_uint(c1.y), __float_as_uint(c1.z), __float_as_uint(c1.w)};
-#pragma unroll
-    for (int c = 0; c < 8; c++) ch[c] = cc[c];
-    const uint32_t meta = __float_as_uint(h.w);
-    if (R.qgeneral) {
-        float tg[8];
-        uint32_t m = qnode_test_general(S, ni, R, tmin, tmax, tg);
-#pragma unroll
-        for (int c = 0; c < 8; c++) tn[c] = tg[c];
-        return m;
-    }
-    const float M = 8388608.0f;                        // 2^23
-    const float P[3] = {h.x, h.y, h.z}, O[3] = {R.o.x, R.o.y, R.o.z}, I[3] = {R.inv.x, R.inv.y, R.inv.z};
-    float Sa[3], An[3], Af[3];
-    uint32_t wn[3][2], wf[3][2];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        float sa = __uint_as_float(((meta >> (8 * a)) & 0xFFu) << 23);   // 2^e
-        float Sx = sa * I[a];
-        float Ax = (P[a] - O[a]) * I[a];
-        float err = __fmul_ru(__fmaf_ru(fabsf(Sx), 256.0f, fabsf(Ax)), 9.5367431640625e-07f);   // × 2^-20
-        An[a] = __fmaf_rd(-M, Sx, __fsub_rd(Ax, err));
-        Af[a] = __fmaf_ru(-M, Sx, __fadd_ru(Ax, err));
-        Sa[a] = Sx;
-        // the near planes are the lower ones for a positive direction
-        bool neg = I[a] < 0.0f;
-        wn[a][0] = neg ? bq[a].z : bq[a].x; wn[a][1] = neg ? bq[a].w : bq[a].y;
-        wf[a][0] = neg ? bq[a].x : bq[a].z; wf[a][1] = neg ? bq[a].y : bq[a].w;
-    }
-    uint32_t mask = 0;
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-        const uint32_t sel = 0x7540u + (uint32_t)(c & 3);
-        float nx = __fmaf_rd(qbyte(wn[0][c >> 2], sel), Sa[0], An[0]);
-        float ny = __fmaf_rd(qbyte(wn[1][c >> 2], sel), Sa[1], An[1]);
-        float nz = __fmaf_rd(qbyte(wn[2][c >> 2], sel), Sa[2], An[2]);
-        float fx = __fmaf_ru(qbyte(wf[0][c >> 2], sel), Sa[0], Af[0]);
-        float fy = __fmaf_ru(qbyte(wf[1][c >> 2], sel), Sa[1], Af[1]);
-        float fz = __fmaf_ru(qbyte(wf[2][c >> 2], sel), Sa[2], Af[2]);
-        float t0 = fmax3f(fmaxf(tmin, nx), ny, nz);
-        float t1 = fmin3f(fminf(tmax, fx), fy, fz);
-        tn[c] = t0;
-        if (t0 <= t1) mask |= 1u << c;
-    }
-    return mask & (meta >> 24);
-}
-
-// General rays (a zero, denormal or extreme direction component, or t_min < 0):
-// the planes decoded with outward rounding, then the general slab test.
-__device__ __noinline__ uint32_t qnode_test_general(const DevScene& S, uint32_t ni, const RayC& R, float tmin,
-                                                    float tmax, float* tn) {
-    const float4* N = S.qnodes + (size_t)ni * 8;
-    float4 h = __ldg(N);
-    const uint32_t meta = __float_as_uint(h.w);
-    const float P[3] = {h.x, h.y, h.z};
-    float lo[3][8], hi[3][8];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        uint4 b = __ldg(reinterpret_cast<const uint4*>(N + 1 + a));
-        float sa = __uint_as_float(((meta >> (8 * a)) & 0xFFu) << 23);
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            uint32_t wl = c < 4 ? b.x : b.y, wh = c < 4 ? b.z : b.w;
-            float ql = (float)((wl >> (8 * (c & 3))) & 0xFFu), qh = (float)((wh >> (8 * (c & 3))) & 0xFFu);
-            lo[a][c] = __fmaf_rd(ql, sa, P[a]);
-            hi[a][c] = __fmaf_ru(qh, sa, P[a]);
-        }
-    }
-    uint32_t mask = 0;
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-        float dax = (lo[0][c] - R.o.x) * R.inv.x, dbx = (hi[0][c] - R.o.x) * R.inv.x;
-        float day = (lo[1][c] - R.o.y) * R.inv.y, dby = (hi[1][c] - R.o.y) * R.inv.y;
-        float daz = (lo[2][c] - R.o.z) * R.inv.z, dbz = (hi[2][c] - R.o.z) * R.inv.z;
-        float lx = fminf(dax, dbx), hx = fmaxf(dax, dbx);
-        float ly = fminf(day, dby), hy = fmaxf(day, dby);
-        float lz = fminf(daz, dbz), hz = fmaxf(daz, dbz);
-        if (isnan(dax) || isnan(dbx)) { lx = -INFINITY; hx = INFINITY; }
-        if (isnan(day) || isnan(dby)) { ly = -INFINITY; hy = INFINITY; }
-        if (isnan(daz) || isnan(dbz)) { lz = -INFINITY; hz = INFINITY; }
-        float t0 = fmaxf(fmaxf(fmaxf(tmin, lx), ly), lz);
-        float t1 = fminf(fminf(fminf(tmax, hx), hy), hz);
-        float t1w = t1 + fabsf(t1) * SLAB_WIDEN;
-        tn[c] = t0;
-        if (t0 <= t1w) mask |= 1u << c;
-    }
-    return mask & (meta >> 24);
-}
-
-// ── 4-wide nodes (7 float4: lower x, y, z, upper x, y, z, references) ──────
-__device__ __noinline__ uint32_t node4_test_general(const DevScene& S, uint32_t ni, const RayC& R, float tmin,
-                                                    float tmax, float* tn);
-
-RT_D uint32_t node4_test(const DevScene& S, uint32_t ni, const RayC& R, float tmin, float tmax, float tn[8],
-                         uint32_t ch[8]) {
-    const float4* N = S.nodes4 + (size_t)ni * 7;
-    float4 c0 = __ldg(N + 6);
-    ch[0] = __float_as_uint(c0.x); ch[1] = __float_as_uint(c0.y);
-    ch[2] = __float_as_uint(c0.z); ch[3] = __float_as_uint(c0.w);
-    if (!R.general) {
-        // the near planes of an axis are the lower ones for a positive direction
-        // (R.nx / 2 is 0 or 3, R.ny / 2 is 1 or 4, R.nz / 2 is 2 or 5)
-        float4 q[6];
-        q[0] = __ldg(N + R.nx / 2); q[1] = __ldg(N + R.ny / 2); q[2] = __ldg(N + R.nz / 2);
-        q[3] = __ldg(N + 3 - R.nx / 2); q[4] = __ldg(N + 5 - R.ny / 2); q[5] = __ldg(N + 7 - R.nz / 2);
-        const float* f = reinterpret_cast<const float*>(q);
-        uint32_t mask = 0;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            float nx = (f[0 + c] - R.o.x) * R.inv.x, fx = (f[12 + c] - R.o.x) * R.invf.x;
-            float ny = (f[4 + c] - R.o.y) * R.inv.y, fy = (f[16 + c] - R.o.y) * R.invf.y;
-            float nz = (f[8 + c] - R.o.z) * R.inv.z, fz = (f[20 + c] - R.o.z) * R.invf.z;
-            float t0 = fmax3f(fmaxf(tmin, nx), ny, nz);
-            float t1 = fmin3f(fminf(tmax, fx), fy, fz);
-            tn[c] = t0;
-            if (t0 <= t1) mask |= 1u << c;     // empty slots hold inverted boxes
-        }
-        return mask;
-    }
-    float tg[4];
-    uint32_t mask = node4_test_general(S, ni, R, tmin, tmax, tg);
-#pragma unroll
-    for (int c = 0; c < 4; c++) tn[c] = tg[c];
-    return mask;
-}
-
-__device__ __noinline__ uint32_t node4_test_general(const DevScene& S, uint32_t ni, const RayC& R, float tmin,
-                                                    float tmax, float* tn) {
-    const float4* N = S.nodes4 + (size_t)ni * 7;
-    float4 q[7];
-#pragma unroll
-    for (int i = 0; i < 7; i++) q[i] = __ldg(N + i);
-    const float* f = reinterpret_cast<const float*>(q);
-    const uint32_t* ch = reinterpret_cast<const uint32_t*>(f + 24);
-    uint32_t mask = 0;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        float dax = (f[0 + c] - R.o.x) * R.inv.x, dbx = (f[12 + c] - R.o.x) * R.inv.x;
-        float day = (f[4 + c] - R.o.y) * R.inv.y, dby = (f[16 + c] - R.o.y) * R.inv.y;
-        float daz = (f[8 + c] - R.o.z) * R.inv.z, dbz = (f[20 + c] - R.o.z) * R.inv.z;
-        float lx = fminf(dax, dbx), hx = fmaxf(dax, dbx);
-        float ly = fminf(day, dby), hy = fmaxf(day, dby);
-        float lz = fminf(daz, dbz), hz = fmaxf(daz, dbz);
-        if (isnan(dax) || isnan(dbx)) { lx = -INFINITY; hx = INFINITY; }
-        if (isnan(day) || isnan(dby)) { ly = -INFINITY; hy = INFINITY; }
-        if (isnan(daz) || isnan(dbz)) { lz = -INFINITY; hz = INFINITY; }
-        float t0 = fmaxf(fmaxf(fmaxf(tmin, lx), ly), lz);
-        float t1 = fminf(fminf(fminf(tmax, hx), hy), hz);
-        float t1w = t1 + fabsf(t1) * SLAB_WIDEN;
-        tn[c] = t0;
-        if (t0 <= t1w && ch[c] != RT_EMPTY_REF) mask |= 1u << c;
-    }
-    return mask;
-}
-
-// the node test and the child-reference words of node `ni` in the layout NF
-// (RT_NODES_FULL, RT_NODES_QUANTISED, RT_NODES_WIDE4), and its width
-template <int NF>
-RT_D uint32_t node_test_any(const DevScene& S, uint32_t ni, const RayC& R, float tmin, float tmax, float tn[8],
-                            uint32_t ch[8]) {
-    if constexpr (NF == RT_NODES_QUANTISED) return qnode_test(S, ni, R, tmin, tmax, tn, ch);
-    else if constexpr (NF == RT_NODES_WIDE4) return node4_test(S, ni, R, tmin, tmax, tn, ch);
-    else return node_test(S, ni, R, tmin, tmax, tn, ch);
-}
-template <int NF>
-RT_D const uint32_t* node_refs(const DevScene& S, uint32_t ni) {
-    if constexpr (NF == RT_NODES_QUANTISED) return reinterpret_cast<const uint32_t*>(S.qnodes + (size_t)ni * 8 + 4);
-    else if constexpr (NF == RT_NODES_WIDE4) return reinterpret_cast<const uint32_t*>(S.nodes4 + (size_t)ni * 7 + 6);
-    else return reinterpret_cast<const uint32_t*>(S.nodes + (size_t)ni * 14 + 12);
-}
-template <int NF> constexpr int node_width() { return NF == RT_NODES_WIDE4 ? 4 : 8; }
 
 }  // namespace
 
 namespace rtk {
 
-// Per-thread traversal stack (the reference keeps 128 entries inline and
-// spills to a heap Vec, bvh.rs:229-239).  The newest RT_SHORT_STACK entries
-// live in a ring: the thread's local memory (RT_STACK_LOCAL, the default) or
-// shared memory laid out [entry][thread], so the lanes of a warp hit 32
-// different banks whatever their depths.  Entry e ≥ RT_SHORT_STACK of a
-// deeper stack waits in the thread's global column spill[(e − RT_SHORT_STACK)
-// · stride] (rt_set_tuning can shrink the ring to fewer slots, so the tests
-// run every traversal through the spill path).  A push beyond the ring first
-// moves the ring slot's old entry to its column, a pop that uncovers a
-// spilled entry brings it back.  `cap` (7 per tree level, sized at scene
-// creation) is never reached by a traversal of the scene's own tree; a lower
-// cap from rt_set_tuning makes the traversal stop with RT_ERR_CAPACITY.
+// Per-thread traversal stack of groups (the reference keeps 128 nodes inline
+// and spills to a heap Vec, bvh.rs:229-239).  A group is the pending children
+// of one node: x = its first child's index, y = their slots (bits 0-7) and the
+// slots of all its inner children (bits 8-15).  The newest RT_SHORT_STACK
+// groups live in a ring: the thread's local memory (RT_STACK_LOCAL, the
+// default) or shared memory laid out [entry][thread].  Entry e ≥ RT_SHORT_STACK
+// of a deeper stack waits in the thread's global column, two words at
+// spill[2(e − RT_SHORT_STACK) · stride] (rt_set_tuning can shrink the ring to
+// fewer slots, so the tests run every traversal through the spill path).  A
+// push beyond the ring first moves the ring slot's old entry to its column, a
+// pop that uncovers a spilled entry brings it back.  A traversal holds at most
+// one group per tree level, so `cap` (sized at scene creation) is never
+// reached in the scene's own tree; a lower cap from rt_set_tuning makes the
+// traversal stop with RT_ERR_CAPACITY.
 constexpr int RING_STRIDE = RT_STACK_LOCAL ? 1 : RT_TRACE_BLOCK;
 struct TStack {
-    uint32_t* ring;          // ring slot k at ring[k · RING_STRIDE] (shared: &ring[threadIdx.x])
-    uint32_t* spill;         // &S.stack_spill[global thread]; entry e at spill[(e − ring_n) · stride]
-    uint32_t stride;
-    int sp, cap;
-    int ring_n;              // ring slots in use: RT_SHORT_STACK, or fewer (a power of two) when tuned
+    uint2* ring;             // ring slot k at ring[k · RING_STRIDE] (shared: &ring[threadIdx.x])
+    int sp;
 
-    RT_D bool room(int k) const { return sp + k <= cap; }
-    RT_D void push(uint32_t v) {
-        int slot = sp & (ring_n - 1);
-        if (sp >= ring_n) spill[(size_t)(sp - ring_n) * stride] = ring[slot * RING_STRIDE];
+    // S.stack_cap entries at most; S.stack_ring ring slots in use (a power of two).
+    // The spill column's address is formed only when an entry goes there.
+    RT_D bool room(const DevScene& S) const { return sp < S.stack_cap; }
+    RT_D uint32_t* column(const DevScene& S, int e) const {
+        return S.stack_spill + (size_t)(2 * e) * (gridDim.x * blockDim.x) + blockIdx.x * blockDim.x + threadIdx.x;
+    }
+    RT_D void push(const DevScene& S, uint2 v) {
+        int slot = sp & (S.stack_ring - 1);
+        if (sp >= S.stack_ring) {
+            uint2 old = ring[slot * RING_STRIDE];
+            uint32_t* e = column(S, sp - S.stack_ring);
+            e[0] = old.x; e[gridDim.x * blockDim.x] = old.y;
+        }
         ring[slot * RING_STRIDE] = v;
         sp++;
     }
-    RT_D uint32_t pop() {
+    RT_D uint2 pop(const DevScene& S) {
         sp--;
-        int slot = sp & (ring_n - 1);
-        uint32_t v = ring[slot * RING_STRIDE];
-        if (sp >= ring_n) ring[slot * RING_STRIDE] = spill[(size_t)(sp - ring_n) * stride];
+        int slot = sp & (S.stack_ring - 1);
+        uint2 v = ring[slot * RING_STRIDE];
+        if (sp >= S.stack_ring) {
+            const uint32_t* e = column(S, sp - S.stack_ring);
+            ring[slot * RING_STRIDE] = make_uint2(e[0], e[gridDim.x * blockDim.x]);
+        }
         return v;
     }
 };
 
-RT_D TStack make_stack(const DevScene& S, uint32_t* ring_base) {
-    TStack st;
-    st.ring = RT_STACK_LOCAL ? ring_base : ring_base + threadIdx.x;
-    st.stride = gridDim.x * blockDim.x;
-    st.spill = S.stack_spill + blockIdx.x * blockDim.x + threadIdx.x;
-    st.sp = 0;
-    st.cap = S.stack_cap;
-    st.ring_n = S.stack_ring;
-    return st;
-}
+// the root as a group of one
+RT_D uint2 root_group() { return make_uint2(0u, 0x0101u); }
 
-// One node visit of the closest-hit traversal: tests the 8 children of `node`,
-// intersects hit leaves in slot order, then continues with the nearest hit inner
-// child (sorted by a 19-comparator network on packed (t | slot) keys) and pushes
-// the others far → near.  Returns false when the traversal is finished.
-template <bool ANA, int NF>
-RT_D bool closest_step(const DevScene& S, const RayC& R, float3 d, float tmin, Best& best,
-                       uint32_t& node, TStack& stk, bool& ok) {
-    constexpr int WN = node_width<NF>();
-    float tn[8];
-    uint32_t ch[8];
-    // the closest hit so far bounds the boxes; widened like every exit distance
-    float cwin = best.t + fabsf(best.t) * SLAB_WIDEN;
-    uint32_t mask = node_test_any<NF>(S, node, R, tmin, R.general ? best.t : cwin, tn, ch);
-    uint32_t leaves = 0;
-#pragma unroll
-    for (int c = 0; c < WN; c++) leaves |= ((ch[c] & RT_LEAF_BIT) ? 1u : 0u) << c;
-    leaves &= mask;
-    if (leaves) {
-        const uint32_t* refs = node_refs<NF>(S, node);
-#pragma unroll 1
-        while (leaves) {
-            int c = __ffs(leaves) - 1;
-            leaves &= leaves - 1;
-            leaf_closest<ANA>(S, __ldg(refs + c), R.o, d, tmin, best);
+// Takes the group's pending slot that is nearest along the ray's octant (the
+// smallest slot XOR octant, bit by bit) and returns its node.
+RT_D uint32_t take_nearest(uint2& g, uint32_t ord) {
+    uint32_t m = g.y & 0xFFu, t;
+    t = m & ord;         if (t) m = t;
+    t = m & (ord >> 8);  if (t) m = t;
+    t = m & (ord >> 16); if (t) m = t;
+    g.y ^= m;
+    return g.x + __popc((g.y >> 8) & (m - 1u));
+}
+// Takes the group's first pending slot.
+RT_D uint32_t take_first(uint2& g) {
+    uint32_t m = g.y & (0u - g.y);
+    g.y ^= m;
+    return g.x + __popc((g.y >> 8) & (m - 1u));
+}
+// After a visit: go on with its hit inner children, else with the rest of the
+// current group, else with the newest one on the stack; false when none is left.
+RT_D bool next_group(const DevScene& S, uint2& g, uint32_t child, uint32_t inner, uint32_t masks, TStack& stk,
+                     bool& ok) {
+    if (inner) {
+        if (g.y & 0xFFu) {
+            if (!stk.room(S)) { ok = false; return false; }
+            stk.push(S, g);
         }
-    }
-    float cw = best.t + fabsf(best.t) * SLAB_WIDEN;
-    uint32_t k[8];
-    int n = 0;
-#pragma unroll
-    for (int c = 0; c < WN; c++) {
-        bool inner = ((mask >> c) & 1u) && !(ch[c] & RT_LEAF_BIT) && tn[c] <= cw;
-        k[c] = inner ? ((__float_as_uint(fmaxf(tn[c], 0.0f)) & ~7u) | (uint32_t)c) : 0xFFFFFFFFu;
-        n += inner ? 1 : 0;
-    }
-    if (n == 0) {
-        if (stk.sp == 0) return false;
-        node = stk.pop();
+        g = make_uint2(child, inner | (masks & 0xFFu) << 8);
         return true;
     }
-    if (n == 2) {
-        // two inner children: continue with the nearer, push the farther
-        uint32_t a = 0xFFFFFFFFu, b = 0xFFFFFFFFu;
-#pragma unroll
-        for (int c = 0; c < WN; c++) {
-            if (k[c] == 0xFFFFFFFFu) continue;
-            if (a == 0xFFFFFFFFu) a = k[c]; else b = k[c];
-        }
-        uint32_t lo = min(a, b), hi = max(a, b);
-        if (!stk.room(1)) { ok = false; return false; }
-        const uint32_t* refs = node_refs<NF>(S, node);
-        stk.push(__ldg(refs + (hi & 7u)));
-        node = __ldg(refs + (lo & 7u));
-    } else if (n > 2) {
-        if constexpr (WN == 4) {
-            CAS(0, 1) CAS(2, 3)
-            CAS(0, 2) CAS(1, 3)
-            CAS(1, 2)
-        } else {
-            CAS(0, 1) CAS(2, 3) CAS(4, 5) CAS(6, 7)
-            CAS(0, 2) CAS(1, 3) CAS(4, 6) CAS(5, 7)
-            CAS(1, 2) CAS(5, 6) CAS(0, 4) CAS(3, 7)
-            CAS(1, 5) CAS(2, 6)
-            CAS(1, 4) CAS(3, 6)
-            CAS(2, 4) CAS(3, 5)
-            CAS(3, 4)
-        }
-        if (!stk.room(n - 1)) { ok = false; return false; }
-        const uint32_t* refs = node_refs<NF>(S, node);
-#pragma unroll
-        for (int j = WN - 1; j >= 1; j--)
-            if (j < n) stk.push(__ldg(refs + (k[j] & 7u)));
-        node = __ldg(refs + (k[0] & 7u));
-    } else {
-        uint32_t c = 0;
-#pragma unroll
-        for (int j = 0; j < WN; j++) if (k[j] != 0xFFFFFFFFu) c = j;
-        node = ch[c];
-    }
+    if (g.y & 0xFFu) return true;
+    if (stk.sp == 0) return false;
+    g = stk.pop(S);
     return true;
 }
 
-// One node visit of the any-hit traversal (bvh.rs:487-530).  Returns false when
-// finished; *hit is set when a primitive was hit.
+// Convex solids a lane met in a visit: the node's first leaf and which of its leaves.
+struct Convex { uint32_t first, which; };
+__device__ __forceinline__ float3 shfl3(float3 v, int l) {
+    return mk(__shfl_sync(0xFFFFFFFFu, v.x, l), __shfl_sync(0xFFFFFFFFu, v.y, l), __shfl_sync(0xFFFFFFFFu, v.z, l));
+}
+
+// One node visit of the closest-hit traversal: tests the children of the
+// group's nearest node and intersects its hit leaves (convex solids are only
+// noted in `cv`); `inner` gets the hit inner children.
 template <bool ANA, int NF>
-RT_D bool any_step(const DevScene& S, const RayC& R, float3 d, float tmin, float tmax,
-                   uint32_t& node, TStack& stk, bool& hit, bool& ok) {
-    constexpr int WN = node_width<NF>();
-    float tn[8];
-    uint32_t ch[8];
-    float tw = tmax + fabsf(tmax) * SLAB_WIDEN;
-    uint32_t mask = node_test_any<NF>(S, node, R, tmin, R.general ? tmax : tw, tn, ch);
-    uint32_t inner = 0, leaves = 0;
-#pragma unroll
-    for (int c = 0; c < WN; c++) {
-        bool lf = ch[c] & RT_LEAF_BIT;
-        leaves |= (lf ? 1u : 0u) << c;
-        inner |= (lf ? 0u : 1u) << c;
-    }
-    leaves &= mask;
-    inner &= mask;
+RT_D void closest_visit(const DevScene& S, const RayC& R, float3 d, float tmin, Best& best, uint2& grp, NodeHead& h,
+                        uint32_t& inner, Convex& cv) {
+    const uint32_t node = take_nearest(grp, R.ord);
+    const uint32_t hits = node_test_any<NF>(S, node, R, tmin, best.t, h);
+    uint32_t leaves = hits & (h.masks >> 8);
+    inner = hits & h.masks & 0xFFu;
+    cv.which = 0u;
     if (leaves) {
-        const uint32_t* refs = node_refs<NF>(S, node);
+        const uint32_t all = h.masks >> 8;
+        cv.first = h.leaf;
 #pragma unroll 1
         while (leaves) {
-            int c = __ffs(leaves) - 1;
+            uint32_t k = __popc(all & ((leaves & (0u - leaves)) - 1u));
             leaves &= leaves - 1;
-            if (leaf_any<ANA>(S, __ldg(refs + c), R.o, d, tmin, tmax)) { hit = true; return false; }
+            if (leaf_closest<ANA>(S, leaf_set<NF>(S), h.leaf + k, R, d, tmin, best) && ANA) cv.which |= 1u << k;
         }
     }
-    if (inner == 0) {
-        if (stk.sp == 0) return false;
-        node = stk.pop();
-        return true;
+}
+// The noted convex solids of the warp's lanes, one test at a time (every lane calls it).
+RT_D void closest_convex(const DevScene& S, const LeafSet& LS, const RayC& R, float3 d, float tmin, Best& best, Convex& cv) {
+    uint32_t need = __ballot_sync(0xFFFFFFFFu, cv.which != 0u);
+    while (need) {
+        const int L = __ffs(need) - 1;
+        const uint32_t leaf = __shfl_sync(0xFFFFFFFFu, cv.first + __ffs(cv.which) - 1u, L);
+        if ((threadIdx.x & 31u) == L) cv.which &= cv.which - 1u;
+        const uint32_t ref = f2u(__ldg(LS.rec + (size_t)leaf * 3 + 2).z);
+        const float4* rec = S.cvx + (size_t)RT_HIT_INDEX(ref) * 2;
+        float4 c0 = __ldg(rec);
+        float t;
+        int pi;
+        bool h = warp_convex(S.cvx_planes + __float_as_int(c0.x), __float_as_int(c0.y), shfl3(R.o, L), shfl3(d, L),
+                             __shfl_sync(0xFFFFFFFFu, tmin, L), __shfl_sync(0xFFFFFFFFu, best.t, L), &t, &pi);
+        if (h && (threadIdx.x & 31u) == L) {
+            uint32_t gid = f2u(__ldg(rec + 1).x);
+            if ((t < best.t || best.ref == RT_MISS_REF || gid < best.gid) && leaf_box(LS.box + (size_t)leaf * 2, R, tmin, best.t)) {
+                best.t = t; best.b1 = __int_as_float(pi); best.b2 = 0.0f; best.ref = ref; best.gid = gid;
+            }
+        }
+        need = __ballot_sync(0xFFFFFFFFu, cv.which != 0u);
     }
-    int first = __ffs(inner) - 1;
-    uint32_t rest = inner & (inner - 1);
-    if (!stk.room(__popc(rest))) { ok = false; return false; }
-#pragma unroll
-    for (int c = 0; c < WN; c++)
-        if ((rest >> c) & 1u) stk.push(ch[c]);
-    node = ch[first];
-    return true;
+}
+
+// One node visit of the any-hit traversal (bvh.rs:487-530): true when a
+// primitive was hit.
+template <bool ANA, int NF>
+RT_D bool any_visit(const DevScene& S, const RayC& R, float3 d, float tmin, float tmax, uint2& grp, NodeHead& h,
+                    uint32_t& inner, Convex& cv) {
+    const uint32_t node = take_first(grp);
+    const uint32_t hits = node_test_any<NF>(S, node, R, tmin, tmax, h);
+    uint32_t leaves = hits & (h.masks >> 8);
+    inner = hits & h.masks & 0xFFu;
+    cv.which = 0u;
+    if (leaves) {
+        const uint32_t all = h.masks >> 8;
+        cv.first = h.leaf;
+#pragma unroll 1
+        while (leaves) {
+            uint32_t k = __popc(all & ((leaves & (0u - leaves)) - 1u));
+            leaves &= leaves - 1;
+            bool convex = false;
+            if (leaf_any<ANA>(S, leaf_set<NF>(S), h.leaf + k, R, d, tmin, tmax, &convex)) { cv.which = 0u; return true; }
+            if (ANA && convex) cv.which |= 1u << k;
+        }
+    }
+    return false;
+}
+// The noted convex solids of the warp's lanes (every lane calls it): true for a lane whose ray hit one.
+RT_D bool any_convex(const DevScene& S, const LeafSet& LS, const RayC& R, float3 d, float tmin, float tmax, Convex& cv) {
+    bool hit = false;
+    uint32_t need = __ballot_sync(0xFFFFFFFFu, cv.which != 0u);
+    while (need) {
+        const int L = __ffs(need) - 1;
+        const uint32_t leaf = __shfl_sync(0xFFFFFFFFu, cv.first + __ffs(cv.which) - 1u, L);
+        if ((threadIdx.x & 31u) == L) cv.which &= cv.which - 1u;
+        const uint32_t ref = f2u(__ldg(LS.rec + (size_t)leaf * 3 + 2).z);
+        float4 c0 = __ldg(S.cvx + (size_t)RT_HIT_INDEX(ref) * 2);
+        float t;
+        int pi;
+        bool h = warp_convex(S.cvx_planes + __float_as_int(c0.x), __float_as_int(c0.y), shfl3(R.o, L), shfl3(d, L),
+                             __shfl_sync(0xFFFFFFFFu, tmin, L), __shfl_sync(0xFFFFFFFFu, tmax, L), &t, &pi);
+        if (h && (threadIdx.x & 31u) == L && leaf_box(LS.box + (size_t)leaf * 2, R, tmin, tmax)) { hit = true; cv.which = 0u; }
+        need = __ballot_sync(0xFFFFFFFFu, cv.which != 0u);
+    }
+    return hit;
 }
 
 RT_D bool nan_ray(float3 o, float3 d, float tmin, float tmax) {
@@ -634,29 +674,40 @@ RT_D bool nan_ray(float3 o, float3 d, float tmin, float tmax) {
 #define RT_REFILL_CLOSEST 24
 #endif
 #define FULLMASK 0xFFFFFFFFu
+// Resident blocks per SM each traversal kernel is compiled for.  Full nodes
+// keep 48 box words in flight: 7 blocks (72 registers; gem extend 9.0 ms against
+// 9.7 at 5, 10.0 at 6 and 10.2 at 8, where ptxas spills).  Quantised nodes need
+// 12: 8 blocks (64 registers; icosphere extend 49.7 ms against 54.6, 50.9, 51.6
+// at 6, 7, 9).  The closest-hit kernel with the convex solids' warp test takes 6
+// (gem room extend 7.0 ms against 7.7 at 7).
+template <int NF, bool ANA, bool ANY> constexpr int trace_minb() {
+    return NF == RT_NODES_QUANTISED ? 8 : ANA && !ANY ? 6 : 7;
+}
+static_assert(RT_TRACE_MINB == 8, "the spill columns are sized for the most resident blocks");
 
 // MODE 0: wavefront extend (queue of path ids, rays in PathState, hits to PathState)
 // MODE 1: API (rays n×8 in memory, hits as int4)
 
 template <int MODE, bool ANA, int NF>
-__global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_TRACE_MINB) k_closest(DevScene S, PathState P, const uint32_t* __restrict__ queue,
+__global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) k_closest(DevScene S, PathState P, const uint32_t* __restrict__ queue,
                                                             const float* __restrict__ rays, uint32_t n_api,
                                                             const uint32_t* count, uint32_t* next,
                                                             int4* __restrict__ out, int* err) {
     const uint32_t n = MODE == 0 ? *count : n_api;
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
 #if RT_STACK_LOCAL
-    uint32_t ring[RT_SHORT_STACK];
+    uint2 ring[RT_SHORT_STACK];
 #else
-    __shared__ uint32_t ring[RT_SHORT_STACK * RT_TRACE_BLOCK];
+    __shared__ uint2 ring[RT_SHORT_STACK * RT_TRACE_BLOCK];
 #endif
-    rtk::TStack stk = rtk::make_stack(S, ring);
+    rtk::TStack stk{RT_STACK_LOCAL ? ring : ring + threadIdx.x, 0};
     bool active = false, exhausted = false, ok = true;
-    uint32_t item = 0, node = 0, pid = 0;
+    uint32_t item = 0, pid = 0;
+    uint2 grp = make_uint2(0u, 0u);
     float3 o = mk(0.f, 0.f, 0.f), d = o;
     RayC R = make_rayc(o, mk(1.f, 1.f, 1.f), 0.0f);
     float tmin = 0.0f;
-    Best best{0.0f, 0.0f, 0.0f, RT_MISS_REF, 0xFFFFFFFFu, 0u};
+    Best best{0.0f, 0.0f, 0.0f, RT_MISS_REF, 0xFFFFFFFFu};
     while (true) {
         uint32_t idle = __ballot_sync(FULLMASK, !active);
         if (!exhausted && __popc(idle) >= RT_REFILL_CLOSEST) {
@@ -680,8 +731,8 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_TRACE_MINB) k_closest(DevSc
                         tmin = r[6]; tmax = r[7];
                     }
                     R = make_rayc(o, d, tmin);
-                    best = Best{tmax, 0.0f, 0.0f, RT_MISS_REF, 0xFFFFFFFFu, 0u};
-                    node = 0; stk.sp = 0;
+                    best = Best{tmax, 0.0f, 0.0f, RT_MISS_REF, 0xFFFFFFFFu};
+                    grp = rtk::root_group(); stk.sp = 0;
                     active = !rtk::nan_ray(o, d, tmin, tmax);
                     if (!active) {
                         if (MODE == 0) P.hit[pid] = make_float4(__uint_as_float(RT_MISS_REF), 0.f, 0.f, 0.f);
@@ -691,16 +742,20 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_TRACE_MINB) k_closest(DevSc
             }
         }
         if (exhausted && __ballot_sync(FULLMASK, active) == 0) break;
+        NodeHead h{0u, 0u, 0u};
+        uint32_t inner = 0u;
+        rtk::Convex cv{0u, 0u};
+        if (active) rtk::closest_visit<ANA, NF>(S, R, d, tmin, best, grp, h, inner, cv);
+        if (ANA) rtk::closest_convex(S, leaf_set<NF>(S), R, d, tmin, best, cv);
         if (active) {
             bool lok = true;
-            bool more = rtk::closest_step<ANA, NF>(S, R, d, tmin, best, node, stk, lok);
+            bool more = rtk::next_group(S, grp, h.child, inner, h.masks, stk, lok);
             if (!lok) ok = false;
             if (!more) {
                 active = false;
                 bool hit = best.ref != RT_MISS_REF;
                 if (MODE == 0) {
-                    uint32_t href = hit ? RT_HIT_MAKE(best.ref, __ldg(S.mat_code + best.mat)) : RT_MISS_REF;
-                    P.hit[pid] = make_float4(__uint_as_float(href), best.t, best.b1, best.b2);
+                    P.hit[pid] = make_float4(__uint_as_float(best.ref), best.t, best.b1, best.b2);
                 } else {
                     out[item] = make_int4(hit ? (int)best.gid : -1, __float_as_int(hit ? best.t : 0.0f),
                                           __float_as_int(hit ? best.b1 : 0.0f), __float_as_int(hit ? best.b2 : 0.0f));
@@ -716,20 +771,21 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_TRACE_MINB) k_closest(DevSc
 // MODE 2: wavefront shadow rays in a scene with media (an unoccluded ray scales
 //         its parked contribution by the media's transmittance)
 template <int MODE, bool ANA, int NF>
-__global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_TRACE_MINB) k_any(DevScene S, PendTargets T, const float4* __restrict__ sq,
+__global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, true>()) k_any(DevScene S, PendTargets T, const float4* __restrict__ sq,
                                                         const float* __restrict__ rays, uint32_t n_api,
                                                         const uint32_t* count, uint32_t* next,
                                                         uint8_t* __restrict__ out, int* err) {
     const uint32_t n = MODE != 1 ? *count : n_api;
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
 #if RT_STACK_LOCAL
-    uint32_t ring[RT_SHORT_STACK];
+    uint2 ring[RT_SHORT_STACK];
 #else
-    __shared__ uint32_t ring[RT_SHORT_STACK * RT_TRACE_BLOCK];
+    __shared__ uint2 ring[RT_SHORT_STACK * RT_TRACE_BLOCK];
 #endif
-    rtk::TStack stk = rtk::make_stack(S, ring);
+    rtk::TStack stk{RT_STACK_LOCAL ? ring : ring + threadIdx.x, 0};
     bool active = false, exhausted = false, ok = true;
-    uint32_t item = 0, node = 0, tag = 0;
+    uint32_t item = 0, tag = 0;
+    uint2 grp = make_uint2(0u, 0u);
     float3 o = mk(0.f, 0.f, 0.f), d = o;
     RayC R = make_rayc(o, mk(1.f, 1.f, 1.f), 0.0f);
     float tmin = 0.0f, tmax = 0.0f;
@@ -756,16 +812,21 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, RT_TRACE_MINB) k_any(DevScene 
                         tmin = r[6]; tmax = r[7];
                     }
                     R = make_rayc(o, d, tmin);
-                    node = 0; stk.sp = 0; hit = false;
+                    grp = rtk::root_group(); stk.sp = 0; hit = false;
                     active = !rtk::nan_ray(o, d, tmin, tmax);
                     if (!active && MODE == 1) out[i] = 0;
                 }
             }
         }
         if (exhausted && __ballot_sync(FULLMASK, active) == 0) break;
+        NodeHead h{0u, 0u, 0u};
+        uint32_t inner = 0u;
+        rtk::Convex cv{0u, 0u};
+        if (active) hit = rtk::any_visit<ANA, NF>(S, R, d, tmin, tmax, grp, h, inner, cv);
+        if (ANA) { if (rtk::any_convex(S, leaf_set<NF>(S), R, d, tmin, tmax, cv)) hit = true; }
         if (active) {
             bool lok = true;
-            bool more = rtk::any_step<ANA, NF>(S, R, d, tmin, tmax, node, stk, hit, lok);
+            bool more = !hit && rtk::next_group(S, grp, h.child, inner, h.masks, stk, lok);
             if (!lok) ok = false;
             if (!more) {
                 active = false;
@@ -906,29 +967,40 @@ __global__ void __launch_bounds__(BIN_BLOCK) k_bin_scatter(PathState A, const ui
 }
 
 namespace rth {
-#ifndef RT_TRACE_GRID_PER_SM
-#define RT_TRACE_GRID_PER_SM RT_TRACE_MINB
-#endif
 // persistent kernels: one wave of resident blocks, or fewer when tuned
-int trace_grid(const DevScene& S, int dev_sms) {
-    int per = S.trace_per_sm > 0 ? std::min(S.trace_per_sm, RT_TRACE_MINB) : RT_TRACE_GRID_PER_SM;
-    return dev_sms * per;
+int trace_grid(const DevScene& S, int dev_sms, int resident) {
+    return dev_sms * (S.trace_per_sm > 0 ? std::min(S.trace_per_sm, resident) : resident);
 }
 
-// the traversal kernels with (ANA) or without analytic solids
-#define RT_TRACE_LAUNCH(K, MODE, ...)                                                                         \
-    do {                                                                                                      \
-        const int g_ = trace_grid(S, sms);                                                                    \
-        const int f_ = S.node_format;                                                                        \
-        if (S.n_analytic > 0) {                                                                               \
-            if (f_ == RT_NODES_QUANTISED)  K<MODE, true, RT_NODES_QUANTISED><<<g_, RT_TRACE_BLOCK, 0, st>>>(__VA_ARGS__); \
-            else if (f_ == RT_NODES_WIDE4) K<MODE, true, RT_NODES_WIDE4><<<g_, RT_TRACE_BLOCK, 0, st>>>(__VA_ARGS__);     \
-            else                           K<MODE, true, RT_NODES_FULL><<<g_, RT_TRACE_BLOCK, 0, st>>>(__VA_ARGS__);      \
-        } else {                                                                                              \
-            if (f_ == RT_NODES_QUANTISED)  K<MODE, false, RT_NODES_QUANTISED><<<g_, RT_TRACE_BLOCK, 0, st>>>(__VA_ARGS__); \
-            else if (f_ == RT_NODES_WIDE4) K<MODE, false, RT_NODES_WIDE4><<<g_, RT_TRACE_BLOCK, 0, st>>>(__VA_ARGS__);     \
-            else                           K<MODE, false, RT_NODES_FULL><<<g_, RT_TRACE_BLOCK, 0, st>>>(__VA_ARGS__);      \
-        }                                                                                                     \
+// The layout a launch reads.  Default (RT_NODES_FULL): the quantised copy for
+// trees whose full nodes are far beyond the L1, where its 80 bytes against 208
+// win more in fetches than its decoding costs (16-spp icosphere frames by
+// subdivision 4, 6, 7, extend + shadow: full 8.8, 12.9, 15.9 ms, quantised 9.2,
+// 12.9, 15.1); and for caller-given rays, which are incoherent as a rule (4M
+// random rays, subdivision 4, 6, 7: full 1.21, 1.60, 1.86 ms, quantised 1.11,
+// 1.42, 1.56), from 256 nodes.
+int trace_format(const DevScene& S, bool caller_rays) {
+    if (S.node_format == RT_NODES_FULL && S.qnodes && S.n_nodes >= (caller_rays ? 256u : 32768u))
+        return RT_NODES_QUANTISED;
+    return S.node_format;
+}
+// the traversal kernels with (ANA) or without analytic solids, by node layout
+#define RT_TRACE_ONE(K, MODE, ANA, NF, ...)                                                          \
+    K<MODE, ANA, NF><<<trace_grid(S, sms, trace_minb<NF, ANA, K##_any>()), RT_TRACE_BLOCK, 0, st>>>(__VA_ARGS__)
+#define RT_TRACE_LAUNCH(K, MODE, ...)                                                                           \
+    do {                                                                                                        \
+        constexpr bool k_closest_any = false, k_any_any = true;                                                 \
+        (void)k_closest_any; (void)k_any_any;                                                                   \
+        const int f_ = trace_format(S, MODE == 1);                                                              \
+        if (S.n_analytic > 0) {                                                                                 \
+            if (f_ == RT_NODES_QUANTISED)  RT_TRACE_ONE(K, MODE, true, RT_NODES_QUANTISED, __VA_ARGS__);        \
+            else if (f_ == RT_NODES_WIDE4) RT_TRACE_ONE(K, MODE, true, RT_NODES_WIDE4, __VA_ARGS__);            \
+            else                           RT_TRACE_ONE(K, MODE, true, RT_NODES_FULL, __VA_ARGS__);             \
+        } else {                                                                                                \
+            if (f_ == RT_NODES_QUANTISED)  RT_TRACE_ONE(K, MODE, false, RT_NODES_QUANTISED, __VA_ARGS__);       \
+            else if (f_ == RT_NODES_WIDE4) RT_TRACE_ONE(K, MODE, false, RT_NODES_WIDE4, __VA_ARGS__);           \
+            else                           RT_TRACE_ONE(K, MODE, false, RT_NODES_FULL, __VA_ARGS__);            \
+        }                                                                                                       \
     } while (0)
 void launch_trace_closest_api(const DevScene& S, const float* rays, uint32_t n, int4* out, uint32_t* next, int* err,
                               int sms, cudaStream_t st) {
@@ -955,6 +1027,7 @@ void launch_shadow(const DevScene& S, const PendTargets& T, const float4* sq, co
     else               RT_TRACE_LAUNCH(k_any, 0, S, T, sq, nullptr, 0, count, next, nullptr, err);
 }
 #undef RT_TRACE_LAUNCH
+#undef RT_TRACE_ONE
 void launch_media(const DevScene& S, const PathState& P, const uint32_t* queue, const uint32_t* count, int sms,
                   cudaStream_t st) {
     if (queue) k_media<1><<<sms * 8, 128, 0, st>>>(S, P, queue, count);
