@@ -154,7 +154,8 @@ struct DevScene {
     // traversal stack beyond the ring: the words of entry e ≥ RT_SHORT_STACK of
     // global thread g at stack_spill[(2(e − RT_SHORT_STACK) + 0, 1) · threads + g];
     // at most stack_cap entries (lowered only by rt_set_tuning)
-    uint32_t* stack_spill;
+    uint32_t* stack_spill;      // closest hit
+    uint32_t* stack_spill_any;  // any hit
     int stack_cap;
     int stack_ring;             // shared-memory ring slots: RT_SHORT_STACK unless tuned (a power of two)
     // textures; per triangle 2 float4 of (u, v) at the corners and 3 float4 of

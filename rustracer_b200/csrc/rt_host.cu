@@ -741,7 +741,8 @@ int32_t rt_scene_destroy(RtScene* s) {
     if (s->ev1) cudaEventDestroy(s->ev1);
     if (s->caller_ev) cudaEventDestroy(s->caller_ev);
     for (auto e : s->fk.join) if (e) cudaEventDestroy(e);
-    if (s->fk.fork) cudaEventDestroy(s->fk.fork);
+    for (auto e : {s->fk.fork, s->fk.shaded, s->fk.folded}) if (e) cudaEventDestroy(e);
+    if (s->fk.shadow) cudaStreamDestroy(s->fk.shadow);
     for (auto q : s->fk.side) if (q) cudaStreamDestroy(q);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -773,7 +774,11 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
     for (auto& q : s->fk.side)
         if (cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess)
             return bail(fail(s, RT_ERR_CUDA, "cudaStreamCreate failed"));
-    if (cudaEventCreateWithFlags(&s->fk.fork, cudaEventDisableTiming) != cudaSuccess)
+    if (cudaStreamCreateWithFlags(&s->fk.shadow, cudaStreamNonBlocking) != cudaSuccess)
+        return bail(fail(s, RT_ERR_CUDA, "cudaStreamCreate failed"));
+    if (cudaEventCreateWithFlags(&s->fk.fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&s->fk.shaded, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&s->fk.folded, cudaEventDisableTiming) != cudaSuccess)
         return bail(fail(s, RT_ERR_CUDA, "cudaEventCreate failed"));
     for (auto& e : s->fk.join)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
@@ -1002,9 +1007,10 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
         size_t spill_words = 2 * (size_t)(std::max(B.max_depth, dev_wide ? W.max_depth4 : 0) + 2);
         size_t spill_threads = (size_t)s->sms * RT_TRACE_MINB * RT_TRACE_BLOCK;
         void* sp_buf = nullptr;
-        if (int rc = dalloc(s, &sp_buf, spill_words * spill_threads * sizeof(uint32_t)))
+        if (int rc = dalloc(s, &sp_buf, 2 * spill_words * spill_threads * sizeof(uint32_t)))
             return bail(rc);
         s->S.stack_spill = (uint32_t*)sp_buf;
+        s->S.stack_spill_any = s->S.stack_spill + spill_words * spill_threads;
         s->ref_nodes = std::move(B.nodes);
         s->leaf_gids = std::move(B.leaves);
         s->n_nodes = dev_wide ? W.n_nodes : (int64_t)s->ref_nodes.size();
@@ -1910,17 +1916,25 @@ static int run_wavefront(RtScene* s, const WaveBufs& W, const RtCamera* cam, con
     uint32_t* hdr = W.counters;
     auto blk = [&](uint64_t it) { return W.counters + CTR_HDR_WORDS + (it % RT_CTR_RING) * RT_CTR_STRIDE; };
     size_t ev_used = 0;
+    // The shadow rays, the caustic lookup and the fold of the ended paths run
+    // beside the next iteration's extension rays: those only need the shading
+    // and the refill, and the next shading waits for the fold.  Each of the two
+    // traversals ends in a tail of few long rays (of a 1080p icosphere iteration
+    // the SMs sit idle 10 % of the closest-hit and 28 % of the any-hit kernel),
+    // and now fills the other's.  Not while stages are timed one by one, nor in
+    // the graph, whose conditional nodes each finish before the next.
     const bool graph = (s->graph_mode || async) && !s->profiling && !(s->cap_out && s->cap_depth >= 0) && W.graphable;
+    const bool overlap = !graph && !s->profiling && !(s->cap_out && s->cap_depth >= 0);
     auto mark = [&](int kind) {
         if (!s->profiling || graph) return;
         if (ev_used >= s->pev.size()) { cudaEvent_t e; cudaEventCreate(&e); s->pev.push_back(e); s->pkind.push_back(0); }
         s->pkind[ev_used] = kind;
         cudaEventRecord(s->pev[ev_used++], s->stream);
     };
-    // launches per iteration: extend, classify, shadow, retire, one shading
+    // launches per iteration: extend, classify, shadow, retire (two halves when they overlap), one shading
     // kernel per class the scene's materials produce (the medium class counted
     // with the media pair), the guide pair and the photon gather
-    const int64_t per_it = 4 + __builtin_popcount(s->S.class_mask & ~(1u << CLS_MEDIUM)) +
+    const int64_t per_it = (overlap ? 5 : 4) + __builtin_popcount(s->S.class_mask & ~(1u << CLS_MEDIUM)) +
                            (R.guide.mode != 0 ? 2 : 0) + (s->S.n_media > 0 ? 2 : 0) + (R.photons ? 1 : 0);
     auto prologue = [&]() {
         CK(cudaMemsetAsync(W.counters, 0, sizeof(uint32_t) * RT_CTR_WORDS, s->stream));
@@ -1965,22 +1979,33 @@ static int run_wavefront(RtScene* s, const WaveBufs& W, const RtCamera* cam, con
             }
             s->cap_n = m;
         }
+        if (overlap && it > 0) CK(cudaStreamWaitEvent(s->stream, s->fk.folded, 0));
         mark(2);
         rth::launch_shade(s->S, A, B, W.Rt, R, c, W.cq, cn + CTR_COUNT, W.sq, s->sms, s->stream, &s->fk);
+        cudaStream_t sh = s->stream;
+        if (overlap) {
+            sh = s->fk.shadow;
+            CK(cudaEventRecord(s->fk.shaded, s->stream));
+            CK(cudaStreamWaitEvent(sh, s->fk.shaded, 0));
+        }
         if (R.photons) {
             // the caustic lookup scales the parked pendC terms and the shadow
             // rays cancel pend0 / pend1: disjoint writes, so the lookup runs
-            // on a side stream beside the shadow rays (joined before retire)
-            CK(cudaEventRecord(s->fk.fork, s->stream));
-            CK(cudaStreamWaitEvent(s->fk.side[0], s->fk.fork, 0));
+            // on a side stream beside the shadow rays (joined before the fold)
+            if (!overlap) CK(cudaEventRecord(s->fk.shaded, s->stream));
+            CK(cudaStreamWaitEvent(s->fk.side[0], s->fk.shaded, 0));
             rth::launch_photon_gather_paths(s->photons, T, A.gq, c + CTR_GATHER_COUNT, s->sms, s->fk.side[0]);
             CK(cudaEventRecord(s->fk.join[0], s->fk.side[0]));
         }
         mark(3);
-        rth::launch_shadow(s->S, T, W.sq, c + CTR_SHADOW_COUNT, c + CTR_SHADOW_NEXT, W.derr, s->sms, s->stream);
-        if (R.photons) CK(cudaStreamWaitEvent(s->stream, s->fk.join[0], 0));
+        rth::launch_shadow(s->S, T, W.sq, c + CTR_SHADOW_COUNT, c + CTR_SHADOW_NEXT, W.derr, s->sms, sh);
+        if (R.photons) CK(cudaStreamWaitEvent(sh, s->fk.join[0], 0));
         mark(0);
-        rth::launch_retire(s->S, B, W.Rt, R, c, hdr, blk(it + 2), cn + CTR_COUNT, s->sms, s->stream);
+        if (overlap) {
+            rth::launch_retire(s->S, B, W.Rt, R, c, hdr, blk(it + 2), cn + CTR_COUNT, true, false, s->sms, sh);
+            CK(cudaEventRecord(s->fk.folded, sh));
+        }
+        rth::launch_retire(s->S, B, W.Rt, R, c, hdr, blk(it + 2), cn + CTR_COUNT, !overlap, true, s->sms, s->stream);
         return RT_OK;
     };
     int64_t nl = 0;
@@ -2021,6 +2046,7 @@ static int run_wavefront(RtScene* s, const WaveBufs& W, const RtCamera* cam, con
                 if (((volatile uint32_t*)s->h_status)[js] == 0) done = true;
             }
         }
+        if (overlap && it > 0) CK(cudaStreamWaitEvent(s->stream, s->fk.folded, 0));
         mark(0);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(tot, W.counters, sizeof(tot), cudaMemcpyDeviceToHost, s->stream));

@@ -80,6 +80,9 @@ struct ShadeFork {
     cudaStream_t side[N];
     cudaEvent_t fork;
     cudaEvent_t join[N];
+    // the shadow rays and the fold of the ended paths, beside the next extension rays
+    cudaStream_t shadow;
+    cudaEvent_t shaded, folded;
 };
 
 // Per-path wavefront state, structure of arrays.  The render loop keeps two
@@ -235,11 +238,12 @@ void launch_generate(const rtd::DevScene& S, const PathState& A, const RenderLau
 void launch_shade(const rtd::DevScene& S, const PathState& A, const PathState& B, const PathState& Rt,
                   const RenderLaunch& R, uint32_t* ctr, const ClassQueues& Q, uint32_t* cout, float4* sq, int sms,
                   cudaStream_t st, const ShadeFork* fk = nullptr);
-// write the ended paths' samples and append new samples, one per ended path
-// while samples remain, to B; add the iteration's ray counts to the header;
-// clear the counter block of iteration it + 2
+// fold: write the ended paths' samples; refill: append new samples, one per
+// ended path while samples remain, to B, add the iteration's ray counts to the
+// header and clear the counter block of iteration it + 2
 void launch_retire(const rtd::DevScene& S, const PathState& B, const PathState& Rt, const RenderLaunch& R,
-                   uint32_t* ctr, uint32_t* hdr, uint32_t* clear_block, uint32_t* cout, int sms, cudaStream_t st);
+                   uint32_t* ctr, uint32_t* hdr, uint32_t* clear_block, uint32_t* cout, bool fold, bool refill, int sms,
+                   cudaStream_t st);
 // active-pixel list of a converged mask, and zero output for converged pixels
 void launch_active_list(const uint8_t* conv, uint32_t width, uint32_t height, uint32_t* list, uint32_t* count,
                         cudaStream_t st);

@@ -442,7 +442,13 @@ __global__ void k_generate(DevScene S, PathState A, const RenderLaunch* __restri
 // An ended path folds its last parked contributions (caustic, area-light NEE,
 // env NEE — the order of renderer.rs:461-540) and writes its sample; for each
 // ended path the next ungenerated sample, if any, is appended to the next set.
+// Two halves, one launch each when the shadow rays run beside the next
+// extension rays (run_wavefront), both in one otherwise: REFILL hands out the
+// new samples and does the iteration's bookkeeping, which only needs the shading
+// kernels; FOLD writes the ended paths' samples and so needs the shadow rays
+// and the caustic lookup.
 #define RETIRE_BLOCK 256
+template <bool FOLD, bool REFILL>
 __global__ void __launch_bounds__(RETIRE_BLOCK) k_retire(DevScene S, PathState B, PathState Rt,
                                                          const RenderLaunch* __restrict__ Rp, uint32_t* ctr,
                                                          uint32_t* hdr, uint32_t* clear_block, uint32_t* cout) {
@@ -450,7 +456,7 @@ __global__ void __launch_bounds__(RETIRE_BLOCK) k_retire(DevScene S, PathState B
     __shared__ BlockQ<1, RETIRE_BLOCK / 32> shq;
     __shared__ unsigned long long gbase;
     uint32_t n = ctr[CTR_RETIRE_COUNT];
-    if (blockIdx.x == 0) {
+    if (REFILL && blockIdx.x == 0) {
         if (threadIdx.x == 0) {
             atomicAdd((unsigned long long*)(hdr + HDR_EXT), (unsigned long long)ctr[CTR_COUNT]);
             atomicAdd((unsigned long long*)(hdr + HDR_SHADOW), (unsigned long long)ctr[CTR_SHADOW_COUNT]);
@@ -461,7 +467,7 @@ __global__ void __launch_bounds__(RETIRE_BLOCK) k_retire(DevScene S, PathState B
     for (uint32_t t0 = blockIdx.x * RETIRE_BLOCK; t0 < n; t0 += gridDim.x * RETIRE_BLOCK) {
         uint32_t j = t0 + threadIdx.x;
         bool act = j < n;
-        if (act) {
+        if (FOLD && act) {
             float4 L = Rt.L[j], a = Rt.pend0[j], b = Rt.pend1[j];
             if (R.photons) { float4 c = Rt.pendC[j]; L.x += c.x; L.y += c.y; L.z += c.z; }
             L.x += a.x; L.y += a.y; L.z += a.z;
@@ -487,6 +493,7 @@ __global__ void __launch_bounds__(RETIRE_BLOCK) k_retire(DevScene S, PathState B
                 }
             }
         }
+        if (!REFILL) continue;
         // one claim of new samples per block: the tile's ended paths are
         // t0 .. t0 + min(n − t0, RETIRE_BLOCK) − 1, in thread order
         uint32_t tile_n = min(n - t0, (uint32_t)RETIRE_BLOCK);
@@ -1302,8 +1309,11 @@ void launch_shade(const DevScene& S, const PathState& A, const PathState& B, con
     for (int i = 0; i < nside; i++) cudaStreamWaitEvent(st, fk->join[i], 0);
 }
 void launch_retire(const DevScene& S, const PathState& B, const PathState& Rt, const RenderLaunch& R, uint32_t* ctr,
-                   uint32_t* hdr, uint32_t* clear_block, uint32_t* cout, int sms, cudaStream_t st) {
-    k_retire<<<sms * 8, RETIRE_BLOCK, 0, st>>>(S, B, Rt, R.dev, ctr, hdr, clear_block, cout);
+                   uint32_t* hdr, uint32_t* clear_block, uint32_t* cout, bool fold, bool refill, int sms,
+                   cudaStream_t st) {
+    if (fold && refill) k_retire<true, true><<<sms * 8, RETIRE_BLOCK, 0, st>>>(S, B, Rt, R.dev, ctr, hdr, clear_block, cout);
+    else if (fold)      k_retire<true, false><<<sms * 8, RETIRE_BLOCK, 0, st>>>(S, B, Rt, R.dev, ctr, hdr, clear_block, cout);
+    else                k_retire<false, true><<<sms * 8, RETIRE_BLOCK, 0, st>>>(S, B, Rt, R.dev, ctr, hdr, clear_block, cout);
 }
 void launch_active_list(const uint8_t* conv, uint32_t width, uint32_t height, uint32_t* list, uint32_t* count,
                         cudaStream_t st) {

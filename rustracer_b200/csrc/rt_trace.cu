@@ -490,12 +490,13 @@ constexpr int RING_STRIDE = RT_STACK_LOCAL ? 1 : RT_TRACE_BLOCK;
 struct TStack {
     uint2* ring;             // ring slot k at ring[k · RING_STRIDE] (shared: &ring[threadIdx.x])
     int sp;
+    bool any;                // the any-hit kernel's columns: it may run beside the closest-hit kernel
 
     // S.stack_cap entries at most; S.stack_ring ring slots in use (a power of two).
     // The spill column's address is formed only when an entry goes there.
     RT_D bool room(const DevScene& S) const { return sp < S.stack_cap; }
     RT_D uint32_t* column(const DevScene& S, int e) const {
-        return S.stack_spill + (size_t)(2 * e) * (gridDim.x * blockDim.x) + blockIdx.x * blockDim.x + threadIdx.x;
+        return (any ? S.stack_spill_any : S.stack_spill) + (size_t)(2 * e) * (gridDim.x * blockDim.x) + blockIdx.x * blockDim.x + threadIdx.x;
     }
     RT_D void push(const DevScene& S, uint2 v) {
         int slot = sp & (S.stack_ring - 1);
@@ -700,7 +701,7 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) 
 #else
     __shared__ uint2 ring[RT_SHORT_STACK * RT_TRACE_BLOCK];
 #endif
-    rtk::TStack stk{RT_STACK_LOCAL ? ring : ring + threadIdx.x, 0};
+    rtk::TStack stk{RT_STACK_LOCAL ? ring : ring + threadIdx.x, 0, false};
     bool active = false, exhausted = false, ok = true;
     uint32_t item = 0, pid = 0;
     uint2 grp = make_uint2(0u, 0u);
@@ -782,7 +783,7 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, true>()) k
 #else
     __shared__ uint2 ring[RT_SHORT_STACK * RT_TRACE_BLOCK];
 #endif
-    rtk::TStack stk{RT_STACK_LOCAL ? ring : ring + threadIdx.x, 0};
+    rtk::TStack stk{RT_STACK_LOCAL ? ring : ring + threadIdx.x, 0, true};
     bool active = false, exhausted = false, ok = true;
     uint32_t item = 0, tag = 0;
     uint2 grp = make_uint2(0u, 0u);
