@@ -1933,9 +1933,9 @@ static int run_wavefront(RtScene* s, const WaveBufs& W, const RtCamera* cam, con
     };
     // launches per iteration: extend, classify, shadow, retire (two halves when they overlap), one shading
     // kernel per class the scene's materials produce (the medium class counted
-    // with the media pair), the guide pair and the photon gather
+    // with the media pair), the guide pair and the photon gather's two
     const int64_t per_it = (overlap ? 5 : 4) + __builtin_popcount(s->S.class_mask & ~(1u << CLS_MEDIUM)) +
-                           (R.guide.mode != 0 ? 2 : 0) + (s->S.n_media > 0 ? 2 : 0) + (R.photons ? 1 : 0);
+                           (R.guide.mode != 0 ? 2 : 0) + (s->S.n_media > 0 ? 2 : 0) + (R.photons ? 2 : 0);
     auto prologue = [&]() {
         CK(cudaMemsetAsync(W.counters, 0, sizeof(uint32_t) * RT_CTR_WORDS, s->stream));
         mark(0);
@@ -1994,7 +1994,10 @@ static int run_wavefront(RtScene* s, const WaveBufs& W, const RtCamera* cam, con
             // on a side stream beside the shadow rays (joined before the fold)
             if (!overlap) CK(cudaEventRecord(s->fk.shaded, s->stream));
             CK(cudaStreamWaitEvent(s->fk.side[0], s->fk.shaded, 0));
-            rth::launch_photon_gather_paths(s->photons, T, A.gq, c + CTR_GATHER_COUNT, s->sms, s->fk.side[0]);
+            // (its list of dense requests goes where the diffuse queue was: the
+            // next classification comes after the join)
+            rth::launch_photon_gather_paths(s->photons, T, A.gq, c + CTR_GATHER_COUNT, W.cq.q[CLS_DIFFUSE],
+                                            c + CTR_GATHER_DENSE, s->sms, s->fk.side[0]);
             CK(cudaEventRecord(s->fk.join[0], s->fk.side[0]));
         }
         mark(3);

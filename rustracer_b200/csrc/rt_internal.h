@@ -51,6 +51,7 @@
 #define CTR_CLS_COUNT      5   // CLS_N entries
 #define CTR_GATHER_COUNT   15  // photon-gather requests of the iteration
 #define CTR_RETIRE_COUNT   16  // paths that ended in the iteration
+#define CTR_GATHER_DENSE   17  // photon-gather requests left to a whole warp
 
 // Render counters: a header of 64-bit totals, then a ring of RT_CTR_RING
 // iteration blocks (iteration it uses block it % RT_CTR_RING; the retire
@@ -149,6 +150,13 @@ struct PhotonMapDev {
     uint64_t generation = 0;                                  // bumped by every build, set and release
     PhotonGrid grid{{0.f, 0.f, 0.f}, 0.f, {1, 1, 1}, -1.f};
     uint2* cells = nullptr;                                   // [start, end) per grid cell
+    // the render path's copy: photons by linear cell of a finer grid (cells ≥ the
+    // gather radius, x fastest, so the cells of a row are one run), and the first
+    // photon of every cell (cells + 1 entries)
+    PhotonGrid fine{{0.f, 0.f, 0.f}, 0.f, {1, 1, 1}, -1.f};
+    float4 *fpos = nullptr, *fpow = nullptr, *fnor = nullptr;
+    uint32_t *fstart = nullptr, *fkey = nullptr, *fkey2 = nullptr;
+    size_t cap_fine = 0;
     // capacities (elements) of the map arrays, the heap, the cell table and the build's work buffers
     size_t cap_map = 0, cap_heap = 0, cap_cells = 0, cap_work = 0, cap_tmp = 0;
     uint8_t* flags = nullptr;                                 // stored flag per traced photon
@@ -259,8 +267,9 @@ cudaError_t photon_set(PhotonMapDev& map, const float4* pos, const float4* pow, 
 void launch_photon_gather_api(const PhotonMapDev& map, const float* q, uint32_t n, float* out, int sms, cudaStream_t st);
 void launch_knn_api(const PhotonMapDev& map, const float* q, uint32_t n, int k, float rmax2, int* idx, float* d2,
                     int* err, int sms, cudaStream_t st);
+// (dense_list: room for every request; dense_count: zero before the call)
 void launch_photon_gather_paths(const PhotonMapDev& map, const PendTargets& T, const float4* gq, const uint32_t* count,
-                                int sms, cudaStream_t st);
+                                uint32_t* dense_list, uint32_t* dense_count, int sms, cudaStream_t st);
 void launch_accumulate(const float* scratch, uint32_t nsamp, uint32_t npix, float* acc, float* m2, uint32_t* cnt,
                        const uint8_t* conv, float clamp, uint32_t min_samples, float floor_, cudaStream_t st);
 // The 8-wide tree collapsed on the device from the binary tree (the host

@@ -437,6 +437,15 @@ __global__ void k_gather_sorted(const uint32_t* order, uint32_t n, const float4*
         dp[i] = sp[j]; dw[i] = sw[j]; dn[i] = sn[j];
     }
 }
+// linear cell of the fine grid per photon, and the photons counted per cell
+__global__ void k_fine_keys(const float4* p, uint32_t n, PhotonGrid G, uint32_t* key, uint32_t* val, uint32_t* count) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        uint32_t c = cell_linear(G, p[i]);
+        key[i] = c;
+        val[i] = i;
+        atomicAdd(count + c, 1u);
+    }
+}
 // leaf boxes (level `leaves` of the heap), then each internal level bottom-up
 __global__ void k_leaf_boxes(const float4* p, uint32_t n, uint32_t nleaf_pow2, float4* blo, float4* bhi) {
     uint32_t first = nleaf_pow2 - 1;
@@ -470,6 +479,9 @@ struct Map {
     const float4 *blo, *bhi;         // heap of boxes
     const uint2* cells;              // [start, end) per grid cell
     PhotonGrid G;
+    const float4 *fpos, *fpow, *fnor;   // by linear cell of F, and the first photon per cell
+    const uint32_t* fstart;
+    PhotonGrid F;
     uint32_t n, nleaf_pow2;
     float r2;                        // radius (or k-NN maximum radius) squared
     uint32_t knn_k;
@@ -480,15 +492,15 @@ struct Map {
 // far more than the rounding of p ± r and of the photons' float distances —
 // so every photon with d² < r2 lies in one of the cells.
 struct CellSpan { int i0[3], i1[3]; };
-RT_D CellSpan cell_span(const Map& M, float3 p, float r2) {
+RT_D CellSpan cell_span(const PhotonGrid& G, float3 p, float r2) {
     float r = sqrtf(r2);
     float q[3] = {p.x, p.y, p.z};
     CellSpan s;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         float m = r * (1.0f + 0x1p-10f) + (fabsf(q[a]) + r) * 0x1p-20f;
-        s.i0[a] = grid_cell(q[a] - m, M.G.lo[a], M.G.inv, M.G.n[a]);
-        s.i1[a] = grid_cell(q[a] + m, M.G.lo[a], M.G.inv, M.G.n[a]);
+        s.i0[a] = grid_cell(q[a] - m, G.lo[a], G.inv, G.n[a]);
+        s.i1[a] = grid_cell(q[a] + m, G.lo[a], G.inv, G.n[a]);
     }
     return s;
 }
@@ -542,7 +554,7 @@ RT_D void for_leaves(const Map& M, float3 p, float r2, F f) {
 template <class F>
 RT_D void for_near(const Map& M, float3 p, float r2, F f) {
     if (r2 <= M.G.r2) {
-        CellSpan s = cell_span(M, p, r2);
+        CellSpan s = cell_span(M.G, p, r2);
         if (span_photons(M, s) <= PH_GRID_WARP_MAX) {
             uint32_t lane = threadIdx.x & 31u;
             for (int z = s.i0[2]; z <= s.i1[2]; z++)
@@ -814,7 +826,7 @@ RT_D float3 warp_irradiance_1pass(const Map& M, float3 p, float3 n, WarpScratch&
     // the ball to collect: within the maximum radius and, in k-NN mode, within
     // the seed subtree's k-th distance (inclusive, so ties at it are kept)
     // (the grid's cells hold a few times the photons in range: no seed there)
-    bool grid = M.r2 <= M.G.r2 && span_photons(M, cell_span(M, p, M.r2)) <= PH_GRID_WARP_MAX;
+    bool grid = M.r2 <= M.G.r2 && span_photons(M, cell_span(M.G, p, M.r2)) <= PH_GRID_WARP_MAX;
     float bound = !grid && M.knn_k > 0 && M.knn_k <= PH_SEED_LEAVES * PH_LEAF ? seed_bound(M, p, n, W) : M.r2;
     uint32_t cnt = 0;
     for_near(M, p, bound, [&](int i) {
@@ -861,7 +873,7 @@ RT_D float3 warp_irradiance_1pass(const Map& M, float3 p, float3 n, WarpScratch&
 RT_D float3 warp_gather(const Map& M, float3 p, float3 n, WarpScratch& W, uint32_t* hist, float* sel) {
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
     if (!(M.r2 <= M.G.r2)) return warp_irradiance_1pass(M, p, n, W, hist, sel);
-    CellSpan s = cell_span(M, p, M.r2);
+    CellSpan s = cell_span(M.G, p, M.r2);
     if (s.i1[0] - s.i0[0] > 1 || s.i1[1] - s.i0[1] > 1 || s.i1[2] - s.i0[2] > 1)
         return warp_irradiance_1pass(M, p, n, W, hist, sel);
     uint32_t st = 0, len = 0;
@@ -1003,31 +1015,198 @@ __global__ void k_knn_api(rtph::Map M, const float* q, uint32_t n, int k, float 
 }
 
 // render path: caustic injection at queued diffuse vertices (renderer.rs:461-467);
-// pendC[pid] holds T·tint·albedo and becomes that × irradiance
-__global__ void __launch_bounds__(RT_SHADE_BLOCK) k_photon_gather_paths(rtph::Map M, PendTargets T,
-                                                                        const float4* __restrict__ gq,
-                                                                        const uint32_t* count) {
-    __shared__ uint32_t hist[RT_SHADE_BLOCK / 32][32];
-    __shared__ float sel[RT_SHADE_BLOCK / 32][PH_SEL_CAP];
-    __shared__ rtph::WarpScratch ws[RT_SHADE_BLOCK / 32];
-    uint32_t n = *count;
-    uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    // one warp per request (its cells' photons are few, and coalesced); the
-    // next request is loaded while this one is gathered
-    float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na;
-    if (gw < n) { na = gq[(size_t)gw * 2]; nb = gq[(size_t)gw * 2 + 1]; }
-    for (uint32_t i = gw; i < n; i += nw) {
-        float4 qa = na, qb = nb;
-        if (i + nw < n) { na = gq[(size_t)(i + nw) * 2]; nb = gq[(size_t)(i + nw) * 2 + 1]; }
-        float3 r = rtph::warp_gather(M, mk(qa.x, qa.y, qa.z), mk(qb.x, qb.y, qb.z), ws[w], hist[w], sel[w]);
-        if (lane == 0) {
-            uint32_t tag = __float_as_uint(qa.w);
-            float4* pc = T.pendC[(tag >> 1) & 1u] + (tag >> 2);
-            float4 f = *pc;
-            bool any = r.x > 0.0f || r.y > 0.0f || r.z > 0.0f;
-            *pc = any ? make_float4(f.x * r.x, f.y * r.y, f.z * r.z, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+// pendC[pid] holds T·tint·albedo and becomes that × irradiance.
+//
+// A ball of the gather radius meets at most 3 × 3 × 3 cells of the fine grid,
+// that is ≤ 9 runs of photons (a row of cells along x is one run).  Two kernels:
+//   k_gather_sparse  one lane per request finds its runs and, when they hold few
+//                    photons, sums them; the others go to a list
+//   k_gather_dense   one warp per listed request, 32 photons of its joined runs
+//                    at a time, with the k-NN selection of warp_irradiance_1pass
+// One warp per request over cells of twice the radius, as before, tested 5
+// photons for one in range and spent two thirds of its instructions on finding
+// each request's 2-3 batches of 32 (gem room: 82 photons tested per request and
+// 8-12 in range, 364 warp instructions; now 40 tested).
+#define PH_ROWS 9
+// photons a lane sums by itself (gem / gem room frames at 24, 48, 96, 144, 256,
+// 512: 32.7 / 24.7, 32.0 / 23.2, 31.6 / 22.3, 31.3 / 22.3, 31.3 / 22.6, 31.8 / 24.8
+// ms; one warp per request 35.0 / 30.5)
+#define PH_LANE_MAX 128u
+RT_D uint2 gather_run(const rtph::Map& M, const rtph::CellSpan& s, int r) {
+    const int y = s.i0[1] + r % 3, z = s.i0[2] + r / 3;
+    if (y > s.i1[1] || z > s.i1[2]) return make_uint2(0u, 0u);
+    const size_t row = (size_t)M.F.n[0] * ((size_t)y + (size_t)M.F.n[1] * z);
+    return make_uint2(__ldg(M.fstart + row + s.i0[0]), __ldg(M.fstart + row + s.i1[0] + 1));
+}
+// more rows than the table holds (a coordinate far beyond the radius, where the
+// span is widened by its rounding): the general gather
+RT_D bool gather_wide(const rtph::CellSpan& s) { return s.i1[1] - s.i0[1] > 2 || s.i1[2] - s.i0[2] > 2; }
+RT_D void gather_result(const PendTargets& T, float tagf, float3 irr) {
+    const uint32_t tag = __float_as_uint(tagf);
+    float4* pc = T.pendC[(tag >> 1) & 1u] + (tag >> 2);
+    if (irr.x > 0.0f || irr.y > 0.0f || irr.z > 0.0f) {
+        float4 f = *pc;
+        *pc = make_float4(f.x * irr.x, f.y * irr.y, f.z * irr.z, 0.f);
+    } else {
+        *pc = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+#define GATHER_BLOCK 128
+__global__ void __launch_bounds__(GATHER_BLOCK) k_gather_sparse(rtph::Map M, PendTargets T,
+                                                                const float4* __restrict__ gq, const uint32_t* count,
+                                                                uint32_t* dense_list, uint32_t* dense_count) {
+    __shared__ uint2 runs[PH_ROWS][GATHER_BLOCK];
+    const uint32_t n = *count, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    // a queue too short to fill the lanes of the grid goes to the warps whole
+    const uint32_t lane_max = n >= gridDim.x * (GATHER_BLOCK / 8) ? PH_LANE_MAX : 0u;
+    for (uint32_t b = blockIdx.x * GATHER_BLOCK; b < n; b += gridDim.x * GATHER_BLOCK) {
+        const uint32_t i = b + threadIdx.x;
+        bool dense = false;
+        if (i < n) {
+            const float4 qa = gq[(size_t)i * 2], qb = gq[(size_t)i * 2 + 1];
+            const float3 p = mk(qa.x, qa.y, qa.z), nn = mk(qb.x, qb.y, qb.z);
+            const rtph::CellSpan s = rtph::cell_span(M.F, p, M.r2);
+            uint32_t total = 0;
+#pragma unroll
+            for (int r = 0; r < PH_ROWS; r++) {
+                const uint2 run = gather_run(M, s, r);
+                runs[r][threadIdx.x] = run;
+                total += run.y - run.x;
+            }
+            dense = gather_wide(s) || total > lane_max;
+            if (!dense) {
+                float3 acc = mk(0.f, 0.f, 0.f);
+                uint32_t cnt = 0, r = 0;
+                uint2 run = runs[0][threadIdx.x];
+                // the runs as one list, two photons a step
+                for (uint32_t k = 0; k < total; k += 2) {
+                    float4 q[2];
+                    uint32_t id[2];
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        id[u] = 0xFFFFFFFFu;
+                        if (k + u < total) {
+                            while (run.x >= run.y) run = runs[++r][threadIdx.x];
+                            id[u] = run.x++;
+                            q[u] = __ldg(M.fpos + id[u]);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        if (id[u] == 0xFFFFFFFFu) continue;
+                        const float d2 = rtph::pdist2(q[u], p);
+                        if (!(d2 < M.r2)) continue;
+                        const float4 nv = __ldg(M.fnor + id[u]), pw = __ldg(M.fpow + id[u]);
+                        if (!(rtph::pdot(nv, nn) > 0.0f)) continue;
+                        acc = acc + mk(pw.x, pw.y, pw.z) * (1.0f - d2 / M.r2);
+                        cnt++;
+                    }
+                }
+                if (M.knn_k > 0 && cnt >= M.knn_k) dense = true;         // the k-th distance has to be found
+                else gather_result(T, qa.w, acc * (2.0f / (PI_F * PI_F * M.r2)));
+            }
         }
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, dense);
+        if (m) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(dense_count, __popc(m));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(m & lt);
+            if (dense) dense_list[at] = i;
+        }
+    }
+}
+__global__ void __launch_bounds__(GATHER_BLOCK) k_gather_dense(rtph::Map M, PendTargets T,
+                                                               const float4* __restrict__ gq,
+                                                               const uint32_t* __restrict__ list,
+                                                               const uint32_t* count) {
+    __shared__ uint32_t hist[GATHER_BLOCK / 32][32];
+    __shared__ float sel[GATHER_BLOCK / 32][PH_SEL_CAP];
+    __shared__ rtph::WarpScratch ws[GATHER_BLOCK / 32];
+    const uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t n = *count;
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    rtph::WarpScratch& W = ws[w];
+    // the next request is loaded while this one is gathered
+    float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na;
+    if (gw < n) { uint32_t j = list[gw]; na = gq[(size_t)j * 2]; nb = gq[(size_t)j * 2 + 1]; }
+    for (uint32_t i = gw; i < n; i += nw) {
+        const float4 qa = na, qb = nb;
+        if (i + nw < n) { uint32_t j = list[i + nw]; na = gq[(size_t)j * 2]; nb = gq[(size_t)j * 2 + 1]; }
+        const float3 p = mk(qa.x, qa.y, qa.z), nn = mk(qb.x, qb.y, qb.z);
+        const rtph::CellSpan s = rtph::cell_span(M.F, p, M.r2);
+        // the runs joined into one list: lane j takes entries j, j + 32, …
+        const uint2 run = lane < PH_ROWS ? gather_run(M, s, (int)lane) : make_uint2(0u, 0u);
+        uint32_t inc = run.y - run.x;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            uint32_t v = __shfl_up_sync(FULL, inc, o);
+            if (lane >= (uint32_t)o) inc += v;
+        }
+        const uint32_t total = __shfl_sync(FULL, inc, PH_ROWS - 1), exc = inc - (run.y - run.x);
+        float3 res = mk(0.f, 0.f, 0.f);
+        if (gather_wide(s) || total > PH_GRID_WARP_MAX) {
+            res = rtph::warp_gather(M, p, nn, W, hist[w], sel[w]);
+        } else {
+            // entry f of run r is photon f + (start − entries before the run)
+            uint32_t ex[PH_ROWS], off[PH_ROWS];
+#pragma unroll
+            for (int r = 0; r < PH_ROWS; r++) {
+                ex[r] = __shfl_sync(FULL, exc, r);
+                off[r] = __shfl_sync(FULL, run.x - exc, r);
+            }
+            // the radius-r sum, gathered in the same pass: the estimate whenever fewer
+            // than k photons are in range (and always in radius mode)
+            float3 acc = mk(0.f, 0.f, 0.f);
+            uint32_t cnt = 0;
+            for (uint32_t base = 0; base < total; base += 32) {
+                const uint32_t f = base + lane;
+                bool c = false;
+                float d2 = 0.0f;
+                uint32_t k = 0;
+                if (f < total) {
+                    uint32_t o = off[0];
+#pragma unroll
+                    for (int r = 1; r < PH_ROWS; r++)
+                        if (ex[r] <= f) o = off[r];
+                    k = f + o;
+                    // position, normal and power in one round trip (the map is L2-resident)
+                    const float4 q = __ldg(M.fpos + k), nv = __ldg(M.fnor + k), pw = __ldg(M.fpow + k);
+                    d2 = rtph::pdist2(q, p);
+                    c = d2 < M.r2 && rtph::pdot(nv, nn) > 0.0f;
+                    if (c) acc = acc + mk(pw.x, pw.y, pw.z) * (1.0f - d2 / M.r2);
+                }
+                const uint32_t m = __ballot_sync(FULL, c);
+                const uint32_t slot = cnt + __popc(m & lt);
+                if (c && slot < PH_CAND_CAP) { W.d2[slot] = d2; W.id[slot] = k; }
+                cnt += __popc(m);
+            }
+            __syncwarp();
+            float r2 = M.r2;
+            if (M.knn_k > 0 && cnt >= M.knn_k) {
+                if (cnt > PH_CAND_CAP) {
+                    res = rtph::warp_irradiance(M, p, nn, hist[w], sel[w]);
+                    r2 = 0.0f;
+                } else {
+                    r2 = rtph::warp_radix_select(W.d2, cnt, M.knn_k, W.hist);
+                    acc = mk(0.f, 0.f, 0.f);
+                    if (r2 > 0.0f)
+                        for (uint32_t j = lane; j < cnt; j += 32) {
+                            const float d2 = W.d2[j];
+                            if (d2 < r2) {
+                                const float4 pw = __ldg(M.fpow + W.id[j]);
+                                acc = acc + mk(pw.x, pw.y, pw.z) * (1.0f - d2 / r2);
+                            }
+                        }
+                    __syncwarp();
+                }
+            }
+            if (r2 > 0.0f) {
+                const float sc = 2.0f / (PI_F * PI_F * r2);
+                res = mk(rtph::warp_sum(acc.x) * sc, rtph::warp_sum(acc.y) * sc, rtph::warp_sum(acc.z) * sc);
+            }
+        }
+        if (lane == 0) gather_result(T, qa.w, res);
     }
 }
 
@@ -1041,7 +1220,7 @@ void PhotonMapDev::release() {
 }
 void PhotonMapDev::free_all() {
     void* ps[] = {pos, pow, nor, blo, bhi, exp_pos, exp_pow, exp_nor, flags, st_pos, st_pow, st_nor,
-                  fl32, scan, key, val, key2, val2, bounds, tmp, cells};
+                  fl32, scan, key, val, key2, val2, bounds, tmp, cells, fpos, fpow, fnor, fstart, fkey, fkey2};
     for (void* p : ps) if (p) cudaFree(p);
     pos = pow = nor = blo = bhi = exp_pos = exp_pow = exp_nor = st_pos = st_pow = st_nor = nullptr;
     flags = nullptr;
@@ -1050,6 +1229,9 @@ void PhotonMapDev::free_all() {
     bounds = nullptr;
     tmp = nullptr;
     cells = nullptr;
+    fpos = fpow = fnor = nullptr;
+    fstart = fkey = fkey2 = nullptr;
+    cap_fine = 0;
     cap_map = cap_heap = cap_cells = cap_work = cap_tmp = 0;
     release();
 }
@@ -1058,6 +1240,7 @@ rtph::Map PhotonMapDev::view() const {
     rtph::Map M;
     M.pos = pos; M.pow = pow; M.nor = nor; M.blo = blo; M.bhi = bhi;
     M.cells = cells; M.G = grid;
+    M.fpos = fpos; M.fpow = fpow; M.fnor = fnor; M.fstart = fstart; M.F = fine;
     M.n = n; M.nleaf_pow2 = nleaf_pow2; M.r2 = r2; M.knn_k = knn_k;
     return M;
 }
@@ -1078,9 +1261,9 @@ static cudaError_t ensure_map(PhotonMapDev& map, size_t n) {
     if (n <= map.cap_map && map.pos) return cudaSuccess;
     size_t c = std::max<size_t>(n, map.cap_map * 5 / 4);
     cudaError_t e;
-    float4** f4[] = {&map.pos, &map.pow, &map.nor, &map.exp_pos, &map.exp_pow, &map.exp_nor};
+    float4** f4[] = {&map.pos, &map.pow, &map.nor, &map.exp_pos, &map.exp_pow, &map.exp_nor, &map.fpos, &map.fpow, &map.fnor};
     for (float4** q : f4) if ((e = grow(*q, c, sizeof(float4)))) return e;
-    uint32_t** u4[] = {&map.val, &map.val2};
+    uint32_t** u4[] = {&map.val, &map.val2, &map.fkey, &map.fkey2};
     for (uint32_t** q : u4) if ((e = grow(*q, c, sizeof(uint32_t)))) return e;
     if ((e = grow(map.key, c, sizeof(uint64_t))) || (e = grow(map.key2, c, sizeof(uint64_t)))) return e;
     if (!map.bounds && (e = grow(map.bounds, 6, sizeof(float)))) return e;
@@ -1097,16 +1280,16 @@ static cudaError_t ensure_tmp(PhotonMapDev& map, size_t bytes) {
 }
 
 // The cell grid for photons in the box [lo, hi] and gather radius² r2: cubic
-// cells of 2r·(1 + 2^-9) — a ball of radius r (widened as cell_span widens it)
-// meets at most 2 cells per axis — or larger, to keep ≤ 1000 cells per axis
-// and ≤ RT_PH_GRID_MAX_CELLS cells in all.  No grid (one cell, r2 < 0) for a
-// zero radius.
-static PhotonGrid make_grid(const float lo[3], const float hi[3], float r2) {
+// cells of radii · r·(1 + 2^-9) — a ball of radius r (widened as cell_span widens
+// it) meets at most 2 (radii 2) or 3 (radii 1) cells per axis — or larger, to
+// keep ≤ 1000 cells per axis and ≤ RT_PH_GRID_MAX_CELLS cells in all.  No grid
+// (one cell, r2 < 0) for a zero radius.
+static PhotonGrid make_grid(const float lo[3], const float hi[3], float r2, double radii) {
     PhotonGrid G{{lo[0], lo[1], lo[2]}, 0.0f, {1, 1, 1}, -1.0f};
     if (!(r2 > 0.0f) || !std::isfinite(r2)) return G;
     double ext = 0.0;
     for (int a = 0; a < 3; a++) ext = std::max(ext, (double)hi[a] - (double)lo[a]);
-    double c = std::max(2.0 * std::sqrt((double)r2) * (1.0 + 1.0 / 512.0), ext / 1000.0);
+    double c = std::max(radii * std::sqrt((double)r2) * (1.0 + 1.0 / 512.0), ext / 1000.0);
     if (!(c > 0.0)) return G;
     for (;;) {
         double cells = 1.0;
@@ -1134,7 +1317,8 @@ static cudaError_t build_tree(PhotonMapDev& map, uint32_t n, cudaStream_t st) {
     float b[6];
     if ((e = cudaMemcpyAsync(b, map.bounds, sizeof(b), cudaMemcpyDeviceToHost, st))) return e;
     if ((e = cudaStreamSynchronize(st))) return e;
-    map.grid = make_grid(b, b + 3, map.r2);
+    map.grid = make_grid(b, b + 3, map.r2, 2.0);
+    map.fine = make_grid(b, b + 3, map.r2, 1.0);
     size_t ncell = (size_t)map.grid.n[0] * map.grid.n[1] * map.grid.n[2];
     if (ncell > map.cap_cells || !map.cells) {
         if ((e = grow(map.cells, ncell, sizeof(uint2)))) return e;
@@ -1160,6 +1344,25 @@ static cudaError_t build_tree(PhotonMapDev& map, uint32_t n, cudaStream_t st) {
                                                                                map.exp_nor, map.pos, map.pow, map.nor);
     k_cell_ranges<<<std::min<uint32_t>((n + 255) / 256, 4096), 256, 0, st>>>(map.pos, n, map.grid, map.cells);
     k_leaf_boxes<<<std::min<uint32_t>((p2 + 255) / 256, 4096), 256, 0, st>>>(map.pos, n, p2, map.blo, map.bhi);
+    // the render path's copy: by linear cell of the fine grid (emission order in a cell)
+    size_t nfine = (size_t)map.fine.n[0] * map.fine.n[1] * map.fine.n[2];
+    if (nfine + 1 > map.cap_fine || !map.fstart) {
+        if ((e = grow(map.fstart, nfine + 1, sizeof(uint32_t)))) return e;
+        map.cap_fine = nfine + 1;
+    }
+    if ((e = cudaMemsetAsync(map.fstart, 0, (nfine + 1) * sizeof(uint32_t), st))) return e;
+    k_fine_keys<<<std::min<uint32_t>((n + 255) / 256, 4096), 256, 0, st>>>(map.exp_pos, n, map.fine, map.fkey, map.val,
+                                                                           map.fstart);
+    int bits = 1;
+    while (bits < 32 && (nfine >> bits) != 0) bits++;
+    size_t tb2 = 0, tb3 = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, tb2, map.fkey, map.fkey2, map.val, map.val2, (int)n, 0, bits, st);
+    cub::DeviceScan::ExclusiveSum(nullptr, tb3, map.fstart, map.fstart, (int)(nfine + 1), st);
+    if ((e = ensure_tmp(map, std::max(tb2, tb3)))) return e;
+    cub::DeviceScan::ExclusiveSum(map.tmp, tb3, map.fstart, map.fstart, (int)(nfine + 1), st);
+    cub::DeviceRadixSort::SortPairs(map.tmp, tb2, map.fkey, map.fkey2, map.val, map.val2, (int)n, 0, bits, st);
+    k_gather_sorted<<<std::min<uint32_t>((n + 255) / 256, 4096), 256, 0, st>>>(map.val2, n, map.exp_pos, map.exp_pow,
+                                                                               map.exp_nor, map.fpos, map.fpow, map.fnor);
     for (uint32_t cnt = p2 / 2; cnt >= 1; cnt /= 2)
         k_level_boxes<<<std::min<uint32_t>((cnt + 255) / 256, 4096), 256, 0, st>>>(cnt - 1, cnt, map.blo, map.bhi);
     return cudaGetLastError();
@@ -1272,8 +1475,9 @@ void launch_knn_api(const PhotonMapDev& map, const float* q, uint32_t n, int k, 
     k_knn_api<<<sms * 4, RT_SHADE_BLOCK, 0, st>>>(map.view(), q, n, k, rmax2, idx, d2, err);
 }
 void launch_photon_gather_paths(const PhotonMapDev& map, const PendTargets& T, const float4* gq, const uint32_t* count,
-                                int sms, cudaStream_t st) {
-    k_photon_gather_paths<<<sms * 8, RT_SHADE_BLOCK, 0, st>>>(map.view(), T, gq, count);
+                                uint32_t* dense_list, uint32_t* dense_count, int sms, cudaStream_t st) {
+    k_gather_sparse<<<sms * 8, GATHER_BLOCK, 0, st>>>(map.view(), T, gq, count, dense_list, dense_count);
+    k_gather_dense<<<sms * 8, GATHER_BLOCK, 0, st>>>(map.view(), T, gq, dense_list, dense_count);
 }
 
 }  // namespace rth
