@@ -136,6 +136,7 @@ struct DevScene {
     int n_lights, n_mats;
     const DevMedium* media;
     int n_media;
+    int noise_medium;           // first noise medium (its tables go to shared memory), or −1
     int n_pbr;                  // PBR materials in the scene (their shading kernel runs only if > 0)
     uint32_t class_mask;        // bit per shading class some material of the scene can produce (host side)
     // analytic convex solids in leaf order: 2 float4 each, (plane offset, count,

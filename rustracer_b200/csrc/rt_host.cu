@@ -1424,6 +1424,8 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
         }
         if ((rc = upload(s, dm.data(), dm.size(), &s->S.media))) return bail(rc);
         s->S.n_media = d->n_media;
+    s->S.noise_medium = -1;
+    for (int32_t i = d->n_media - 1; i >= 0; i--) if (d->media[i].type == RT_MEDIUM_NOISE) s->S.noise_medium = i;
     }
 
     std::call_once(g_elut_once, build_elut);

@@ -30,13 +30,50 @@ RT_D float medium_rnd(const MedRng& r, uint32_t i) {
     return (float)(pcg3d_x(r.a, r.b, r.c ^ (i * 0x9E3779B9u)) >> 8) * (1.0f / 16777216.0f);
 }
 
-RT_D float perlin_noise(const float4* vec, const int32_t* perm, float3 p) {
+// The Perlin tables of a noise medium: 256 gradient vectors and the three
+// permutations.  From global memory, or from a block's shared copy laid out so
+// that no two lanes of a warp meet in a bank: 8 copies of the vectors, copy
+// j = lane mod 8 in the 16-byte bank group j, and 32 of the permutations (the
+// three of an index in one word), copy j = lane in bank j.  A noise value gathers
+// 8 vectors and 6 permutation entries at random; through the L1 that was ≈9 and
+// ≈3.5 passes per gather and the bound of both media kernels, here it is 4 and 1.
+struct GlobalNoise {
+    const float4* vec_;
+    const int32_t* perm_;
+    RT_D float4 vec(int i) const { return __ldg(vec_ + i); }
+    RT_D int perm(int axis, int i) const { return (int)__ldg(perm_ + 256 * axis + i); }
+};
+struct SharedNoise {
+    const float4* vec_;          // + lane mod 8
+    const uint32_t* perm_;       // + lane
+    RT_D float4 vec(int i) const { return vec_[i * 8]; }
+    RT_D int perm(int axis, int i) const { return (int)((perm_[i * 32] >> (8 * axis)) & 255u); }
+};
+#define RT_NOISE_SMEM (256 * 8 * 16 + 256 * 32 * 4)
+// fills the block's copy of medium m's tables; every thread calls it
+RT_D SharedNoise load_noise(const DevMedium& m, void* smem) {
+    float4* v = reinterpret_cast<float4*>(smem);
+    uint32_t* p = reinterpret_cast<uint32_t*>(v + 256 * 8);
+    for (int i = threadIdx.x; i < 256 * 8; i += blockDim.x) v[i] = __ldg(m.vec + (i >> 3));
+    for (int i = threadIdx.x; i < 256 * 32; i += blockDim.x) {
+        int e = i >> 5;
+        p[i] = (uint32_t)__ldg(m.perm + e) | (uint32_t)__ldg(m.perm + 256 + e) << 8 | (uint32_t)__ldg(m.perm + 512 + e) << 16;
+    }
+    __syncthreads();
+    return SharedNoise{v + (threadIdx.x & 7u), p + (threadIdx.x & 31u)};
+}
+
+template <class Tab>
+RT_D float perlin_noise(const Tab& tab, float3 p) {
     float fx = floorf(p.x), fy = floorf(p.y), fz = floorf(p.z);
     float u = p.x - fx, v = p.y - fy, w = p.z - fz;
     u = u * u * (3.0f - 2.0f * u);
     v = v * v * (3.0f - 2.0f * v);
     w = w * w * (3.0f - 2.0f * w);
     int i = (int)fx, j = (int)fy, k = (int)fz;
+    const int pi[2] = {tab.perm(0, i & 255), tab.perm(0, (i + 1) & 255)};
+    const int pj[2] = {tab.perm(1, j & 255), tab.perm(1, (j + 1) & 255)};
+    const int pk[2] = {tab.perm(2, k & 255), tab.perm(2, (k + 1) & 255)};
     float accum = 0.0f;
 #pragma unroll
     for (int di = 0; di < 2; di++)
@@ -44,9 +81,7 @@ RT_D float perlin_noise(const float4* vec, const int32_t* perm, float3 p) {
         for (int dj = 0; dj < 2; dj++)
 #pragma unroll
             for (int dk = 0; dk < 2; dk++) {
-                int idx = (int)__ldg(perm + ((i + di) & 255)) ^ (int)__ldg(perm + 256 + ((j + dj) & 255)) ^
-                          (int)__ldg(perm + 512 + ((k + dk) & 255));
-                float4 c = __ldg(vec + idx);
+                float4 c = tab.vec(pi[di] ^ pj[dj] ^ pk[dk]);
                 float fi = (float)di, fj = (float)dj, fk = (float)dk;
                 float dt = c.x * (u - fi) + c.y * (v - fj) + c.z * (w - fk);
                 accum += (fi * u + (1.0f - fi) * (1.0f - u)) * (fj * v + (1.0f - fj) * (1.0f - v)) *
@@ -54,11 +89,12 @@ RT_D float perlin_noise(const float4* vec, const int32_t* perm, float3 p) {
             }
     return accum;
 }
-RT_D float medium_density_at(const DevMedium& m, float3 p) {
+template <class Tab>
+RT_D float medium_density_at(const DevMedium& m, const Tab& tab, float3 p) {
     float accum = 0.0f, weight = 1.0f;
     float3 q = p * m.noise_scale;
     for (int i = 0; i < 7; i++) {
-        accum += weight * perlin_noise(m.vec, m.perm, q);
+        accum += weight * perlin_noise(tab, q);
         weight *= 0.5f;
         q = mk(q.x * 2.0f, q.y * 2.0f, q.z * 2.0f);
     }
@@ -208,7 +244,8 @@ RT_D float grid_transmittance(const DevMedium& m, float3 o, float3 d, float a, f
 
 // scatter distance for t_max = ∞ (INFINITY when the ray leaves first);
 // delta tracking is bounded at 4096 steps
-RT_D float medium_sample(const DevMedium& m, float3 o, float3 d, float lam, float tmin) {
+template <class Tab>
+RT_D float medium_sample(const DevMedium& m, const Tab& tab, float3 o, float3 d, float lam, float tmin) {
     float t1, t2;
     if (!bound_hit(m, o, d, -INFINITY, INFINITY, &t1)) return INFINITY;
     if (!bound_hit(m, o, d, t1 + 0.0001f, INFINITY, &t2)) return INFINITY;
@@ -229,25 +266,30 @@ RT_D float medium_sample(const DevMedium& m, float3 o, float3 d, float lam, floa
     for (uint32_t k = 0; k < 4096u; k++) {
         t -= inv_maj * logf(fmaxf(medium_rnd(g, 2u * k), 1.1920928955078125e-07f));
         if (t >= t2) return INFINITY;
-        float dens = medium_density_at(m, ray_at(o, d, t));
+        float dens = medium_density_at(m, tab, ray_at(o, d, t));
         if (medium_rnd(g, 2u * k + 1u) < dens / m.density) return t;
     }
     return INFINITY;
 }
 
-// nearest medium event before tsurf: medium index or -1
-RT_D int media_event(const DevScene& S, float3 o, float3 d, float lam, float tmin, float tsurf, float* t_out) {
+// nearest medium event before tsurf: medium index or -1 (`sh`: the shared
+// tables of medium S.noise_medium, or null)
+RT_D int media_event(const DevScene& S, const SharedNoise* sh, float3 o, float3 d, float lam, float tmin, float tsurf,
+                     float* t_out) {
     int best = -1;
     float bt = tsurf;
     for (int mi = 0; mi < S.n_media; mi++) {
-        float t = medium_sample(S.media[mi], o, d, lam, tmin);
+        const DevMedium& m = S.media[mi];
+        float t = sh && mi == S.noise_medium ? medium_sample(m, *sh, o, d, lam, tmin)
+                                             : medium_sample(m, GlobalNoise{m.vec, m.perm}, o, d, lam, tmin);
         if (t < bt) { bt = t; best = mi; }
     }
     *t_out = bt;
     return best;
 }
 
-RT_D float medium_transmittance(const DevMedium& m, float3 o, float3 d, float tmin, float tmax) {
+template <class Tab>
+RT_D float medium_transmittance(const DevMedium& m, const Tab& tab, float3 o, float3 d, float tmin, float tmax) {
     float t1, t2;
     if (!bound_hit(m, o, d, -INFINITY, INFINITY, &t1)) return 1.0f;
     if (!bound_hit(m, o, d, t1 + 0.0001f, INFINITY, &t2)) return 1.0f;
@@ -260,15 +302,17 @@ RT_D float medium_transmittance(const DevMedium& m, float3 o, float3 d, float tm
     float seg_t = l / len, sum = 0.0f;
     for (int i = 0; i < 16; i++) {
         float t = a + seg_t * ((float)i + 0.5f) / 16.0f;
-        sum += medium_density_at(m, ray_at(o, d, t));
+        sum += medium_density_at(m, tab, ray_at(o, d, t));
     }
     return expf(-sum / 16.0f * l);
 }
 
-RT_D float media_transmittance(const DevScene& S, float3 o, float3 d, float tmin, float tmax) {
+RT_D float media_transmittance(const DevScene& S, const SharedNoise* sh, float3 o, float3 d, float tmin, float tmax) {
     float tr = 1.0f;
     for (int mi = 0; mi < S.n_media; mi++) {
-        tr *= medium_transmittance(S.media[mi], o, d, tmin, tmax);
+        const DevMedium& m = S.media[mi];
+        tr *= sh && mi == S.noise_medium ? medium_transmittance(m, *sh, o, d, tmin, tmax)
+                                         : medium_transmittance(m, GlobalNoise{m.vec, m.perm}, o, d, tmin, tmax);
         if (tr <= 0.0f) return 0.0f;
     }
     return tr;

@@ -57,7 +57,7 @@ RT_D float3 tex_value(const DevScene& S, int id, float u, float v, float3 p) {
         float acc = 0.0f, wgt = 1.0f;
         float3 q = mk(p.x * t.scale, p.y * t.scale, p.z * t.scale);
         for (int i = 0; i < 7; i++) {                                               // perlin.rs:61-71
-            acc += wgt * perlin_noise(t.vec, t.perm, q);
+            acc += wgt * perlin_noise(GlobalNoise{t.vec, t.perm}, q);
             wgt *= 0.5f;
             q = mk(q.x * 2.0f, q.y * 2.0f, q.z * 2.0f);
         }

@@ -769,8 +769,6 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) 
 
 // MODE 0: wavefront shadow rays (an occluded ray cancels its parked contribution)
 // MODE 1: API any-hit (occluded flags)
-// MODE 2: wavefront shadow rays in a scene with media (an unoccluded ray scales
-//         its parked contribution by the media's transmittance)
 template <int MODE, bool ANA, int NF>
 __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, true>()) k_any(DevScene S, PendTargets T, const float4* __restrict__ sq,
                                                         const float* __restrict__ rays, uint32_t n_api,
@@ -834,14 +832,6 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, true>()) k
                 if (MODE != 1) {
                     if (hit) {
                         T.pend[tag & 3u][tag >> 2] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    } else if (MODE == 2) {
-                        // world.transmittance (bvh.rs:532-575): the media scale what got through
-                        float tr = media_transmittance(S, o, d, tmin, tmax);
-                        if (tr < 1.0f) {
-                            float4* pp = T.pend[tag & 3u] + (tag >> 2);
-                            float4 v = *pp;
-                            *pp = make_float4(v.x * tr, v.y * tr, v.z * tr, v.w);
-                        }
                     }
                 } else {
                     out[item] = hit ? 1 : 0;
@@ -858,9 +848,16 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, true>()) k
 // ids follow the primitives: a tie goes to the surface).
 // MODE 0: wavefront paths (dense set, wavelength in meta.w)
 // MODE 1: photons (queued, wavelength in ray_d.w)
-template <int MODE>
-__global__ void k_media(DevScene S, PathState P, const uint32_t* __restrict__ queue, const uint32_t* count) {
+// NOISE: a noise medium's tables in the block's shared memory
+#define MEDIA_BLOCK 512
+template <int MODE, bool NOISE>
+__global__ void __launch_bounds__(MEDIA_BLOCK, 2) k_media(DevScene S, PathState P, const uint32_t* __restrict__ queue,
+                                                          const uint32_t* count) {
+    extern __shared__ __align__(16) unsigned char media_mem[];
     uint32_t n = *count;
+    if (blockIdx.x * blockDim.x >= n) return;             // uniform in the block
+    SharedNoise tab{nullptr, nullptr};
+    if (NOISE) tab = load_noise(S.media[S.noise_medium], media_mem);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t pid = MODE == 1 ? queue[i] : i;
         float4 ro = P.ray_o[pid], rd = P.ray_d[pid], hv = P.hit[pid];
@@ -869,8 +866,34 @@ __global__ void k_media(DevScene S, PathState P, const uint32_t* __restrict__ qu
         if (rtk::nan_ray(o, d, 0.001f, INFINITY)) continue;
         float tsurf = __float_as_uint(hv.x) == RT_MISS_REF ? INFINITY : hv.y;
         float tm;
-        int med = media_event(S, o, d, lam, 0.001f, tsurf, &tm);
+        int med = media_event(S, NOISE ? &tab : nullptr, o, d, lam, 0.001f, tsurf, &tm);
         if (med >= 0) P.hit[pid] = make_float4(__uint_as_float(RT_HIT_MEDIUM_BASE | (uint32_t)med), tm, 0.f, 0.f);
+    }
+}
+
+// The shadow rays of a scene with media, after the any-hit kernel: a ray whose
+// parked contribution was not cancelled scales it by the media's transmittance
+// (bvh.rs:532-575).  One thread per ray here; inside the traversal kernel the
+// transmittance (16 points × 7 octaves of noise) ran for the one or two lanes
+// that had just finished their rays while the rest of the warp waited.
+template <bool NOISE>
+__global__ void __launch_bounds__(MEDIA_BLOCK, 2) k_media_shadow(DevScene S, PendTargets T,
+                                                                 const float4* __restrict__ sq, const uint32_t* count) {
+    extern __shared__ __align__(16) unsigned char media_mem[];
+    const uint32_t n = *count;
+    if (blockIdx.x * blockDim.x >= n) return;             // uniform in the block
+    SharedNoise tab{nullptr, nullptr};
+    if (NOISE) tab = load_noise(S.media[S.noise_medium], media_mem);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 a = sq[(size_t)i * 2], b = sq[(size_t)i * 2 + 1];
+        const uint32_t tag = __float_as_uint(b.w);
+        float4* pp = T.pend[tag & 3u] + (tag >> 2);
+        const float4 v = *pp;
+        if (v.x == 0.0f && v.y == 0.0f && v.z == 0.0f) continue;
+        const float3 o = mk(a.x, a.y, a.z), d = mk(b.x, b.y, b.z);
+        if (rtk::nan_ray(o, d, 0.001f, a.w)) continue;
+        const float tr = media_transmittance(S, NOISE ? &tab : nullptr, o, d, 0.001f, a.w);
+        if (tr < 1.0f) *pp = make_float4(v.x * tr, v.y * tr, v.z * tr, v.w);
     }
 }
 
@@ -886,7 +909,7 @@ __global__ void k_media_api(DevScene S, const float* __restrict__ rays, uint32_t
         int4 h = out[i];
         float tsurf = h.x < 0 ? r[7] : __int_as_float(h.y);
         float tm;
-        int med = media_event(S, o, d, 550.0f, r[6], tsurf, &tm);
+        int med = media_event(S, nullptr, o, d, 550.0f, r[6], tsurf, &tm);
         if (med >= 0) out[i] = make_int4(n_prims + med, __float_as_int(tm), 0, 0);
     }
 }
@@ -898,7 +921,7 @@ __global__ void k_transmittance_api(DevScene S, const float* __restrict__ rays, 
         const float* r = rays + (size_t)i * 8;
         float3 o = mk(r[0], r[1], r[2]), d = mk(r[3], r[4], r[5]);
         float tr = (occ && occ[i]) ? 0.0f : 1.0f;
-        if (tr > 0.0f && S.n_media > 0 && !rtk::nan_ray(o, d, r[6], r[7])) tr = media_transmittance(S, o, d, r[6], r[7]);
+        if (tr > 0.0f && S.n_media > 0 && !rtk::nan_ray(o, d, r[6], r[7])) tr = media_transmittance(S, nullptr, o, d, r[6], r[7]);
         out[i] = tr;
     }
 }
@@ -1003,6 +1026,17 @@ int trace_format(const DevScene& S, bool caller_rays) {
             else                           RT_TRACE_ONE(K, MODE, false, RT_NODES_FULL, __VA_ARGS__);            \
         }                                                                                                       \
     } while (0)
+// the media kernels with (two 64 KB blocks per SM) or without shared noise tables
+#define RT_COMMA ,
+#define RT_MEDIA_LAUNCH(K, ARG, ...)                                                                              \
+    do {                                                                                                          \
+        if (S.noise_medium >= 0) {                                                                                \
+            cudaFuncSetAttribute(K<ARG true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_NOISE_SMEM);        \
+            K<ARG true><<<sms * 2, MEDIA_BLOCK, RT_NOISE_SMEM, st>>>(__VA_ARGS__);                                \
+        } else {                                                                                                  \
+            K<ARG false><<<sms * 2, MEDIA_BLOCK, 0, st>>>(__VA_ARGS__);                                           \
+        }                                                                                                         \
+    } while (0)
 void launch_trace_closest_api(const DevScene& S, const float* rays, uint32_t n, int4* out, uint32_t* next, int* err,
                               int sms, cudaStream_t st) {
     RT_TRACE_LAUNCH(k_closest, 1, S, PathState{}, nullptr, rays, n, nullptr, next, out, err);
@@ -1024,15 +1058,15 @@ void launch_extend(const DevScene& S, const PathState& P, const uint32_t* queue,
 }
 void launch_shadow(const DevScene& S, const PendTargets& T, const float4* sq, const uint32_t* count,
                    uint32_t* next, int* err, int sms, cudaStream_t st) {
-    if (S.n_media > 0) RT_TRACE_LAUNCH(k_any, 2, S, T, sq, nullptr, 0, count, next, nullptr, err);
-    else               RT_TRACE_LAUNCH(k_any, 0, S, T, sq, nullptr, 0, count, next, nullptr, err);
+    RT_TRACE_LAUNCH(k_any, 0, S, T, sq, nullptr, 0, count, next, nullptr, err);
+    if (S.n_media > 0) RT_MEDIA_LAUNCH(k_media_shadow, , S, T, sq, count);
 }
 #undef RT_TRACE_LAUNCH
 #undef RT_TRACE_ONE
 void launch_media(const DevScene& S, const PathState& P, const uint32_t* queue, const uint32_t* count, int sms,
                   cudaStream_t st) {
-    if (queue) k_media<1><<<sms * 8, 128, 0, st>>>(S, P, queue, count);
-    else       k_media<0><<<sms * 8, 128, 0, st>>>(S, P, nullptr, count);
+    if (queue) RT_MEDIA_LAUNCH(k_media, 1 RT_COMMA, S, P, queue, count);
+    else       RT_MEDIA_LAUNCH(k_media, 0 RT_COMMA, S, P, nullptr, count);
 }
 void launch_media_api(const DevScene& S, const float* rays, uint32_t n, int4* out, int32_t n_prims, int fill_miss,
                       int sms, cudaStream_t st) {
