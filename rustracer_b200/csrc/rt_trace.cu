@@ -686,6 +686,20 @@ template <int NF, bool ANA, bool ANY> constexpr int trace_minb() {
 }
 static_assert(RT_TRACE_MINB == 8, "the spill columns are sized for the most resident blocks");
 
+// Lanes of a warp that take rays: all of them — but in a scene with convex
+// solids, whose tests the warp runs one after the other (warp_convex), rays too
+// few to fill the grid's warps are spread over them, down to 4 a warp (gem room
+// 22.3 -> 21.0 ms: its 50 bounces end in many small launches).  Without such
+// solids the spread only keeps more warps busy beside the shadow rays and the
+// caustic lookup (gem 31.2 -> 31.9 ms).  Asked anew at each refill: no register
+// is kept for it.
+template <bool ANA>
+RT_D uint32_t warp_lanes(uint32_t n) {
+    const uint32_t warps = gridDim.x * (RT_TRACE_BLOCK / 32);
+    if (!ANA || n >= warps * 31u) return FULLMASK;
+    return (1u << max(4u, (n + warps - 1) / warps)) - 1u;
+}
+
 // MODE 0: wavefront extend (queue of path ids, rays in PathState, hits to PathState)
 // MODE 1: API (rays n×8 in memory, hits as int4)
 
@@ -712,11 +726,12 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) 
     while (true) {
         uint32_t idle = __ballot_sync(FULLMASK, !active);
         if (!exhausted && __popc(idle) >= RT_REFILL_CLOSEST) {
+            if (ANA) idle &= warp_lanes<ANA>(n);
             uint32_t k = __popc(idle), base = 0;
-            if (lane == 0) base = atomicAdd(next, k);
+            if (lane == 0 && (!ANA || k)) base = atomicAdd(next, k);
             base = __shfl_sync(FULLMASK, base, 0);
-            if (base + k >= n) exhausted = true;
-            if (!active) {
+            if ((!ANA || k) && base + k >= n) exhausted = true;
+            if (ANA ? (idle >> lane) & 1u : !active) {
                 uint32_t i = base + __popc(idle & lt);
                 if (i < n) {
                     item = i;
@@ -792,11 +807,12 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, true>()) k
     while (true) {
         uint32_t idle = __ballot_sync(FULLMASK, !active);
         if (!exhausted && __popc(idle) >= RT_REFILL) {
+            if (ANA) idle &= warp_lanes<ANA>(n);
             uint32_t k = __popc(idle), base = 0;
-            if (lane == 0) base = atomicAdd(next, k);
+            if (lane == 0 && (!ANA || k)) base = atomicAdd(next, k);
             base = __shfl_sync(FULLMASK, base, 0);
-            if (base + k >= n) exhausted = true;
-            if (!active) {
+            if ((!ANA || k) && base + k >= n) exhausted = true;
+            if (ANA ? (idle >> lane) & 1u : !active) {
                 uint32_t i = base + __popc(idle & lt);
                 if (i < n) {
                     item = i;
