@@ -247,11 +247,11 @@ void launch_shade(const rtd::DevScene& S, const PathState& A, const PathState& B
                   const RenderLaunch& R, uint32_t* ctr, const ClassQueues& Q, uint32_t* cout, float4* sq, int sms,
                   cudaStream_t st, const ShadeFork* fk = nullptr);
 // fold: write the ended paths' samples; refill: append new samples, one per
-// ended path while samples remain, to B, add the iteration's ray counts to the
-// header and clear the counter block of iteration it + 2
+// ended path while samples remain, to B; book (implied by refill): add the
+// iteration's ray counts to the header and clear the counter block of iteration it + 2
 void launch_retire(const rtd::DevScene& S, const PathState& B, const PathState& Rt, const RenderLaunch& R,
-                   uint32_t* ctr, uint32_t* hdr, uint32_t* clear_block, uint32_t* cout, bool fold, bool refill, int sms,
-                   cudaStream_t st);
+                   uint32_t* ctr, uint32_t* hdr, uint32_t* clear_block, uint32_t* cout, bool fold, bool refill, bool book,
+                   int grid, cudaStream_t st);
 // active-pixel list of a converged mask, and zero output for converged pixels
 void launch_active_list(const uint8_t* conv, uint32_t width, uint32_t height, uint32_t* list, uint32_t* count,
                         cudaStream_t st);

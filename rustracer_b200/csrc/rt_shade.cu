@@ -444,11 +444,12 @@ __global__ void k_generate(DevScene S, PathState A, const RenderLaunch* __restri
 // ended path the next ungenerated sample, if any, is appended to the next set.
 // Two halves, one launch each when the shadow rays run beside the next
 // extension rays (run_wavefront), both in one otherwise: REFILL hands out the
-// new samples and does the iteration's bookkeeping, which only needs the shading
-// kernels; FOLD writes the ended paths' samples and so needs the shadow rays
-// and the caustic lookup.
+// new samples, which only needs the shading kernels; FOLD writes the ended
+// paths' samples and so needs the shadow rays and the caustic lookup.  BOOK: the
+// launch that does the iteration's bookkeeping (once no sample is left to hand
+// out there is no refill, and the fold does it).
 #define RETIRE_BLOCK 256
-template <bool FOLD, bool REFILL>
+template <bool FOLD, bool REFILL, bool BOOK>
 __global__ void __launch_bounds__(RETIRE_BLOCK) k_retire(DevScene S, PathState B, PathState Rt,
                                                          const RenderLaunch* __restrict__ Rp, uint32_t* ctr,
                                                          uint32_t* hdr, uint32_t* clear_block, uint32_t* cout) {
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(RETIRE_BLOCK) k_retire(DevScene S, PathState B
     __shared__ BlockQ<1, RETIRE_BLOCK / 32> shq;
     __shared__ unsigned long long gbase;
     uint32_t n = ctr[CTR_RETIRE_COUNT];
-    if (REFILL && blockIdx.x == 0) {
+    if (BOOK && blockIdx.x == 0) {
         if (threadIdx.x == 0) {
             atomicAdd((unsigned long long*)(hdr + HDR_EXT), (unsigned long long)ctr[CTR_COUNT]);
             atomicAdd((unsigned long long*)(hdr + HDR_SHADOW), (unsigned long long)ctr[CTR_SHADOW_COUNT]);
@@ -1309,11 +1310,14 @@ void launch_shade(const DevScene& S, const PathState& A, const PathState& B, con
     for (int i = 0; i < nside; i++) cudaStreamWaitEvent(st, fk->join[i], 0);
 }
 void launch_retire(const DevScene& S, const PathState& B, const PathState& Rt, const RenderLaunch& R, uint32_t* ctr,
-                   uint32_t* hdr, uint32_t* clear_block, uint32_t* cout, bool fold, bool refill, int sms,
+                   uint32_t* hdr, uint32_t* clear_block, uint32_t* cout, bool fold, bool refill, bool book, int grid,
                    cudaStream_t st) {
-    if (fold && refill) k_retire<true, true><<<sms * 8, RETIRE_BLOCK, 0, st>>>(S, B, Rt, R.dev, ctr, hdr, clear_block, cout);
-    else if (fold)      k_retire<true, false><<<sms * 8, RETIRE_BLOCK, 0, st>>>(S, B, Rt, R.dev, ctr, hdr, clear_block, cout);
-    else                k_retire<false, true><<<sms * 8, RETIRE_BLOCK, 0, st>>>(S, B, Rt, R.dev, ctr, hdr, clear_block, cout);
+#define RT_RETIRE(F, N, K) k_retire<F, N, K><<<grid, RETIRE_BLOCK, 0, st>>>(S, B, Rt, R.dev, ctr, hdr, clear_block, cout)
+    if (fold && refill) RT_RETIRE(true, true, true);
+    else if (refill)    RT_RETIRE(false, true, true);
+    else if (book)      RT_RETIRE(true, false, true);
+    else                RT_RETIRE(true, false, false);
+#undef RT_RETIRE
 }
 void launch_active_list(const uint8_t* conv, uint32_t width, uint32_t height, uint32_t* list, uint32_t* count,
                         cudaStream_t st) {
