@@ -121,6 +121,14 @@ struct PendTargets {
 #define PF_TINT_MASK    (3u << 9)
 #define PF_SEC_ALIVE    (1u << 11)
 #define PF_REC_OPEN     (1u << 12)   // the newest guide record waits for its base radiance
+// parked contributions the path carries: without the bit the slot was not
+// written and is not read (a conductor or a miss parks none, most scenes use
+// one of the two); likewise thr, wts and L of a path at depth 0 are not stored:
+// they are (1, 1, 1, 1), the fresh weights and 0
+#define PF_PEND0        (1u << 13)
+#define PF_PEND1        (1u << 14)
+#define PF_PENDC        (1u << 15)
+#define PF_PEND_MASK    (PF_PEND0 | PF_PEND1 | PF_PENDC)
 
 namespace rtph { struct Map; }
 

@@ -374,10 +374,6 @@ RT_D void init_path(const DevScene& S, const PathState& P, const RenderLaunch& R
     uint32_t i = R.active ? __ldg(R.active + j) : tile_order_pixel(j, width, height);
     uint32_t row = i / width, col = i - row * width;
     uint32_t sample = sample0 + k;
-    P.L[pid] = make_float4(0.f, 0.f, 0.f, 0.f);
-    P.pend0[pid] = make_float4(0.f, 0.f, 0.f, 0.f);
-    P.pend1[pid] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (R.photons) P.pendC[pid] = make_float4(0.f, 0.f, 0.f, 0.f);
     Rng rng = make_rng(seed, i, sample);
     float wd = (float)max(width - 1u, 1u), hd = (float)max(height - 1u, 1u);
     uint32_t s2 = strata * strata, ray_y = height - 1u - row;
@@ -423,8 +419,6 @@ RT_D void init_path(const DevScene& S, const PathState& P, const RenderLaunch& R
     if (lam0 >= S.lam_lo + S.lam_range) lam0 = nextafterf(S.lam_lo + S.lam_range, 0.0f);
     P.ray_o[pid] = make_float4(o.x, o.y, o.z, 0.f);
     P.ray_d[pid] = make_float4(d.x, d.y, d.z, 0.f);
-    P.thr[pid] = make_float4(1.f, 1.f, 1.f, 1.f);
-    P.wts[pid] = make_float4(1.f, H > 1 ? 1.f : 0.f, H > 2 ? 1.f : 0.f, H > 3 ? 1.f : 0.f);
     P.meta[pid] = make_uint4(i, k, PF_PREV_SPEC | (H > 1 ? PF_SEC_ALIVE : 0u) | (job << PF_JOB_SHIFT),
                              __float_as_uint(lam0));
     if (R.guide.mode == 2) P.rec[pid] = rtg::REC_NONE;
@@ -469,11 +463,11 @@ __global__ void __launch_bounds__(RETIRE_BLOCK) k_retire(DevScene S, PathState B
         uint32_t j = t0 + threadIdx.x;
         bool act = j < n;
         if (FOLD && act) {
-            float4 L = Rt.L[j], a = Rt.pend0[j], b = Rt.pend1[j];
-            if (R.photons) { float4 c = Rt.pendC[j]; L.x += c.x; L.y += c.y; L.z += c.z; }
-            L.x += a.x; L.y += a.y; L.z += a.z;
-            L.x += b.x; L.y += b.y; L.z += b.z;
             uint4 meta = Rt.meta[j];
+            float4 L = Rt.L[j];
+            if (meta.z & PF_PENDC) { float4 c = Rt.pendC[j]; L.x += c.x; L.y += c.y; L.z += c.z; }
+            if (meta.z & PF_PEND0) { float4 a = Rt.pend0[j]; L.x += a.x; L.y += a.y; L.z += a.z; }
+            if (meta.z & PF_PEND1) { float4 b = Rt.pend1[j]; L.x += b.x; L.y += b.y; L.z += b.z; }
             float* out;
             if (R.n_jobs) {
                 const JobDev& J = R.jobs[meta.z >> PF_JOB_SHIFT];
@@ -744,11 +738,16 @@ k_shade(DevScene S, PathState A, PathState B, PathState Rt,
         uint32_t head = rtg::REC_NONE;   // newest guide record of the path
         if (active) {
             meta = A.meta[pid];
-            float4 thr = A.thr[pid], w = A.wts[pid], L = A.L[pid];
-            float4 p0 = A.pend0[pid], p1 = A.pend1[pid];
+            // a fresh path's throughput, weights and radiance are not stored, and of the
+            // parked contributions only those the last bounce made
+            float4 thr = make_float4(1.f, 1.f, 1.f, 1.f), L = zero4, p0 = zero4, p1 = zero4;
+            float4 w = make_float4(1.f, H > 1 ? 1.f : 0.f, H > 2 ? 1.f : 0.f, H > 3 ? 1.f : 0.f);
+            if (meta.z & PF_DEPTH_MASK) { thr = A.thr[pid]; w = A.wts[pid]; L = A.L[pid]; }
+            if (meta.z & PF_PEND0) p0 = A.pend0[pid];
+            if (meta.z & PF_PEND1) p1 = A.pend1[pid];
             // fold the previous bounce's parked contributions in the reference's
             // order: caustic injection, area-light NEE, env NEE (renderer.rs:461-540)
-            if (R.photons) {
+            if (meta.z & PF_PENDC) {
                 float4 pc = A.pendC[pid];
                 L.x += pc.x; L.y += pc.y; L.z += pc.z;
             }
@@ -1116,6 +1115,7 @@ k_shade(DevScene S, PathState A, PathState B, PathState Rt,
         // block-aggregated compaction: paths that go on into B, ended paths into
         // the retire records; parked contributions and shadow rays follow them
         bool ended = active && !cont;
+        meta.z = (meta.z & ~PF_PEND_MASK) | (sh0 ? PF_PEND0 : 0u) | (sh1 ? PF_PEND1 : 0u) | (gath ? PF_PENDC : 0u);
         uint32_t cnt[NQ], off[NQ];
         uint32_t slot = 0, rs = 0;
         if constexpr (NQ == 1) {
@@ -1132,12 +1132,16 @@ k_shade(DevScene S, PathState A, PathState B, PathState Rt,
         }
         if (cont) {
             B.ray_o[slot] = o_out; B.ray_d[slot] = d_out; B.thr[slot] = thr_out; B.wts[slot] = w_out;
-            B.meta[slot] = meta; B.L[slot] = Lout; B.pend0[slot] = np0; B.pend1[slot] = np1;
-            if (R.photons) B.pendC[slot] = npc;
+            B.meta[slot] = meta; B.L[slot] = Lout;
+            if (sh0) B.pend0[slot] = np0;
+            if (sh1) B.pend1[slot] = np1;
+            if (gath) B.pendC[slot] = npc;
             if (R.guide.mode == 2) B.rec[slot] = head;
         } else if (ended) {
-            Rt.meta[rs] = meta; Rt.L[rs] = Lout; Rt.pend0[rs] = np0; Rt.pend1[rs] = np1;
-            if (R.photons) Rt.pendC[rs] = npc;
+            Rt.meta[rs] = meta; Rt.L[rs] = Lout;
+            if (sh0) Rt.pend0[rs] = np0;
+            if (sh1) Rt.pend1[rs] = np1;
+            if (gath) Rt.pendC[rs] = npc;
             if (R.guide.mode == 2) Rt.rec[rs] = head;
         }
         if constexpr (NQ == 4) {
