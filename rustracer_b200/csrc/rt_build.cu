@@ -20,6 +20,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 #include "rt_internal.h"
@@ -46,6 +47,67 @@ __device__ __forceinline__ void unite6(float* a, const float* b) {
 __device__ __forceinline__ int bin_of(float c, float cmn, float ext) {
     float t = (c - cmn) / ext;
     return min((int)((float)NB * t), NB - 1);
+}
+
+// ── triangles ───────────────────────────────────────────────────────────────
+// The box of every triangle (triangle.rs:128-140: over v0, v0 + e1, v0 + e2,
+// padded as aabb.rs:18-29), the arithmetic of the host's boxes.
+__global__ void k_tri_boxes(const float* __restrict__ v, int32_t n, float* box) {
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float* p = v + (size_t)i * 9;
+        for (int a = 0; a < 3; a++) {
+            float c0 = p[a], c1 = c0 + (p[3 + a] - c0), c2 = c0 + (p[6 + a] - c0);
+            float mn = fminf(fminf(c0, c1), c2), mx = fmaxf(fmaxf(c0, c1), c2);
+            float pd = mx - mn < 0.0001f ? 0.0001f : 0.0f;
+            box[(size_t)i * 6 + a] = mn - pd;
+            box[(size_t)i * 6 + 3 + a] = mx + pd;
+        }
+    }
+}
+// the union of n boxes, as ordered-integer images (initialised by k_stats_init)
+__global__ void k_union_boxes(const float* __restrict__ box, int32_t n, int32_t* out) {
+    float v[6];
+    for (int k = 0; k < 3; k++) { v[k] = INFINITY; v[3 + k] = -INFINITY; }
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        for (int k = 0; k < 3; k++) {
+            v[k] = fminf(v[k], box[(size_t)i * 6 + k]);
+            v[3 + k] = fmaxf(v[3 + k], box[(size_t)i * 6 + 3 + k]);
+        }
+    for (int k = 0; k < 6; k++)
+        for (int o = 16; o > 0; o >>= 1) {
+            float x = __shfl_xor_sync(0xFFFFFFFFu, v[k], o);
+            v[k] = k < 3 ? fminf(v[k], x) : fmaxf(v[k], x);
+        }
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 6; k++) { if (k < 3) atomicMin(out + k, f2o(v[k])); else atomicMax(out + k, f2o(v[k])); }
+}
+// the triangle records in leaf order (rt_device.cuh) from the caller's arrays
+__global__ void k_tri_records(const int32_t* __restrict__ order, int32_t n, rth::RawTris T, float4* tri, float4* nrm,
+                              float4* uv, float4* tan) {
+    for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int32_t g = order[k];
+        const float* v = T.v + (size_t)g * 9;
+        float e1[3], e2[3];
+        for (int a = 0; a < 3; a++) { e1[a] = v[3 + a] - v[a]; e2[a] = v[6 + a] - v[a]; }
+        tri[(size_t)k * 3] = make_float4(v[0], v[1], v[2], e1[0]);
+        tri[(size_t)k * 3 + 1] = make_float4(e1[1], e1[2], e2[0], e2[1]);
+        tri[(size_t)k * 3 + 2] = make_float4(e2[2], __int_as_float(g), __int_as_float(T.mat[g]), __int_as_float(T.n ? 1 : 0));
+        if (T.n) {
+            const float* q = T.n + (size_t)g * 9;
+            nrm[(size_t)k * 3] = make_float4(q[0], q[1], q[2], q[3]);
+            nrm[(size_t)k * 3 + 1] = make_float4(q[4], q[5], q[6], q[7]);
+            nrm[(size_t)k * 3 + 2] = make_float4(q[8], 0.f, 0.f, 0.f);
+        }
+        if (T.uv) {
+            const float* u = T.uv + (size_t)g * 6;
+            const float* t = T.tan + (size_t)g * 9;
+            uv[(size_t)k * 2] = make_float4(u[0], u[1], u[2], u[3]);
+            uv[(size_t)k * 2 + 1] = make_float4(u[4], u[5], 0.f, 0.f);
+            tan[(size_t)k * 3] = make_float4(t[0], t[1], t[2], t[3]);
+            tan[(size_t)k * 3 + 1] = make_float4(t[4], t[5], t[6], t[7]);
+            tan[(size_t)k * 3 + 2] = make_float4(t[8], 0.f, 0.f, 0.f);
+        }
+    }
 }
 
 // node statistics: box (6), centroid bounds (6), then per axis per bin a count
@@ -1031,11 +1093,18 @@ cudaError_t pack_nodes(const rtd::DevScene& S, const float4* in, int64_t n_nodes
     return e;
 }
 
-// Build the binary SAH tree of n primitive boxes (host, 6 floats each) on the
-// device; idx (n), bl / br (n − 1 child refs: ≥ 0 node, < 0 leaf −(pos + 1))
+void launch_tri_records(const int32_t* order, int32_t n, const RawTris& T, float4* tri, float4* nrm, float4* uv,
+                        float4* tan, int sms, cudaStream_t st) {
+    k_tri_records<<<std::max(1, std::min((n + 255) / 256, sms * 8)), 256, 0, st>>>(order, n, T, tri, nrm, uv, tan);
+}
+
+// Build the binary SAH tree of n primitive boxes on the device: those of the
+// first n_tris from the triangles tri_v (device, 9 floats each; their union goes
+// to tri_bounds), the others from boxes_h (host, 6 floats each); idx (n), bl / br (n − 1 child refs: ≥ 0 node, < 0 leaf −(pos + 1))
 // and bbox ((n − 1) × 6) are written on the host.  Returns 0 or a CUDA error.
-int gpu_build_binary(const float* boxes_h, int32_t n, int32_t* idx_h, int32_t* bl_h, int32_t* br_h, float* bbox_h,
-                     int32_t* root_h, int sms, cudaStream_t st, WideOut* wide) {
+int gpu_build_binary(const float* boxes_h, const float* tri_v, int32_t n_tris, float* tri_bounds, int32_t n,
+                     int32_t* idx_h, int32_t* bl_h, int32_t* br_h, float* bbox_h, int32_t* root_h, int sms,
+                     cudaStream_t st, WideOut* wide) {
     float *box = nullptr, *cen = nullptr, *bbox = nullptr;
     int32_t *idx = nullptr, *tmp = nullptr, *bl = nullptr, *br = nullptr, *root = nullptr, *cnt = nullptr;
     int32_t *stats = nullptr, *mids = nullptr, *axes = nullptr, *chunk_seg = nullptr, *chunk_lo = nullptr;
@@ -1059,7 +1128,21 @@ int gpu_build_binary(const float* boxes_h, int32_t n, int32_t* idx_h, int32_t* b
     ok(cudaMalloc(&small, ((size_t)n / 2 + 2) * sizeof(Seg)));
     ok(cudaMalloc(&beg, max_segs * 4)); ok(cudaMalloc(&end, max_segs * 4));
     if (e == cudaSuccess) {
-        ok(cudaMemcpyAsync(box, boxes_h, (size_t)n * 24, cudaMemcpyHostToDevice, st));
+        if (n > n_tris)
+            ok(cudaMemcpyAsync(box + (size_t)n_tris * 6, boxes_h, (size_t)(n - n_tris) * 24, cudaMemcpyHostToDevice, st));
+        if (n_tris > 0) {
+            const int g = std::max(1, std::min((n_tris + 255) / 256, sms * 8));
+            k_tri_boxes<<<g, 256, 0, st>>>(tri_v, n_tris, box);
+            k_stats_init<<<1, 256, 0, st>>>(stats, 1);
+            k_union_boxes<<<g, 256, 0, st>>>(box, n_tris, stats);
+            int32_t u[6];
+            ok(cudaMemcpyAsync(u, stats, sizeof(u), cudaMemcpyDeviceToHost, st));
+            ok(cudaStreamSynchronize(st));
+            for (int k = 0; k < 6; k++) {
+                int32_t b = u[k] >= 0 ? u[k] : u[k] ^ 0x7FFFFFFF;
+                memcpy(tri_bounds + k, &b, 4);
+            }
+        }
         k_centroids<<<sms * 8, 256, 0, st>>>(box, n, cen, idx);
         ok(cudaMemsetAsync(cnt, 0, 8, st));
         ok(cudaMemsetAsync(root, 0, 4, st));

@@ -296,10 +296,17 @@ struct WideOut {
     int64_t n_nodes4 = 0;
     int32_t max_depth4 = 0;
 };
+// the caller's triangle arrays on the device (normals, texture coordinates and tangents may be null)
+struct RawTris { const float *v, *n, *uv, *tan; const int32_t* mat; };
+// triangle records in leaf order: record k from triangle order[k]
+void launch_tri_records(const int32_t* order, int32_t n, const RawTris& T, float4* tri, float4* nrm, float4* uv,
+                        float4* tan, int sms, cudaStream_t st);
 // binary tree on the device, then (wide == null) its arrays copied to the host
-// or (wide != null) the device collapse into *wide
-int gpu_build_binary(const float* boxes_h, int32_t n, int32_t* idx_h, int32_t* bl_h, int32_t* br_h, float* bbox_h,
-                     int32_t* root_h, int sms, cudaStream_t st, WideOut* wide = nullptr);
+// or (wide != null) the device collapse into *wide; the first n_tris primitives
+// are the triangles tri_v (device), the others have boxes_h (host)
+int gpu_build_binary(const float* boxes_h, const float* tri_v, int32_t n_tris, float* tri_bounds, int32_t n,
+                     int32_t* idx_h, int32_t* bl_h, int32_t* br_h, float* bbox_h, int32_t* root_h, int sms,
+                     cudaStream_t st, WideOut* wide = nullptr);
 // the packed nodes the traversal reads, from a reference-layout tree of n
 // nodes of `width` 8 or 4 and its leaves (see rt_build.cu); qout: the
 // quantised copy too (8-wide)
