@@ -13,10 +13,9 @@
 //
 // Large nodes are split level by level: atomics (order-independent min / max
 // and counts) gather the node box, centroid bounds and bin statistics, one
-// thread per node chooses the split, and a segmented stable radix sort by bin
-// reorders the primitives.  Nodes below SMALL primitives are finished by one
-// warp each.  Compiled without FMA
-// contraction so every comparison sees the host's values.
+// thread per node chooses the split, and a stable counting sort by bin reorders
+// the primitives.  Nodes below SMALL primitives are finished by one warp each.
+// Compiled without FMA contraction so every comparison sees the host's values.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -32,6 +31,29 @@ constexpr int SMALL = 192;       // nodes below this many primitives: one warp
 constexpr int CHUNK = 4096;      // primitives per block in the level kernels
 
 struct Seg { int32_t lo, hi, parent, side; };   // side 0: parent's left child, 1: right, −1: root
+
+// Scratch of one call: one allocation cut into 256-byte aligned parts.  A build
+// made 33 scratch allocations and as many releases, driver calls of 0.1-0.3 ms
+// each once they are large (327,680 triangles: 20.3 ms a build, of 4.7 ms in
+// kernels; 7.2 ms with one allocation per call, one copy each way per level and
+// k_scatter's sort).
+struct Arena {
+    void* base = nullptr;
+    size_t total = 0;
+    std::vector<std::pair<void**, size_t>> parts;
+    template <typename T>
+    void part(T** p, size_t bytes) {
+        parts.push_back({(void**)p, total});
+        total += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+    }
+    cudaError_t open() {
+        cudaError_t e = cudaMalloc(&base, total);
+        if (e != cudaSuccess) { base = nullptr; return e; }
+        for (auto& q : parts) *q.first = (char*)base + q.second;
+        return e;
+    }
+    ~Arena() { if (base) cudaFree(base); }
+};
 
 // ordered-integer images of floats for atomicMin / atomicMax
 __device__ __forceinline__ int f2o(float f) { int i = __float_as_int(f); return i >= 0 ? i : i ^ 0x7FFFFFFF; }
@@ -309,15 +331,95 @@ __global__ void k_split(const Seg* __restrict__ segs, int32_t nseg, const int32_
 __global__ void k_keys(const Seg* __restrict__ segs, const int32_t* __restrict__ chunk_seg,
                        const int32_t* __restrict__ chunk_lo, int32_t nchunks, const int32_t* __restrict__ idx,
                        const float* __restrict__ cen, const int32_t* __restrict__ st, const int32_t* __restrict__ axes,
-                       uint8_t* keys) {
+                       uint8_t* keys, int32_t* hist) {
+    __shared__ int32_t cnt[NB];
     for (int32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        if (threadIdx.x < NB) cnt[threadIdx.x] = 0;
+        __syncthreads();
         int32_t s = chunk_seg[c];
         int ax = axes[s];
         const int32_t* g = st + (size_t)s * ST_WORDS;
         float cmn = ax >= 0 ? o2f(g[6 + ax]) : 0.0f, ext = ax >= 0 ? o2f(g[9 + ax]) - cmn : 1.0f;
         int32_t lo = chunk_lo[c], hi = min(lo + CHUNK, segs[s].hi);
-        for (int32_t k = lo + threadIdx.x; k < hi; k += blockDim.x)
-            keys[k] = ax >= 0 ? (uint8_t)bin_of(cen[(size_t)idx[k] * 3 + ax], cmn, ext) : (uint8_t)0;
+        for (int32_t k = lo + threadIdx.x; k < hi; k += blockDim.x) {
+            int b = ax >= 0 ? bin_of(cen[(size_t)idx[k] * 3 + ax], cmn, ext) : 0;
+            keys[k] = (uint8_t)b;
+            atomicAdd(&cnt[b], 1);
+        }
+        __syncthreads();
+        if (threadIdx.x < NB) hist[(size_t)threadIdx.x * nchunks + c] = cnt[threadIdx.x];
+        __syncthreads();
+    }
+}
+
+// The stable sort of every large node's primitives by bin: k_keys counts each
+// chunk's bins, k_offsets turns the counts into first positions (one block per
+// node, one warp per bin, the node's chunks first[s] .. first[s + 1]), k_scatter
+// places the chunk's primitives in order.  A segmented radix sort gives a node to
+// one block, so the first levels ran on one, two, four ... of 148 SMs
+// (327,680 triangles: 1.12 ms of sorting; 0.23 ms here).
+__global__ void __launch_bounds__(NB * 32) k_offsets(const Seg* __restrict__ segs, const int32_t* __restrict__ first,
+                                                     int32_t nchunks, int32_t* hist) {
+    __shared__ int32_t tot[NB];
+    const int32_t s = blockIdx.x, b = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int32_t c0 = first[s], c1 = first[s + 1];
+    int32_t* h = hist + (size_t)b * nchunks;
+    int32_t sum = 0;
+    for (int32_t c = c0 + lane; c < c1; c += 32) sum += h[c];
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    if (lane == 0) tot[b] = sum;
+    __syncthreads();
+    int32_t run = segs[s].lo;
+    for (int q = 0; q < b; q++) run += tot[q];
+    for (int32_t c = c0; c < c1; c += 32) {
+        int32_t v = c + lane < c1 ? h[c + lane] : 0, x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            int32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (c + lane < c1) h[c + lane] = run + x - v;
+        run += __shfl_sync(0xFFFFFFFFu, x, 31);
+    }
+}
+constexpr int SCATTER_WARPS = 8, SCATTER_RUN = CHUNK / SCATTER_WARPS;   // consecutive primitives per warp
+__global__ void __launch_bounds__(SCATTER_WARPS * 32)
+k_scatter(const Seg* __restrict__ segs, const int32_t* __restrict__ chunk_seg, const int32_t* __restrict__ chunk_lo,
+          int32_t nchunks, const int32_t* __restrict__ hist, const uint8_t* __restrict__ keys,
+          const int32_t* __restrict__ from, int32_t* to) {
+    __shared__ int32_t at[SCATTER_WARPS][NB + 1];   // [NB]: lanes past the chunk's end
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t below = (1u << lane) - 1u;
+    for (int32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        if (lane <= NB) at[w][lane] = 0;
+        __syncwarp();
+        const int32_t lo = chunk_lo[c] + w * SCATTER_RUN, hi = min(chunk_lo[c] + CHUNK, segs[chunk_seg[c]].hi);
+        for (int i = 0; i < SCATTER_RUN; i += 32) {
+            const int32_t k = lo + i + lane;
+            const int b = k < hi ? keys[k] : NB;
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, b);
+            if (!(peers & below)) at[w][b] += __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        if (threadIdx.x < NB) {
+            int32_t run = hist[(size_t)threadIdx.x * nchunks + c];
+            for (int q = 0; q < SCATTER_WARPS; q++) {
+                int32_t v = at[q][threadIdx.x];
+                at[q][threadIdx.x] = run;
+                run += v;
+            }
+        }
+        __syncthreads();
+        for (int i = 0; i < SCATTER_RUN; i += 32) {
+            const int32_t k = lo + i + lane;
+            const int b = k < hi ? keys[k] : NB;
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, b);
+            if (k < hi) to[at[w][b] + __popc(peers & below)] = from[k];
+            __syncwarp();
+            if (!(peers & below)) at[w][b] += __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
     }
 }
 
@@ -935,20 +1037,17 @@ static cudaError_t collapse_wide(const int32_t* bl, const int32_t* br, const flo
     auto scan = [&](const int32_t* in, int32_t* out, int32_t m) {
         size_t need = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, need, in, out, m, st);
-        if (need > tmp_bytes) {
-            if (tmp) cudaFree(tmp);
-            tmp = nullptr;
-            if (!ok(cudaMalloc(&tmp, need))) return;
-            tmp_bytes = need;
-        }
+        if (need > tmp_bytes) { ok(cudaErrorMemoryAllocation); return; }   // m ≤ n: never
         ok(cub::DeviceScan::ExclusiveSum(tmp, need, in, out, m, st));
     };
-    ok(cudaMalloc(&kids, (size_t)nn * 8 * 4)); ok(cudaMalloc(&nk, (size_t)nn * 4));
-    ok(cudaMalloc(&order, ((size_t)nn + 1) * 4)); ok(cudaMalloc(&cnt, ((size_t)nn + 1) * 4));
-    ok(cudaMalloc(&pos, ((size_t)nn + 1) * 4));
-    ok(cudaMalloc(&S, (size_t)nn * 4)); ok(cudaMalloc(&L, (size_t)nn * 4));
-    ok(cudaMalloc(&P, (size_t)nn * 4)); ok(cudaMalloc(&LB, (size_t)nn * 4));
-    ok(cudaMalloc(&leaf_gid, (size_t)n * 4)); ok(cudaMalloc(&flags, (size_t)n * 16)); ok(cudaMalloc(&scans, (size_t)n * 16));
+    cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, cnt, pos, n, st);
+    Arena A;
+    A.part(&kids, (size_t)nn * 8 * 4); A.part(&nk, (size_t)nn * 4);
+    A.part(&order, ((size_t)nn + 1) * 4); A.part(&cnt, ((size_t)nn + 1) * 4); A.part(&pos, ((size_t)nn + 1) * 4);
+    A.part(&S, (size_t)nn * 4); A.part(&L, (size_t)nn * 4); A.part(&P, (size_t)nn * 4); A.part(&LB, (size_t)nn * 4);
+    A.part(&leaf_gid, (size_t)n * 4); A.part(&flags, (size_t)n * 16); A.part(&scans, (size_t)n * 16);
+    A.part(&tmp, tmp_bytes);
+    ok(A.open());
     int grid = sms * 8;
     std::vector<int32_t> lvl_off;
     // the wide nodes of one width: each binary node's opening, the wide roots
@@ -1028,8 +1127,6 @@ static cudaError_t collapse_wide(const int32_t* bl, const int32_t* br, const flo
             ok(cudaGetLastError());
         }
     }
-    void* all[] = {kids, nk, order, cnt, pos, S, L, P, LB, leaf_gid, flags, scans, tmp};
-    for (void* p : all) if (p) cudaFree(p);
     if (e != cudaSuccess) {
         void* outs[] = {W->nodes, W->export_ch, W->nodes4};
         for (void* p : outs) if (p) cudaFree(p);
@@ -1055,9 +1152,11 @@ cudaError_t pack_nodes(const rtd::DevScene& S, const float4* in, int64_t n_nodes
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t r) { if (e == cudaSuccess && r != cudaSuccess) e = r; return e == cudaSuccess; };
     cub::DeviceScan::ExclusiveSum(nullptr, need, cnt, base, n, st);
-    ok(cudaMalloc(&slots, (size_t)n * 4)); ok(cudaMalloc(&cnt, (size_t)n * 8)); ok(cudaMalloc(&base, (size_t)n * 8));
+    Arena A;
+    A.part(&slots, (size_t)n * 4); A.part(&cnt, (size_t)n * 8); A.part(&base, (size_t)n * 8);
+    A.part(&index, (size_t)n * 4); A.part(&fail, 4); A.part(&tmp, need);
+    ok(A.open());
     ok(cudaMalloc((void**)&lout->rec, (size_t)n_leaves * 48)); ok(cudaMalloc((void**)&lout->box, (size_t)n_leaves * 32));
-    ok(cudaMalloc(&index, (size_t)n * 4)); ok(cudaMalloc(&fail, 4)); ok(cudaMalloc(&tmp, std::max<size_t>(need, 16)));
     ok(cudaMalloc(out, (size_t)n * (width == 8 ? RT_NODE_F4 : RT_NODE4_F4) * 16));
     if (qout) ok(cudaMalloc(qout, (size_t)n * RT_QNODE_F4 * 16));
     if (e == cudaSuccess) {
@@ -1080,8 +1179,6 @@ cudaError_t pack_nodes(const rtd::DevScene& S, const float4* in, int64_t n_nodes
         ok(cudaGetLastError());
         if (e == cudaSuccess && hfail && qout) { cudaFree(*qout); *qout = nullptr; }
     }
-    void* all[] = {slots, cnt, base, index, fail, tmp};
-    for (void* p : all) if (p) cudaFree(p);
     if (e != cudaSuccess) {
         if (*out) cudaFree(*out);
         if (lout->rec) cudaFree((void*)lout->rec);
@@ -1100,33 +1197,32 @@ void launch_tri_records(const int32_t* order, int32_t n, const RawTris& T, float
 
 // Build the binary SAH tree of n primitive boxes on the device: those of the
 // first n_tris from the triangles tri_v (device, 9 floats each; their union goes
-// to tri_bounds), the others from boxes_h (host, 6 floats each); idx (n), bl / br (n − 1 child refs: ≥ 0 node, < 0 leaf −(pos + 1))
-// and bbox ((n − 1) × 6) are written on the host.  Returns 0 or a CUDA error.
+// to tri_bounds), the others from boxes_h (host, 6 floats each);
+// idx (n), bl / br (n − 1 child refs: ≥ 0 node, < 0 leaf −(pos + 1)) and bbox ((n − 1) × 6) are written on the host.  Returns 0 or a CUDA error.
 int gpu_build_binary(const float* boxes_h, const float* tri_v, int32_t n_tris, float* tri_bounds, int32_t n,
                      int32_t* idx_h, int32_t* bl_h, int32_t* br_h, float* bbox_h, int32_t* root_h, int sms,
                      cudaStream_t st, WideOut* wide) {
     float *box = nullptr, *cen = nullptr, *bbox = nullptr;
     int32_t *idx = nullptr, *tmp = nullptr, *bl = nullptr, *br = nullptr, *root = nullptr, *cnt = nullptr;
-    int32_t *stats = nullptr, *mids = nullptr, *axes = nullptr, *chunk_seg = nullptr, *chunk_lo = nullptr;
-    uint8_t *keys = nullptr, *keys2 = nullptr;
-    Seg *cur = nullptr, *nxt = nullptr, *small = nullptr;
-    int32_t *beg = nullptr, *end = nullptr;
-    void* cub_tmp = nullptr;
-    size_t cub_bytes = 0;
+    int32_t *stats = nullptr, *mids = nullptr, *axes = nullptr;
+    uint8_t* keys = nullptr;
+    Seg *nxt = nullptr, *small = nullptr;
+    int32_t *lvl = nullptr, *hist = nullptr;
     int32_t nn = std::max(n - 1, 1);
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t r) { if (e == cudaSuccess && r != cudaSuccess) e = r; return e == cudaSuccess; };
     size_t max_chunks = (size_t)n / CHUNK + (size_t)n / SMALL + 2;
     size_t max_segs = (size_t)n / SMALL + 2;
-    ok(cudaMalloc(&box, (size_t)n * 24)); ok(cudaMalloc(&cen, (size_t)n * 12)); ok(cudaMalloc(&bbox, (size_t)nn * 24));
-    ok(cudaMalloc(&idx, (size_t)n * 4)); ok(cudaMalloc(&tmp, (size_t)n * 4));
-    ok(cudaMalloc(&bl, (size_t)nn * 4)); ok(cudaMalloc(&br, (size_t)nn * 4)); ok(cudaMalloc(&root, 4));
-    ok(cudaMalloc(&cnt, 8)); ok(cudaMalloc(&keys, (size_t)n)); ok(cudaMalloc(&keys2, (size_t)n));
-    ok(cudaMalloc(&stats, max_segs * ST_WORDS * 4)); ok(cudaMalloc(&mids, max_segs * 4)); ok(cudaMalloc(&axes, max_segs * 4));
-    ok(cudaMalloc(&chunk_seg, max_chunks * 4)); ok(cudaMalloc(&chunk_lo, max_chunks * 4));
-    ok(cudaMalloc(&cur, max_segs * sizeof(Seg))); ok(cudaMalloc(&nxt, max_segs * sizeof(Seg)));
-    ok(cudaMalloc(&small, ((size_t)n / 2 + 2) * sizeof(Seg)));
-    ok(cudaMalloc(&beg, max_segs * 4)); ok(cudaMalloc(&end, max_segs * 4));
+    Arena A;
+    A.part(&box, (size_t)n * 24); A.part(&cen, (size_t)n * 12); A.part(&bbox, (size_t)nn * 24);
+    A.part(&idx, (size_t)n * 4); A.part(&tmp, (size_t)n * 4);
+    A.part(&bl, (size_t)nn * 4); A.part(&br, (size_t)nn * 4); A.part(&root, 4);
+    A.part(&keys, (size_t)n);
+    A.part(&stats, max_segs * ST_WORDS * 4); A.part(&mids, max_segs * 4); A.part(&axes, max_segs * 4);
+    A.part(&lvl, (5 * max_segs + 1 + 2 * max_chunks) * 4); A.part(&hist, max_chunks * NB * 4);
+    A.part(&cnt, 16 + max_segs * sizeof(Seg));
+    A.part(&small, ((size_t)n / 2 + 2) * sizeof(Seg));
+    ok(A.open());
     if (e == cudaSuccess) {
         if (n > n_tris)
             ok(cudaMemcpyAsync(box + (size_t)n_tris * 6, boxes_h, (size_t)(n - n_tris) * 24, cudaMemcpyHostToDevice, st));
@@ -1160,48 +1256,42 @@ int gpu_build_binary(const float* boxes_h, const float* tri_v, int32_t n_tris, f
     } else {
         level.push_back(r0);
     }
-    std::vector<int32_t> cs, cl, bh, eh;
+    // a level's nodes, each node's first chunk and the chunks' nodes and starts
+    // go to the device in one copy; its children come back in one
+    nxt = (Seg*)(cnt + 4);
+    std::vector<int32_t> up, down;
     while (e == cudaSuccess && !level.empty()) {
-        int32_t ns = (int32_t)level.size();
-        cs.clear(); cl.clear(); bh.clear(); eh.clear();
-        for (int32_t s = 0; s < ns; s++) {
-            for (int32_t lo = level[s].lo; lo < level[s].hi; lo += CHUNK) { cs.push_back(s); cl.push_back(lo); }
-            bh.push_back(level[s].lo); eh.push_back(level[s].hi);
-        }
-        int32_t nch = (int32_t)cs.size();
-        ok(cudaMemcpyAsync(cur, level.data(), ns * sizeof(Seg), cudaMemcpyHostToDevice, st));
-        ok(cudaMemcpyAsync(chunk_seg, cs.data(), nch * 4, cudaMemcpyHostToDevice, st));
-        ok(cudaMemcpyAsync(chunk_lo, cl.data(), nch * 4, cudaMemcpyHostToDevice, st));
-        ok(cudaMemcpyAsync(beg, bh.data(), ns * 4, cudaMemcpyHostToDevice, st));
-        ok(cudaMemcpyAsync(end, eh.data(), ns * 4, cudaMemcpyHostToDevice, st));
+        int32_t ns = (int32_t)level.size(), nch = 0;
+        up.resize((size_t)ns * 5 + 1);
+        memcpy(up.data(), level.data(), (size_t)ns * sizeof(Seg));
+        for (int32_t s = 0; s < ns; s++) { up[(size_t)ns * 4 + s] = nch; nch += (level[s].hi - level[s].lo + CHUNK - 1) / CHUNK; }
+        up[(size_t)ns * 5] = nch;
+        up.resize((size_t)ns * 5 + 1 + 2 * (size_t)nch);
+        int32_t* q = up.data() + (size_t)ns * 5 + 1;
+        for (int32_t s = 0; s < ns; s++)
+            for (int32_t lo = level[s].lo; lo < level[s].hi; lo += CHUNK, q++) { q[0] = s; q[nch] = lo; }
+        ok(cudaMemcpyAsync(lvl, up.data(), up.size() * 4, cudaMemcpyHostToDevice, st));
+        const Seg* cur = (const Seg*)lvl;
+        const int32_t *first = lvl + (size_t)ns * 4, *chunk_seg = first + ns + 1, *chunk_lo = chunk_seg + nch;
         int grid = std::min(nch, sms * 16);
         k_stats_init<<<std::min((ns * ST_WORDS + 255) / 256, sms * 8), 256, 0, st>>>(stats, ns);
         k_stats_bounds<<<grid, 256, 0, st>>>(cur, chunk_seg, chunk_lo, nch, idx, box, cen, stats);
         k_stats_bins<<<grid, 256, 0, st>>>(cur, chunk_seg, chunk_lo, nch, idx, box, cen, stats);
         k_split<<<(ns + 127) / 128, 128, 0, st>>>(cur, ns, stats, mids, axes, bl, br, root, bbox);
-        k_keys<<<grid, 256, 0, st>>>(cur, chunk_seg, chunk_lo, nch, idx, cen, stats, axes, keys);
-        // stable sort of every large node's primitives by bin (the counting sort)
-        size_t need = 0;
-        cub::DeviceSegmentedRadixSort::SortPairs(nullptr, need, keys, keys2, idx, tmp, n, ns, beg, end, 0, 4, st);
-        if (need > cub_bytes) {
-            if (cub_tmp) cudaFree(cub_tmp);
-            cub_tmp = nullptr;
-            if (!ok(cudaMalloc(&cub_tmp, need))) break;
-            cub_bytes = need;
-        }
-        ok(cub::DeviceSegmentedRadixSort::SortPairs(cub_tmp, need, keys, keys2, idx, tmp, n, ns, beg, end, 0, 4, st));
+        k_keys<<<grid, 256, 0, st>>>(cur, chunk_seg, chunk_lo, nch, idx, cen, stats, axes, keys, hist);
+        k_offsets<<<ns, NB * 32, 0, st>>>(cur, first, nch, hist);
+        k_scatter<<<grid, SCATTER_WARPS * 32, 0, st>>>(cur, chunk_seg, chunk_lo, nch, hist, keys, idx, tmp);
         k_copy_back<<<grid, 256, 0, st>>>(cur, chunk_seg, chunk_lo, nch, tmp, idx);
-        ok(cudaMemsetAsync(cnt, 0, 4, st));
+        ok(cudaMemsetAsync(cnt, 0, 8, st));
         LevelOut out{nxt, cnt, small + n_small, cnt + 1};
         k_children<<<(ns + 127) / 128, 128, 0, st>>>(cur, ns, mids, box, idx, bl, br, root, bbox, out);
-        int32_t counts[2];
-        ok(cudaMemcpyAsync(counts, cnt, 8, cudaMemcpyDeviceToHost, st));
+        down.resize(4 + std::min(2 * (size_t)ns, max_segs) * 4);
+        ok(cudaMemcpyAsync(down.data(), cnt, down.size() * 4, cudaMemcpyDeviceToHost, st));
         ok(cudaStreamSynchronize(st));
-        ok(cudaMemsetAsync(cnt + 1, 0, 4, st));
-        n_small += counts[1];
-        level.resize(counts[0]);
-        if (counts[0]) ok(cudaMemcpyAsync(level.data(), nxt, counts[0] * sizeof(Seg), cudaMemcpyDeviceToHost, st));
-        ok(cudaStreamSynchronize(st));
+        if (e != cudaSuccess) break;
+        n_small += down[1];
+        level.resize(down[0]);
+        memcpy(level.data(), down.data() + 4, (size_t)down[0] * sizeof(Seg));
     }
     if (e == cudaSuccess && n_small > 0)
     {
@@ -1231,9 +1321,6 @@ int gpu_build_binary(const float* boxes_h, const float* tri_v, int32_t n_tris, f
         ok(cudaMemcpyAsync(root_h, root, 4, cudaMemcpyDeviceToHost, st));
         ok(cudaStreamSynchronize(st));
     }
-    void* all[] = {box, cen, bbox, idx, tmp, bl, br, root, cnt, keys, keys2, stats, mids, axes, chunk_seg, chunk_lo,
-                   cur, nxt, small, beg, end, cub_tmp};
-    for (void* p : all) if (p) cudaFree(p);
     return (int)e;
 }
 
