@@ -320,7 +320,26 @@ void launch_develop(const float* lin, const float* sum, const uint32_t* cnt, uin
 }  // namespace rth
 
 // host state of the path-guiding network (rt_guide.cu)
+#include <future>
 #include <string>
+namespace rth {
+// f(0) … f(n − 1), n ≤ 16, each on a thread of its own where one can be had
+template <typename F>
+void on_threads(int n, F&& f) {
+    std::future<void> job[16];
+    for (int w = 1; w < n; w++) {
+        try {
+            job[w] = std::async([&f, w] { f(w); });    // without a thread: runs in get()
+        } catch (...) {
+        }
+    }
+    f(0);
+    for (int w = 1; w < n; w++) {
+        if (job[w].valid()) job[w].get();
+        else f(w);
+    }
+}
+}  // namespace rth
 namespace rtgh {
 struct Guide;
 Guide* create(const RtGuideParams& p, const float scene_lo[3], const float scene_hi[3], std::string* err);
