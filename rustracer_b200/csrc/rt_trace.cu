@@ -674,6 +674,11 @@ RT_D bool nan_ray(float3 o, float3 d, float tmin, float tmax) {
 #ifndef RT_REFILL_CLOSEST
 #define RT_REFILL_CLOSEST 24
 #endif
+// with split leaves (below) the idle lanes are dearer: 4M caller rays 1.42 -> 1.34
+// ms at 16, 1.43 at 20, 1.48 at 28; icosphere extend 12.54 -> 12.45, 12.39, 13.09
+#ifndef RT_REFILL_SPLIT
+#define RT_REFILL_SPLIT 16
+#endif
 #define FULLMASK 0xFFFFFFFFu
 // Resident blocks per SM each traversal kernel is compiled for.  Full nodes
 // keep 48 box words in flight: 7 blocks (72 registers; gem extend 9.0 ms against
@@ -703,6 +708,19 @@ RT_D uint32_t warp_lanes(uint32_t n) {
 // MODE 0: wavefront extend (queue of path ids, rays in PathState, hits to PathState)
 // MODE 1: API (rays n×8 in memory, hits as int4)
 
+// Closest hit over quantised nodes, without convex solids: an iteration is at
+// most one node visit and one leaf test per lane, and a lane with leaves left
+// tests them in the next iterations while the others visit nodes, instead of
+// holding the warp in a loop as long as its longest list.  Each lane's own order
+// of visits and tests is the same, so its hits are.  Bound by issue slots at 14-17
+// of 32 lanes (1,310,720 triangles, 1080p at 64 samples: extend 50.0 -> 45.2 ms;
+// 4M caller rays against 327,680 triangles 1.58 -> 1.41 ms).  Waiting for 3, 6 or
+// 10 lanes with leaves before testing any was slower (46.6, 48.7, 54.6 ms).  The
+// loop stays for full nodes, where the list's two words spill (96 B at 72
+// registers; 24 thumbnails 20.2 -> 21.1 ms, equal at 80 registers), and for
+// any-hit rays, where it made no difference (14.8 ms both).
+template <bool ANA, int NF> constexpr bool split_leaves() { return !ANA && NF == RT_NODES_QUANTISED; }
+
 template <int MODE, bool ANA, int NF>
 __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) k_closest(DevScene S, PathState P, const uint32_t* __restrict__ queue,
                                                             const float* __restrict__ rays, uint32_t n_api,
@@ -723,9 +741,12 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) 
     RayC R = make_rayc(o, mk(1.f, 1.f, 1.f), 0.0f);
     float tmin = 0.0f;
     Best best{0.0f, 0.0f, 0.0f, RT_MISS_REF, 0xFFFFFFFFu};
+    // split leaves: the pending ones of the last visited node (bits 0-7), all its
+    // leaves (8-15) and whether no group is left (16); its first leaf
+    uint32_t pend = 0u, first = 0u;
     while (true) {
         uint32_t idle = __ballot_sync(FULLMASK, !active);
-        if (!exhausted && __popc(idle) >= RT_REFILL_CLOSEST) {
+        if (!exhausted && __popc(idle) >= (split_leaves<ANA, NF>() ? RT_REFILL_SPLIT : RT_REFILL_CLOSEST)) {
             if (ANA) idle &= warp_lanes<ANA>(n);
             uint32_t k = __popc(idle), base = 0;
             if (lane == 0 && (!ANA || k)) base = atomicAdd(next, k);
@@ -758,17 +779,41 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) 
             }
         }
         if (exhausted && __ballot_sync(FULLMASK, active) == 0) break;
-        NodeHead h{0u, 0u, 0u};
-        uint32_t inner = 0u;
-        rtk::Convex cv{0u, 0u};
-        if (active) rtk::closest_visit<ANA, NF>(S, R, d, tmin, best, grp, h, inner, cv);
-        if (ANA) rtk::closest_convex(S, leaf_set<NF>(S), R, d, tmin, best, cv);
+        bool done = false;
+        if constexpr (!split_leaves<ANA, NF>()) {
+            NodeHead h{0u, 0u, 0u};
+            uint32_t inner = 0u;
+            rtk::Convex cv{0u, 0u};
+            if (active) rtk::closest_visit<ANA, NF>(S, R, d, tmin, best, grp, h, inner, cv);
+            if (ANA) rtk::closest_convex(S, leaf_set<NF>(S), R, d, tmin, best, cv);
+            if (active) {
+                bool lok = true;
+                done = !rtk::next_group(S, grp, h.child, inner, h.masks, stk, lok);
+                if (!lok) ok = false;
+            }
+        } else {
+            if (active && !(pend & 0xFFu)) {
+                NodeHead h{0u, 0u, 0u};
+                const uint32_t node = rtk::take_nearest(grp, R.ord);
+                const uint32_t hits = node_test_any<NF>(S, node, R, tmin, best.t, h);
+                bool lok = true;
+                const bool more = rtk::next_group(S, grp, h.child, hits & h.masks & 0xFFu, h.masks, stk, lok);
+                if (!lok) ok = false;
+                pend = (hits & (h.masks >> 8)) | (h.masks & 0xFF00u) | (more ? 0u : 1u << 16);
+                first = h.leaf;
+            }
+            if (pend & 0xFFu) {
+                const uint32_t leaves = pend & 0xFFu;
+                const uint32_t k = __popc(((pend >> 8) & 0xFFu) & ((leaves & (0u - leaves)) - 1u));
+                pend &= pend - 1u;
+                leaf_closest<ANA>(S, leaf_set<NF>(S), first + k, R, d, tmin, best);
+            }
+            done = active && (pend >> 16) && !(pend & 0xFFu);
+        }
         if (active) {
-            bool lok = true;
-            bool more = rtk::next_group(S, grp, h.child, inner, h.masks, stk, lok);
-            if (!lok) ok = false;
-            if (!more) {
+            if (done) {
                 active = false;
+                pend = 0u;
                 bool hit = best.ref != RT_MISS_REF;
                 if (MODE == 0) {
                     P.hit[pid] = make_float4(__uint_as_float(best.ref), best.t, best.b1, best.b2);
@@ -1015,12 +1060,14 @@ int trace_grid(const DevScene& S, int dev_sms, int resident) {
 // The layout a launch reads.  Default (RT_NODES_FULL): the quantised copy for
 // trees whose full nodes are far beyond the L1, where its 80 bytes against 208
 // win more in fetches than its decoding costs (16-spp icosphere frames by
-// subdivision 4, 6, 7, extend + shadow: full 8.8, 12.9, 15.9 ms, quantised 9.2,
-// 12.9, 15.1); and for caller-given rays, which are incoherent as a rule (4M
-// random rays, subdivision 4, 6, 7: full 1.21, 1.60, 1.86 ms, quantised 1.11,
-// 1.42, 1.56), from 256 nodes.
+// subdivision 5, 6, 7, with 5,776, 26,984, 123,710 nodes: full 15.6, 17.9, 20.5 ms,
+// quantised 15.7, 17.2, 19.0; without split leaves, as in scenes with analytic
+// solids, 16.2, 17.9, 19.9); and for caller-given rays, which are incoherent as a
+// rule (4M random rays, subdivision 4, 6, 7: full 1.21, 1.60, 1.86 ms, quantised
+// 1.11, 1.42, 1.56), from 256 nodes.
 int trace_format(const DevScene& S, bool caller_rays) {
-    if (S.node_format == RT_NODES_FULL && S.qnodes && S.n_nodes >= (caller_rays ? 256u : 32768u))
+    const uint32_t from = caller_rays ? 256u : S.n_analytic > 0 ? 32768u : 8192u;
+    if (S.node_format == RT_NODES_FULL && S.qnodes && S.n_nodes >= from)
         return RT_NODES_QUANTISED;
     return S.node_format;
 }
