@@ -606,7 +606,7 @@ typedef struct RtTuning {
     /* Node layout the traversal reads (every layout keeps a node's children
      * next to each other in octant order, with one header): RT_NODES_FULL (0,
      * the default), the reference's float boxes (bvh.rs:25-32), 208 bytes per
-     * node — or, where it measured faster (trees far beyond the L1, caller-given
+     * node — or, where it measured faster (trees of a few hundred nodes, caller-given
      * rays), the quantised copy when the scene has one; RT_NODES_QUANTISED (1,
      * when the scene's extents allow it), 80-byte nodes whose child boxes are
      * 8-bit offsets rounded outward; RT_NODES_WIDE4 (2, scenes whose tree

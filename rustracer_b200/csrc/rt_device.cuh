@@ -269,39 +269,6 @@ enum {
 // whole line (the ray is inside the closed slab) so culling stays conservative.
 
 // ── primitive hit tests: same f32 operation sequence as the reference ────────
-// convex_hit (diamond.rs:202-253): the interval inside every half-space; the
-// entry for outside rays, the exit for rays inside; *plane = crossing plane.
-RT_D bool convex_test(const float4* pl, int n, float3 o, float3 d, float tmin, float tmax, float* t_out,
-                      int* plane) {
-    float t_enter = tmin, t_exit = tmax;
-    int enter_i = -1, exit_i = -1;
-    bool entry_found = false;
-    for (int i = 0; i < n; i++) {
-        float4 q = __ldg(pl + i);
-        float3 nv = make_float3(q.x, q.y, q.z);
-        float nd = nv.x * d.x + nv.y * d.y + nv.z * d.z;
-        float no = nv.x * o.x + nv.y * o.y + nv.z * o.z;
-        float t_face = (q.w - no) / nd;
-        if (fabsf(nd) < 1e-8f) {
-            if (no > q.w) return false;
-            continue;
-        }
-        if (nd < 0.0f) {
-            if (t_face > t_enter) { t_enter = t_face; enter_i = i; entry_found = true; }
-        } else {
-            if (t_face < t_exit || (exit_i < 0 && t_face == t_exit)) { t_exit = t_face; exit_i = i; }
-        }
-        if (t_enter > t_exit) return false;
-    }
-    if (t_enter > t_exit) return false;
-    if (t_enter == t_exit && t_enter < tmax) return false;
-    if (entry_found) { *t_out = t_enter; *plane = enter_i; return true; }
-    // an interior ray whose exit lies beyond tmax crosses nothing in [tmin, tmax]
-    if (exit_i < 0 || t_exit > tmax) return false;
-    *t_out = t_exit; *plane = exit_i;
-    return true;
-}
-
 // ── cylinder, cone, disk, infinite plane (cylinder.rs, cone.rs, disk.rs, plane.rs)
 // Record P[0..7]: (centre, radius) (unit normal, height) (u axis, wave amplitude)
 // (v axis, wave scale) (rotation row 0, scale) (row 1, 1/scale) (row 2, placed)

@@ -30,13 +30,15 @@ struct Best { float t, b1, b2; uint32_t ref, gid; };
 
 RT_D uint32_t f2u(float f) { return __float_as_uint(f); }
 
-// convex_test (rt_device.cuh) of one ray by the whole warp: a brilliant has 97
-// planes and a step cut up to several hundred, one lane's serial loop over
-// them idles the other 31, and the loop's result — the entry is the largest
-// crossing of the planes facing the ray, the exit the smallest of the others,
-// the first plane of equal ones — does not depend on the order.  Lane l takes
-// planes l, l + 32, …; a −0 crossing counts as 0 in the comparison, as it does
-// there.  Every lane calls it with the same arguments; all get the result.
+// A convex solid (convex_hit, diamond.rs:202-253): the interval inside every
+// half-space, the entry for outside rays, the exit for rays inside; *plane is the
+// crossing plane.  One ray by the whole warp: a brilliant has 97 planes and a
+// step cut up to several hundred, one lane's serial loop over them idles the
+// other 31, and the loop's result — the entry is the largest crossing of the
+// planes facing the ray, the exit the smallest of the others, the first plane of
+// equal ones — does not depend on the order.  Lane l takes planes l, l + 32, …; a
+// −0 crossing counts as 0 in the comparison, as it does there.  Every lane calls
+// it with the same arguments; all get the result.
 RT_D uint32_t order_key(float t) {                  // monotone in t
     uint32_t u = __float_as_uint(t + 0.0f);
     return (u & 0x80000000u) ? ~u : u | 0x80000000u;
@@ -779,7 +781,16 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) 
             }
         }
         if (exhausted && __ballot_sync(FULLMASK, active) == 0) break;
-        bool done = false;
+        auto finish = [&] {
+            active = false;
+            bool hit = best.ref != RT_MISS_REF;
+            if (MODE == 0) {
+                P.hit[pid] = make_float4(__uint_as_float(best.ref), best.t, best.b1, best.b2);
+            } else {
+                out[item] = make_int4(hit ? (int)best.gid : -1, __float_as_int(hit ? best.t : 0.0f),
+                                      __float_as_int(hit ? best.b1 : 0.0f), __float_as_int(hit ? best.b2 : 0.0f));
+            }
+        };
         if constexpr (!split_leaves<ANA, NF>()) {
             NodeHead h{0u, 0u, 0u};
             uint32_t inner = 0u;
@@ -788,8 +799,9 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) 
             if (ANA) rtk::closest_convex(S, leaf_set<NF>(S), R, d, tmin, best, cv);
             if (active) {
                 bool lok = true;
-                done = !rtk::next_group(S, grp, h.child, inner, h.masks, stk, lok);
+                bool more = rtk::next_group(S, grp, h.child, inner, h.masks, stk, lok);
                 if (!lok) ok = false;
+                if (!more) finish();
             }
         } else {
             if (active && !(pend & 0xFFu)) {
@@ -808,19 +820,9 @@ __global__ void __launch_bounds__(RT_TRACE_BLOCK, trace_minb<NF, ANA, false>()) 
                 pend &= pend - 1u;
                 leaf_closest<ANA>(S, leaf_set<NF>(S), first + k, R, d, tmin, best);
             }
-            done = active && (pend >> 16) && !(pend & 0xFFu);
-        }
-        if (active) {
-            if (done) {
-                active = false;
+            if (active && (pend >> 16) && !(pend & 0xFFu)) {
                 pend = 0u;
-                bool hit = best.ref != RT_MISS_REF;
-                if (MODE == 0) {
-                    P.hit[pid] = make_float4(__uint_as_float(best.ref), best.t, best.b1, best.b2);
-                } else {
-                    out[item] = make_int4(hit ? (int)best.gid : -1, __float_as_int(hit ? best.t : 0.0f),
-                                          __float_as_int(hit ? best.b1 : 0.0f), __float_as_int(hit ? best.b2 : 0.0f));
-                }
+                finish();
             }
         }
     }
@@ -1057,16 +1059,18 @@ int trace_grid(const DevScene& S, int dev_sms, int resident) {
     return dev_sms * (S.trace_per_sm > 0 ? std::min(S.trace_per_sm, resident) : resident);
 }
 
-// The layout a launch reads.  Default (RT_NODES_FULL): the quantised copy for
-// trees whose full nodes are far beyond the L1, where its 80 bytes against 208
-// win more in fetches than its decoding costs (16-spp icosphere frames by
-// subdivision 5, 6, 7, with 5,776, 26,984, 123,710 nodes: full 15.6, 17.9, 20.5 ms,
-// quantised 15.7, 17.2, 19.0; without split leaves, as in scenes with analytic
-// solids, 16.2, 17.9, 19.9); and for caller-given rays, which are incoherent as a
-// rule (4M random rays, subdivision 4, 6, 7: full 1.21, 1.60, 1.86 ms, quantised
-// 1.11, 1.42, 1.56), from 256 nodes.
+// The layout a launch reads.  Default (RT_NODES_FULL): the quantised copy, whose
+// 80 bytes against 208 win more in fetches than its decoding costs, from 256
+// nodes on in scenes without convex solids or shapes, where its closest-hit
+// kernel also splits the leaf tests (16-spp icosphere frames of 1,960, 5,776,
+// 26,984, 123,710 nodes: full 14.5, 15.8, 17.9, 20.5 ms, quantised 14.5, 15.6,
+// 17.2, 19.0; gem with photons, 715 nodes, 30.3 and 29.0), and for caller-given
+// rays, which are incoherent as a rule (4M random rays, 1,960, 26,984, 123,710
+// nodes: full 1.21, 1.60, 1.86 ms, quantised 1.11, 1.42, 1.33); in scenes with
+// such solids from 32,768 (16-spp frames by the unsplit kernels: 5,776 nodes 15.6
+// and 16.2 ms, 26,984 17.9 and 17.8).
 int trace_format(const DevScene& S, bool caller_rays) {
-    const uint32_t from = caller_rays ? 256u : S.n_analytic > 0 ? 32768u : 8192u;
+    const uint32_t from = caller_rays || S.n_analytic == 0 ? 256u : 32768u;
     if (S.node_format == RT_NODES_FULL && S.qnodes && S.n_nodes >= from)
         return RT_NODES_QUANTISED;
     return S.node_format;
