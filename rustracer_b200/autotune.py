@@ -21,7 +21,7 @@ import math
 
 from . import abi
 
-SPACE = {"max_paths": (1 << 21, 1 << 22, 1 << 23), "trace_blocks_per_sm": (4, 6), "shade_blocks_per_sm": (4, 8, 16),
+SPACE = {"max_paths": (1 << 21, 1 << 22, 1 << 23), "trace_blocks_per_sm": (6, 8), "shade_blocks_per_sm": (4, 8, 16),
          "node_format": (abi.RT_NODES_FULL, abi.RT_NODES_QUANTISED, abi.RT_NODES_WIDE4)}
 PROBE_SAMPLES = 1 << 24
 _cache = {}
