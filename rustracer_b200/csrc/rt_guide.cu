@@ -189,7 +189,7 @@ struct TrainArgs {
     uint32_t seed;
     __nv_bfloat16* act;      // ACT_ROWS × batch
     float* grad;             // N_PARAMS
-    float* loss;             // Σ −w log p over the batch
+    double* loss_part;       // Σ −w log p of every 16 rows
 };
 
 RTG_D bool train_row(const TrainArgs& A, uint32_t row, uint32_t n, float4* s) {
@@ -224,7 +224,6 @@ __global__ void __launch_bounds__(GW * 32) k_train(GuideDev G, TrainArgs A) {
     uint32_t n = A.select ? *A.n_dev : A.n;
     float scale = 1.0f / (float)(A.select ? A.batch : max(A.n, 1u));
     size_t B = A.batch;
-    float lsum = 0.0f;
     for (uint32_t base = (blockIdx.x * GW + warp) * 32; base < A.batch; base += gridDim.x * GW * 32) {
         float4 s[3];
         bool valid = train_row(A, base + lane, n, s);
@@ -251,17 +250,21 @@ __global__ void __launch_bounds__(GW * 32) k_train(GuideDev G, TrainArgs A) {
             // loss gradient of row row0 + lane
             float4 r[3] = {};
             bool rv = false;
+            float row_loss = 0.0f;
             if (lane < 16) {
                 rv = train_row(A, row0 + lane, n, r) && r[0].w > 0.0f;
                 float g[NOUT];
                 if (rv) {
-                    lsum += loss_grad(S_o + lane * LDO, r[1].x, r[1].y, r[1].z, r[2].x, r[2].y, r[2].z, r[0].w, scale,
+                    row_loss = loss_grad(S_o + lane * LDO, r[1].x, r[1].y, r[1].z, r[2].x, r[2].y, r[2].z, r[0].w, scale,
                                       G.amax, G.lkmax, g);
                 } else {
                     for (int k = 0; k < NOUT; k++) g[k] = 0.0f;
                 }
                 for (int k = 0; k < NOUTP; k++) S_do[lane * LDT3 + k] = __float2bfloat16_rn(k < NOUT ? g[k] : 0.0f);
             }
+            double tile_loss = row_loss;
+            for (int o = 8; o > 0; o >>= 1) tile_loss += __shfl_down_sync(0xFFFFFFFFu, tile_loss, o);
+            if (lane == 0) A.loss_part[row0 / 16] = tile_loss;
             __syncwarp();
             uint32_t dO[3][4];
             load_frags<3>(S_do, LDT3, dO);
@@ -321,7 +324,22 @@ __global__ void __launch_bounds__(GW * 32) k_train(GuideDev G, TrainArgs A) {
             __syncwarp();
         }
     }
-    if (lsum != 0.0f) atomicAdd(A.loss, lsum);
+}
+// The loss from the tiles' sums, in one block and a fixed order.  The rows' sum
+// is formed in doubles and rounded once: 65,536 rows added to one float by
+// unordered atomics came out up to 3e-6 apart from call to call.
+constexpr int LOSS_BLOCK = 256;
+__global__ void __launch_bounds__(LOSS_BLOCK) k_loss(const double* __restrict__ part, uint32_t n, float* loss) {
+    __shared__ double sum[LOSS_BLOCK];
+    double v = 0.0;
+    for (uint32_t i = threadIdx.x; i < n; i += LOSS_BLOCK) v += part[i];
+    sum[threadIdx.x] = v;
+    __syncthreads();
+    for (int o = LOSS_BLOCK / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o) sum[threadIdx.x] += sum[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss = (float)sum[0];
 }
 
 // ∂loss/∂W_l = Σ_b dZ_{l+1}[b]ᵀ · H_l[b]: block (chunk, l); warp w owns output rows 16w..16w+15
@@ -451,7 +469,8 @@ static bool alloc_act(Guide* g, uint32_t batch) {
     if (g->act) cudaFree(g->act);
     g->act = nullptr;
     g->act_batch = 0;
-    if (cudaMalloc(&g->act, (size_t)ACT_ROWS * batch * 2) != cudaSuccess) return false;
+    // the planes, then the sums of the loss per 16 rows
+    if (cudaMalloc(&g->act, (size_t)ACT_ROWS * batch * 2 + batch / 16 * sizeof(double)) != cudaSuccess) return false;
     g->act_batch = batch;
     return true;
 }
@@ -626,13 +645,18 @@ void eval(Guide* g, const float* q, uint32_t n, const float* dirs, const float* 
     k_guide_api<<<blocks, GW * 32, api_smem(), st>>>(view(g), q, n, dirs, u, raw, out);
 }
 
+// where a step over `batch` rows leaves its sums of the loss
+static double* loss_part(const Guide* g, uint32_t batch) {
+    return reinterpret_cast<double*>(g->act + (size_t)ACT_ROWS * batch);
+}
+
 // one forward/backward pass and, if `adam`, one Adam step
 static cudaError_t step(Guide* g, const TrainArgs& a0, bool adam, int sms, cudaStream_t st) {
     cudaError_t e;
     TrainArgs a = a0;
     a.act = g->act;
     a.grad = g->grad;
-    a.loss = g->loss;
+    a.loss_part = loss_part(g, a.batch);
     if ((e = cudaMemsetAsync(g->grad, 0, N_PARAMS * 4, st))) return e;
     uint32_t blocks = std::min<uint32_t>(a.batch / (GW * 32), (uint32_t)sms * 2);
     k_train<<<blocks, GW * 32, train_smem(), st>>>(view(g), a);
@@ -662,10 +686,11 @@ cudaError_t train_explicit(Guide* g, const float4* samples, uint32_t n, int step
     a.select = 0;
     int runs = std::max(steps, 1);
     for (int i = 0; i < runs; i++) {
-        if ((e = cudaMemsetAsync(g->loss, 0, 4, st))) return e;
         if ((e = step(g, a, steps > 0, sms, st))) return e;
     }
     if (loss_host) {
+        k_loss<<<1, LOSS_BLOCK, 0, st>>>(loss_part(g, batch), batch / 16, g->loss);
+        if ((e = cudaGetLastError())) return e;
         if ((e = cudaMemcpyAsync(loss_host, g->loss, 4, cudaMemcpyDeviceToHost, st))) return e;
     }
     return cudaStreamSynchronize(st);
@@ -704,7 +729,6 @@ cudaError_t train_pass(Guide* g, int sms, cudaStream_t st, int64_t* launches) {
             a.batch = batch;
             a.select = 1;
             a.seed = mix32((uint32_t)g->prm.seed ^ mix32((uint32_t)g->steps + 1u));
-            if ((e = cudaMemsetAsync(g->loss, 0, 4, st))) return e;
             if ((e = step(g, a, true, sms, st))) return e;
         }
     }
