@@ -162,7 +162,7 @@ __device__ __noinline__ uint32_t node_test_general(const float4* N, float3 o, fl
         if (isnan(daz) || isnan(dbz)) { lz = -INFINITY; hz = INFINITY; }
         float t0 = fmaxf(fmaxf(fmaxf(tmin, lx), ly), lz);
         float t1 = fminf(fminf(fminf(tmax, hx), hy), hz);
-        float t1w = t1 + fabsf(t1) * SLAB_WIDEN;
+        float t1w = t1 + fabsf(t1) * (EXIT_WIDEN - 1.0f);
         if (t0 <= t1w) mask |= 1u << c;
     }
     return mask;
@@ -288,7 +288,7 @@ __device__ __noinline__ uint32_t qnode_test_general(const float4* N, float3 o, f
         if (isnan(daz) || isnan(dbz)) { lz = -INFINITY; hz = INFINITY; }
         float t0 = fmaxf(fmaxf(fmaxf(tmin, lx), ly), lz);
         float t1 = fminf(fminf(fminf(tmax, hx), hy), hz);
-        float t1w = t1 + fabsf(t1) * SLAB_WIDEN;
+        float t1w = t1 + fabsf(t1) * (EXIT_WIDEN - 1.0f);
         if (t0 <= t1w) mask |= 1u << c;
     }
     return mask;
@@ -314,7 +314,7 @@ __device__ __noinline__ uint32_t node4_test_general(const float4* N, float3 o, f
         if (isnan(daz) || isnan(dbz)) { lz = -INFINITY; hz = INFINITY; }
         float t0 = fmaxf(fmaxf(fmaxf(tmin, lx), ly), lz);
         float t1 = fminf(fminf(fminf(tmax, hx), hy), hz);
-        float t1w = t1 + fabsf(t1) * SLAB_WIDEN;
+        float t1w = t1 + fabsf(t1) * (EXIT_WIDEN - 1.0f);
         if (t0 <= t1w) mask |= 1u << c;
     }
     return mask;
@@ -354,15 +354,19 @@ RT_D uint32_t node_test_any(const DevScene& S, uint32_t ni, const RayC& R, float
 template <int NF>
 RT_D const LeafSet& leaf_set(const DevScene& S) { return NF == RT_NODES_WIDE4 ? S.leaves4 : S.leaves; }
 
-// The node tests let every leaf through that this test accepts; a primitive's
-// hit counts only if the leaf's own float box is met too, in the arithmetic of the
-// reference-layout slab test: planes (b − o)·inv, the exit widened by 2^-15,
-// the bound by 2^-16 (rays with a zero direction component or t_min < 0: both
-// planes with min / max, a NaN slab spanning the whole line).  A triangle seen
-// edge-on at its box's corner can have a t far off its box, so without this the
-// layout and the looseness of the node tests would show in a hit (one in 10^8
-// camera rays of the icosphere).  Asked for accepted hits only: ahead of every
-// primitive test it cost 12 % of the closest-hit kernel (48.3 → 54.0 ms).
+// A primitive's hit counts only if the ray meets the leaf's own float box, in the
+// arithmetic of the reference-layout slab test: planes (b − o)·inv, the exit
+// widened by 2^-15, the bound by 2^-16 (rays with a zero direction component or
+// t_min < 0: both planes with min / max, a NaN slab spanning the whole line).  The
+// node tests are the looser ones in every layout.  A triangle seen edge-on at its
+// box's corner can have a t far off its box, so without this the looseness would
+// show in a hit (one in 10^8 camera rays of the icosphere).  The closest hit so
+// far is no bound here (closest-hit rays pass an infinite t_max): whether a hit
+// counts depends on the primitive and the ray, not on the order of the tests.
+// (What the order still decides, as in the reference, is whether the traversal
+// comes to a primitive at all whose box begins beyond the closest hit while its
+// computed t lies before.)  Asked for accepted hits only: ahead of every primitive
+// test it cost 12 % of the closest-hit kernel (48.3 → 54.0 ms).
 __device__ __noinline__ bool leaf_box_general(float4 lo, float4 hi, float3 o, float3 inv, float tmin, float tmax) {
     const float W = 1.000030517578125f;   // 1 + 2^-15
     const float L[3] = {lo.x, lo.y, lo.z}, H[3] = {hi.x, hi.y, hi.z}, O[3] = {o.x, o.y, o.z}, I[3] = {inv.x, inv.y, inv.z};
@@ -435,7 +439,7 @@ RT_D bool leaf_closest(const DevScene& S, const LeafSet& LS, uint32_t k, const R
         b2 = 0.0f;
     }
     if (h && (t < best.t || best.ref == RT_MISS_REF || gid < best.gid) &&
-        leaf_box(LS.box + (size_t)k * 2, R, tmin, best.t)) {
+        leaf_box(LS.box + (size_t)k * 2, R, tmin, INFINITY)) {
         best.t = t; best.b1 = b1; best.b2 = b2; best.ref = ref; best.gid = gid;
     }
     return false;
@@ -603,7 +607,7 @@ RT_D void closest_convex(const DevScene& S, const LeafSet& LS, const RayC& R, fl
                              __shfl_sync(0xFFFFFFFFu, tmin, L), __shfl_sync(0xFFFFFFFFu, best.t, L), &t, &pi);
         if (h && (threadIdx.x & 31u) == L) {
             uint32_t gid = f2u(__ldg(rec + 1).x);
-            if ((t < best.t || best.ref == RT_MISS_REF || gid < best.gid) && leaf_box(LS.box + (size_t)leaf * 2, R, tmin, best.t)) {
+            if ((t < best.t || best.ref == RT_MISS_REF || gid < best.gid) && leaf_box(LS.box + (size_t)leaf * 2, R, tmin, INFINITY)) {
                 best.t = t; best.b1 = __int_as_float(pi); best.b2 = 0.0f; best.ref = ref; best.gid = gid;
             }
         }
