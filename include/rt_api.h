@@ -604,15 +604,15 @@ typedef struct RtTuning {
      * spill path. */
     uint32_t stack_ring;
     /* Node layout the traversal reads (every layout keeps a node's children
-     * next to each other in octant order, with one header): RT_NODES_FULL (0,
-     * the default), the reference's float boxes (bvh.rs:25-32), 208 bytes per
-     * node — or, where it measured faster (trees of a few hundred nodes, caller-given
-     * rays), the quantised copy when the scene has one; RT_NODES_QUANTISED (1,
-     * when the scene's extents allow it), 80-byte nodes whose child boxes are
-     * 8-bit offsets rounded outward; RT_NODES_WIDE4 (2, scenes whose tree
-     * was built on the device), 4-wide nodes of 112 bytes over the same binary
-     * SAH tree — the reference's BVH width choice (bvh.rs:10-14).  The hits do
-     * not depend on it. */
+     * next to each other in octant order, with one header): RT_NODES_FULL (0),
+     * the reference's float boxes (bvh.rs:25-32), 208 bytes per node;
+     * RT_NODES_QUANTISED (1, when the scene's extents allow it), 80-byte nodes
+     * whose child boxes are 8-bit offsets rounded outward; RT_NODES_WIDE4 (2,
+     * scenes whose tree was built on the device), 4-wide nodes of 112 bytes over
+     * the same binary SAH tree — the reference's BVH width choice
+     * (bvh.rs:10-14); RT_NODES_AUTO (3, what a scene starts with): each launch
+     * reads the full or the quantised nodes, whichever measured faster for the
+     * size of the tree and the kind of rays.  The hits do not depend on it. */
     uint32_t node_format;
     /* 1: every render call runs its wavefront as one CUDA graph — the path
      * pool's first fill, then one conditional node per iteration up to the
@@ -628,6 +628,7 @@ typedef struct RtTuning {
 #define RT_NODES_FULL      0
 #define RT_NODES_QUANTISED 1
 #define RT_NODES_WIDE4     2
+#define RT_NODES_AUTO      3
 int32_t rt_set_tuning(RtScene* scene, const RtTuning* tuning);
 
 /* The stream the caller queues its own work on (a cudaStream_t; NULL = the

@@ -124,7 +124,7 @@ struct DevScene {
     // and upper x, y, z planes of 4 children, header), and their leaves
     const float4* nodes4;
     LeafSet leaves4;
-    int node_format;            // as set by rt_set_tuning (RT_NODES_FULL: the launch picks, see trace_format)
+    int node_format;            // as set by rt_set_tuning (RT_NODES_AUTO: the launch picks, see trace_format)
     uint32_t n_nodes;           // 8-wide nodes
     const float4* tri;
     const float4* tri_n;

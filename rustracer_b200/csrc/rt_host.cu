@@ -759,6 +759,7 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return bail(fail(s, RT_ERR_CUDA, "no CUDA device"));
     if (device < 0 || device >= ndev) return bail(fail(s, RT_ERR_INVALID, "device index out of range"));
     s->device = device;
+    s->S.node_format = RT_NODES_AUTO;
     if (cudaSetDevice(device) != cudaSuccess) return bail(fail(s, RT_ERR_CUDA, "cudaSetDevice failed"));
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, device);
@@ -1170,7 +1171,6 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
         if ((rc = upload(s, gcvx.data(), gcvx.size(), &s->S.cvx))) return bail(rc);
         if ((rc = upload(s, wpl.data(), wpl.size(), &s->S.cvx_planes))) return bail(rc);
         if ((rc = upload(s, wsh.data(), wsh.size(), &s->S.cvx_shade))) return bail(rc);
-        s->S.node_format = RT_NODES_FULL;
         if (dev_wide) {
             s->d_ref_nodes = W.nodes;
             d_ref4 = W.nodes4;
@@ -2576,8 +2576,8 @@ extern "C" int32_t rt_set_tuning(RtScene* s, const RtTuning* t) {
         return fail(s, RT_ERR_INVALID, "trace_blocks_per_sm must be in 0..8, shade_blocks_per_sm in 0..32");
     if (t->stack_ring != 0 && (t->stack_ring > RT_SHORT_STACK || (t->stack_ring & (t->stack_ring - 1)) != 0))
         return fail(s, RT_ERR_INVALID, "stack_ring must be 0 or a power of two up to " + std::to_string(RT_SHORT_STACK));
-    if (t->node_format != RT_NODES_QUANTISED && t->node_format != RT_NODES_FULL && t->node_format != RT_NODES_WIDE4)
-        return fail(s, RT_ERR_INVALID, "node_format must be RT_NODES_FULL, RT_NODES_QUANTISED or RT_NODES_WIDE4");
+    if (t->node_format > RT_NODES_AUTO)
+        return fail(s, RT_ERR_INVALID, "node_format must be RT_NODES_FULL, RT_NODES_QUANTISED, RT_NODES_WIDE4 or RT_NODES_AUTO");
     if (t->node_format == RT_NODES_QUANTISED && !s->qnodes_ok && !s->empty)
         return fail(s, RT_ERR_INVALID, "the scene's extents exceed the quantised node layout");
     if (t->node_format == RT_NODES_WIDE4 && !s->wide4_ok && !s->empty)
@@ -2596,6 +2596,7 @@ extern "C" int32_t rt_set_tuning(RtScene* s, const RtTuning* t) {
     s->S.stack_ring = t->stack_ring ? (int)t->stack_ring : RT_SHORT_STACK;
     s->S.node_format = (s->qnodes_ok && t->node_format == RT_NODES_QUANTISED) ? RT_NODES_QUANTISED
                      : (s->wide4_ok && t->node_format == RT_NODES_WIDE4)    ? RT_NODES_WIDE4
+                     : t->node_format == RT_NODES_AUTO                      ? RT_NODES_AUTO
                                                                             : RT_NODES_FULL;
     s->graph_mode = t->graph != 0;
     return RT_OK;

@@ -1063,7 +1063,7 @@ int trace_grid(const DevScene& S, int dev_sms, int resident) {
     return dev_sms * (S.trace_per_sm > 0 ? std::min(S.trace_per_sm, resident) : resident);
 }
 
-// The layout a launch reads.  Default (RT_NODES_FULL): the quantised copy, whose
+// The layout a launch reads.  RT_NODES_AUTO: the quantised copy, whose
 // 80 bytes against 208 win more in fetches than its decoding costs, from 256
 // nodes on in scenes without convex solids or shapes, where its closest-hit
 // kernel also splits the leaf tests (16-spp icosphere frames of 1,960, 5,776,
@@ -1075,9 +1075,8 @@ int trace_grid(const DevScene& S, int dev_sms, int resident) {
 // and 16.2 ms, 26,984 17.9 and 17.8).
 int trace_format(const DevScene& S, bool caller_rays) {
     const uint32_t from = caller_rays || S.n_analytic == 0 ? 256u : 32768u;
-    if (S.node_format == RT_NODES_FULL && S.qnodes && S.n_nodes >= from)
-        return RT_NODES_QUANTISED;
-    return S.node_format;
+    if (S.node_format != RT_NODES_AUTO) return S.node_format;
+    return S.qnodes && S.n_nodes >= from ? RT_NODES_QUANTISED : RT_NODES_FULL;
 }
 // the traversal kernels with (ANA) or without analytic solids, by node layout
 #define RT_TRACE_ONE(K, MODE, ANA, NF, ...)                                                          \

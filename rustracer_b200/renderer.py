@@ -453,17 +453,26 @@ class GpuScene:
     # ── diagnostics ──────────────────────────────────────────────────────
     # ── launch tuning (rt_set_tuning) ─────────────────────────────────────
     def set_tuning(self, max_paths=0, trace_blocks_per_sm=0, shade_blocks_per_sm=0, max_iterations=0,
-                   stack_limit=0, stack_ring=0, node_format=0, graph=0):
+                   stack_limit=0, stack_ring=0, node_format=None, graph=0, node_auto=False):
+        """Zeros and a node_format of None select the built-in values; node_auto=True
+        leaves the node layout to the library whatever node_format says (so that
+        set_tuning(**get_tuning()) changes nothing)."""
+        if node_format is None or node_auto:
+            node_format = abi.RT_NODES_AUTO
         t = abi.RtTuning(int(max_paths), int(trace_blocks_per_sm), int(shade_blocks_per_sm), int(max_iterations),
                          int(stack_limit), int(stack_ring), int(node_format), int(graph))
         self._check(lib().rt_set_tuning(self.h, C.byref(t)))
 
     def get_tuning(self):
+        """The values in force; node_format is the layout that was set, and 0 with
+        node_auto True where none was and the library picks one per launch."""
         t = abi.RtTuning()
         self._check(lib().rt_get_tuning(self.h, C.byref(t)))
         return dict(max_paths=t.max_paths, trace_blocks_per_sm=t.trace_blocks_per_sm,
                     shade_blocks_per_sm=t.shade_blocks_per_sm, max_iterations=t.max_iterations,
-                    stack_limit=t.stack_limit, stack_ring=t.stack_ring, node_format=t.node_format, graph=t.graph)
+                    stack_limit=t.stack_limit, stack_ring=t.stack_ring,
+                    node_format=0 if t.node_format == abi.RT_NODES_AUTO else t.node_format, graph=t.graph,
+                    node_auto=t.node_format == abi.RT_NODES_AUTO)
 
     # ── path guiding (rt_guide_*) ─────────────────────────────────────────
     def guide_init(self, params=None):
