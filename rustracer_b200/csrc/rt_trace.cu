@@ -1063,18 +1063,21 @@ int trace_grid(const DevScene& S, int dev_sms, int resident) {
     return dev_sms * (S.trace_per_sm > 0 ? std::min(S.trace_per_sm, resident) : resident);
 }
 
-// The layout a launch reads.  RT_NODES_AUTO: the quantised copy, whose
-// 80 bytes against 208 win more in fetches than its decoding costs, from 256
-// nodes on in scenes without convex solids or shapes, where its closest-hit
-// kernel also splits the leaf tests (16-spp icosphere frames of 1,960, 5,776,
-// 26,984, 123,710 nodes: full 14.5, 15.8, 17.9, 20.5 ms, quantised 14.5, 15.6,
-// 17.2, 19.0; gem with photons, 715 nodes, 30.3 and 29.0), and for caller-given
-// rays, which are incoherent as a rule (4M random rays, 1,960, 26,984, 123,710
-// nodes: full 1.21, 1.60, 1.86 ms, quantised 1.11, 1.42, 1.33); in scenes with
-// such solids from 32,768 (16-spp frames by the unsplit kernels: 5,776 nodes 15.6
-// and 16.2 ms, 26,984 17.9 and 17.8).
+// The layout a launch reads.  RT_NODES_AUTO: the quantised copy where its 80 bytes
+// against 208 win more in fetches than its decoding costs, and where its
+// closest-hit kernel also splits the leaf tests.
+// Renders without convex solids or shapes: from 640 nodes on (720p frames at 8
+// samples of triangle soups of 360, 509, 635, 1,577 nodes: full 6.16, 7.15, 7.81,
+// 10.23 ms, quantised 6.47, 7.35, 7.84, 9.82; icospheres of 419, 1,920, 5,950,
+// 26,712 nodes: 3.53, 4.08, 4.46, 5.17 and 3.57, 4.06, 4.41, 4.98; gem with
+// photons, 715 nodes, 30.3 and 29.0).
+// Caller-given rays, incoherent as a rule: from 256 (4M random rays, 26, 189, 419,
+// 1,920, 26,712 nodes: full 0.71, 1.65, 0.91, 1.24, 1.52 ms, quantised 0.68, 1.48,
+// 0.80, 0.96, 1.13; the little it gives below is not taken).
+// Renders with such solids, whose kernel does not split: from 32,768 (16-spp frames
+// by the unsplit kernels: 5,776 nodes 15.6 and 16.2 ms, 26,984 17.9 and 17.8).
 int trace_format(const DevScene& S, bool caller_rays) {
-    const uint32_t from = caller_rays || S.n_analytic == 0 ? 256u : 32768u;
+    const uint32_t from = caller_rays ? 256u : S.n_analytic == 0 ? 640u : 32768u;
     if (S.node_format != RT_NODES_AUTO) return S.node_format;
     return S.qnodes && S.n_nodes >= from ? RT_NODES_QUANTISED : RT_NODES_FULL;
 }
