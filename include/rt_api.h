@@ -594,8 +594,9 @@ typedef struct RtTuning {
      * a render call whose wavefront has not drained after max_iterations
      * iterations returns RT_ERR_TIMEOUT; a traversal that needs more than
      * stack_limit stack entries (the pending children of one node each) stops
-     * and the call returns RT_ERR_CAPACITY.  rt_get_tuning reports the stack
-     * entries in force (7 per tree level; a traversal needs at most one). */
+     * and the call returns RT_ERR_CAPACITY.  rt_get_tuning reports the limit
+     * (built in: 7 entries per tree level; a traversal needs at most one, and
+     * the stacks hold no more). */
     uint32_t max_iterations;       /* 0 or ≥ 1 */
     uint32_t stack_limit;          /* 0 or 1 .. the built-in capacity */
     /* Traversal stack entries kept in a per-thread ring (local memory) before the

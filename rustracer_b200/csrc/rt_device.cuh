@@ -154,7 +154,7 @@ struct DevScene {
     int trace_per_sm, shade_per_sm;   // launch tuning (host side; 0 = the built-in grids)
     // traversal stack beyond the ring: the words of entry e ≥ RT_SHORT_STACK of
     // global thread g at stack_spill[(2(e − RT_SHORT_STACK) + 0, 1) · threads + g];
-    // at most stack_cap entries (lowered only by rt_set_tuning)
+    // at most stack_cap entries, which a column holds (lowered only by rt_set_tuning)
     uint32_t* stack_spill;      // closest hit
     uint32_t* stack_spill_any;  // any hit
     int stack_cap;

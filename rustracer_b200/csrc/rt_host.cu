@@ -505,7 +505,9 @@ struct RtScene {
     std::vector<DevBuf> owned;
     int64_t n_nodes = 0, n_leaves = 0, n_prims = 0;
     int32_t max_depth = 0;
-    int stack_cap_built = 0;          // traversal stack entries the spill columns hold
+    int stack_cap_built = 0;          // the largest stack_limit (7 entries per tree level)
+    int stack_limit = 0;              // as set by rt_set_tuning (0: the built-in capacity)
+    int stack_rows = 0;               // traversal stack entries a spill column holds
     bool qnodes_ok = false;           // the quantised node copy exists (extents within 255·2^60)
     bool wide4_ok = false;            // the 4-wide node copy exists (trees built on the device)
     std::vector<DevLight> h_lights;   // host copy of the NEE light list (photon emitters from lights)
@@ -1033,17 +1035,18 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
         s->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tb).count();
         s->max_depth = B.max_depth;
         // traversal stack: at most one 8-byte entry (a node's pending children)
-        // per tree level, so the capacity of 7 · (depth + 1) entries always
-        // suffices; entries beyond the ring spill to a column per persistent
-        // traversal thread (grid ≤ SMs × RT_TRACE_MINB blocks)
+        // per tree level; entries beyond the ring spill to a column per persistent
+        // traversal thread (grid ≤ SMs × RT_TRACE_MINB blocks).  A column holds
+        // stack_rows entries, also with a ring shrunk by rt_set_tuning, and no
+        // push goes beyond them (TStack::room), whatever stack_limit allows
         if (B.max_depth > 4096) return bail(fail(s, RT_ERR_CAPACITY, "BVH deeper than 4096 levels"));
         s->stack_cap_built = 7 * (B.max_depth + 1) + 8;
         // the 4-wide tree is deeper
         if (dev_wide) s->stack_cap_built = std::max(s->stack_cap_built, 3 * (W.max_depth4 + 1) + 8);
-        s->S.stack_cap = s->stack_cap_built;
+        s->stack_rows = std::max(B.max_depth, dev_wide ? W.max_depth4 : 0) + 2;
+        s->S.stack_cap = std::min(s->stack_cap_built, s->stack_rows);
         s->S.stack_ring = RT_SHORT_STACK;
-        // also room for a ring shrunk by rt_set_tuning
-        size_t spill_words = 2 * (size_t)(std::max(B.max_depth, dev_wide ? W.max_depth4 : 0) + 2);
+        size_t spill_words = 2 * (size_t)s->stack_rows;
         size_t spill_threads = (size_t)s->sms * RT_TRACE_MINB * RT_TRACE_BLOCK;
         void* sp_buf = nullptr;
         if (int rc = dalloc(s, &sp_buf, 2 * spill_words * spill_threads * sizeof(uint32_t)))
@@ -2584,7 +2587,7 @@ extern "C" int32_t rt_set_tuning(RtScene* s, const RtTuning* t) {
         return fail(s, RT_ERR_INVALID, "4-wide nodes exist for trees built on the device only");
     if (t->stack_limit != 0 && (int64_t)t->stack_limit > s->stack_cap_built)
         return fail(s, RT_ERR_INVALID, "stack_limit must be 0 or at most " + std::to_string(s->stack_cap_built) +
-                                           " (the entries the scene's stack columns hold)");
+                                           " (7 entries per tree level)");
     if (t->graph > 1) return fail(s, RT_ERR_INVALID, "graph must be 0 or 1");
     ENTER(s);
     CK(cudaStreamSynchronize(s->stream));
@@ -2592,7 +2595,8 @@ extern "C" int32_t rt_set_tuning(RtScene* s, const RtTuning* t) {
     s->S.trace_per_sm = (int)t->trace_blocks_per_sm;
     s->S.shade_per_sm = (int)t->shade_blocks_per_sm;
     s->max_iterations = t->max_iterations;
-    s->S.stack_cap = t->stack_limit ? (int)t->stack_limit : s->stack_cap_built;
+    s->stack_limit = (int)t->stack_limit;
+    s->S.stack_cap = std::min(s->stack_limit ? s->stack_limit : s->stack_cap_built, s->stack_rows);
     s->S.stack_ring = t->stack_ring ? (int)t->stack_ring : RT_SHORT_STACK;
     s->S.node_format = (s->qnodes_ok && t->node_format == RT_NODES_QUANTISED) ? RT_NODES_QUANTISED
                      : (s->wide4_ok && t->node_format == RT_NODES_WIDE4)    ? RT_NODES_WIDE4
@@ -2614,7 +2618,7 @@ extern "C" int32_t rt_get_tuning(const RtScene* s, RtTuning* t) {
     t->trace_blocks_per_sm = (uint32_t)s->S.trace_per_sm;
     t->shade_blocks_per_sm = (uint32_t)s->S.shade_per_sm;
     t->max_iterations = (uint32_t)s->max_iterations;
-    t->stack_limit = (uint32_t)s->S.stack_cap;
+    t->stack_limit = (uint32_t)(s->stack_limit ? s->stack_limit : s->stack_cap_built);
     t->stack_ring = (uint32_t)s->S.stack_ring;
     t->node_format = (uint32_t)s->S.node_format;
     t->graph = s->graph_mode ? 1u : 0u;

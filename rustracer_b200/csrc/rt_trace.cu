@@ -489,9 +489,9 @@ namespace rtk {
 // fewer slots, so the tests run every traversal through the spill path).  A
 // push beyond the ring first moves the ring slot's old entry to its column, a
 // pop that uncovers a spilled entry brings it back.  A traversal holds at most
-// one group per tree level, so `cap` (sized at scene creation) is never
-// reached in the scene's own tree; a lower cap from rt_set_tuning makes the
-// traversal stop with RT_ERR_CAPACITY.
+// one group per tree level, so S.stack_cap (what a column holds, from the tree's
+// depth) is never reached in the scene's own tree; a lower one from rt_set_tuning
+// makes the traversal stop with RT_ERR_CAPACITY.
 constexpr int RING_STRIDE = RT_STACK_LOCAL ? 1 : RT_TRACE_BLOCK;
 struct TStack {
     uint2* ring;             // ring slot k at ring[k · RING_STRIDE] (shared: &ring[threadIdx.x])
