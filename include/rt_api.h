@@ -611,7 +611,8 @@ typedef struct RtTuning {
      * whose child boxes are 8-bit offsets rounded outward; RT_NODES_WIDE4 (2,
      * scenes whose tree was built on the device), 4-wide nodes of 112 bytes over
      * the same binary SAH tree — the reference's BVH width choice
-     * (bvh.rs:10-14); RT_NODES_AUTO (3, what a scene starts with): each launch
+     * (bvh.rs:10-14), packed when they are first selected (about 190 bytes a
+     * primitive; RT_ERR_NOMEM leaves the tuning as it was); RT_NODES_AUTO (3, what a scene starts with): each launch
      * reads the full or the quantised nodes, whichever measured faster for the
      * size of the tree and the kind of rays.  The hits do not depend on it. */
     uint32_t node_format;

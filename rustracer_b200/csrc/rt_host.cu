@@ -509,7 +509,11 @@ struct RtScene {
     int stack_limit = 0;              // as set by rt_set_tuning (0: the built-in capacity)
     int stack_rows = 0;               // traversal stack entries a spill column holds
     bool qnodes_ok = false;           // the quantised node copy exists (extents within 255·2^60)
-    bool wide4_ok = false;            // the 4-wide node copy exists (trees built on the device)
+    // the 4-wide tree as the build leaves it (trees built on the device), until
+    // RT_NODES_WIDE4 is first selected: then its packed nodes take its place
+    float4* ref4 = nullptr;
+    int64_t n_ref4 = 0;
+    bool wide4_ok() const { return ref4 || S.nodes4; }
     std::vector<DevLight> h_lights;   // host copy of the NEE light list (photon emitters from lights)
     std::vector<float> h_emission;    // per material: RGB emission of a light material (3 floats)
     float photon_stage_ms[3] = {0, 0, 0};   // last photon build: trace, compaction, tree
@@ -729,7 +733,7 @@ int32_t rt_scene_destroy(RtScene* s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     for (auto& b : s->owned) cudaFree(b.p);
     void* ps[] = {s->counters, s->d_err, s->scratch, s->d_conv, s->acc, s->m2, s->cnt, s->stage, s->d_active,
-                  s->b_acc, s->b_m2, s->b_cnt, s->d_jobs, s->d_R, s->d_gstat, s->d_bins};
+                  s->b_acc, s->b_m2, s->b_cnt, s->d_jobs, s->d_R, s->d_gstat, s->d_bins, s->ref4};
     if (s->wg.exec) cudaGraphExecDestroy(s->wg.exec);
     if (s->wg.graph) cudaGraphDestroy(s->wg.graph);
     if (s->h_tot) cudaFreeHost(s->h_tot);
@@ -998,8 +1002,6 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
 
     // ── BVH ─────────────────────────────────────────────────────────────────
     std::vector<float4> gnodes;
-    const float4* d_ref4 = nullptr;      // the 4-wide tree in reference-like layout, and its node count
-    int64_t n_ref4 = 0;
     std::vector<float4> gquad, gsph;
     if (n > 0) {
         static const std::vector<Box> no_boxes;
@@ -1018,8 +1020,10 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
             int brc = rth::gpu_build_binary(bx.data(), raw.v, (int32_t)d->n_tris, tbnd, (int32_t)n, nullptr, nullptr,
                                             nullptr, nullptr, &root, s->sms, s->stream, &W);
             if (brc) return bail(fail(s, RT_ERR_CUDA, std::string("device BVH build: ") + cudaGetErrorString((cudaError_t)brc)));
-            void* owned_ptrs[] = {W.nodes, W.export_ch, W.nodes4};
+            void* owned_ptrs[] = {W.nodes, W.export_ch};
             for (void* p : owned_ptrs) if (p) s->owned.push_back(DevBuf{p, 0});
+            s->ref4 = W.nodes4;
+            s->n_ref4 = W.n_nodes4;
             B.max_depth = W.max_depth;
             if (d->n_tris > 0) {
                 Box t{h3(tbnd[0], tbnd[1], tbnd[2]), h3(tbnd[3], tbnd[4], tbnd[5])};
@@ -1176,8 +1180,6 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
         if ((rc = upload(s, wsh.data(), wsh.size(), &s->S.cvx_shade))) return bail(rc);
         if (dev_wide) {
             s->d_ref_nodes = W.nodes;
-            d_ref4 = W.nodes4;
-            n_ref4 = W.n_nodes4;
         } else if ((rc = upload(s, gnodes.data(), gnodes.size(), &s->d_ref_nodes))) {
             return bail(rc);
         }
@@ -1316,18 +1318,15 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
     if ((rc = upload(s, codes.data(), codes.size(), &s->S.mat_code))) return bail(rc);
     // the node arrays the traversal reads (their leaf references carry the class codes)
     if (n > 0) {
-        float4 *pk = nullptr, *qk = nullptr, *pk4 = nullptr;
-        LeafSet lk{nullptr, nullptr}, lk4{nullptr, nullptr};
+        float4 *pk = nullptr, *qk = nullptr;
+        LeafSet lk{nullptr, nullptr};
         cudaError_t pe = rth::pack_nodes(s->S, s->d_ref_nodes, s->n_nodes, s->n_leaves, 8, &pk, &lk, &qk, s->sms, s->stream);
-        if (pe == cudaSuccess && d_ref4)
-            pe = rth::pack_nodes(s->S, d_ref4, n_ref4, s->n_leaves, 4, &pk4, &lk4, nullptr, s->sms, s->stream);
-        for (const float4* p : {(const float4*)pk, lk.rec, lk.box, (const float4*)qk, (const float4*)pk4, lk4.rec, lk4.box})
+        for (const float4* p : {(const float4*)pk, lk.rec, lk.box, (const float4*)qk})
             if (p) s->owned.push_back(DevBuf{(void*)p, 0});
         if (pe != cudaSuccess) return bail(fail(s, RT_ERR_CUDA, std::string("packing the BVH nodes: ") + cudaGetErrorString(pe)));
-        s->S.nodes = pk; s->S.leaves = lk; s->S.qnodes = qk; s->S.nodes4 = pk4; s->S.leaves4 = lk4;
+        s->S.nodes = pk; s->S.leaves = lk; s->S.qnodes = qk;
         s->S.n_nodes = (uint32_t)s->n_nodes;
         s->qnodes_ok = qk != nullptr;
-        s->wide4_ok = pk4 != nullptr;
     }
     // shading classes the scene can produce: a miss always, a hit's class from
     // its material's code (launches of the other classes' kernels are skipped)
@@ -2571,6 +2570,26 @@ extern "C" int32_t rt_last_render_stats(const RtScene* s, double* ms, int64_t* e
     return RT_OK;
 }
 
+// The packed 4-wide nodes and their leaves (80 B a primitive), made when they are
+// first asked for: most scenes never read them.
+static int ensure_wide4(RtScene* s) {
+    if (!s->ref4) return RT_OK;
+    float4* pk = nullptr;
+    LeafSet lk{nullptr, nullptr};
+    cudaError_t e = rth::pack_nodes(s->S, s->ref4, s->n_ref4, s->n_leaves, 4, &pk, &lk, nullptr, s->sms, s->stream);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(s, e == cudaErrorMemoryAllocation ? RT_ERR_NOMEM : RT_ERR_CUDA,
+                    std::string("packing the 4-wide nodes: ") + cudaGetErrorString(e));
+    }
+    for (const float4* p : {(const float4*)pk, lk.rec, lk.box}) s->owned.push_back(DevBuf{(void*)p, 0});
+    s->S.nodes4 = pk;
+    s->S.leaves4 = lk;
+    cudaFree(s->ref4);
+    s->ref4 = nullptr;
+    return RT_OK;
+}
+
 extern "C" int32_t rt_set_tuning(RtScene* s, const RtTuning* t) {
     if (!s || !t) return RT_ERR_INVALID;
     if (t->max_paths != 0 && (t->max_paths < (1u << 16) || t->max_paths > MAX_PATHS))
@@ -2583,7 +2602,7 @@ extern "C" int32_t rt_set_tuning(RtScene* s, const RtTuning* t) {
         return fail(s, RT_ERR_INVALID, "node_format must be RT_NODES_FULL, RT_NODES_QUANTISED, RT_NODES_WIDE4 or RT_NODES_AUTO");
     if (t->node_format == RT_NODES_QUANTISED && !s->qnodes_ok && !s->empty)
         return fail(s, RT_ERR_INVALID, "the scene's extents exceed the quantised node layout");
-    if (t->node_format == RT_NODES_WIDE4 && !s->wide4_ok && !s->empty)
+    if (t->node_format == RT_NODES_WIDE4 && !s->wide4_ok() && !s->empty)
         return fail(s, RT_ERR_INVALID, "4-wide nodes exist for trees built on the device only");
     if (t->stack_limit != 0 && (int64_t)t->stack_limit > s->stack_cap_built)
         return fail(s, RT_ERR_INVALID, "stack_limit must be 0 or at most " + std::to_string(s->stack_cap_built) +
@@ -2591,6 +2610,8 @@ extern "C" int32_t rt_set_tuning(RtScene* s, const RtTuning* t) {
     if (t->graph > 1) return fail(s, RT_ERR_INVALID, "graph must be 0 or 1");
     ENTER(s);
     CK(cudaStreamSynchronize(s->stream));
+    if (t->node_format == RT_NODES_WIDE4)
+        if (int rc = ensure_wide4(s)) return rc;
     s->max_paths = t->max_paths ? t->max_paths : MAX_PATHS;
     s->S.trace_per_sm = (int)t->trace_blocks_per_sm;
     s->S.shade_per_sm = (int)t->shade_blocks_per_sm;
@@ -2599,7 +2620,7 @@ extern "C" int32_t rt_set_tuning(RtScene* s, const RtTuning* t) {
     s->S.stack_cap = std::min(s->stack_limit ? s->stack_limit : s->stack_cap_built, s->stack_rows);
     s->S.stack_ring = t->stack_ring ? (int)t->stack_ring : RT_SHORT_STACK;
     s->S.node_format = (s->qnodes_ok && t->node_format == RT_NODES_QUANTISED) ? RT_NODES_QUANTISED
-                     : (s->wide4_ok && t->node_format == RT_NODES_WIDE4)    ? RT_NODES_WIDE4
+                     : (s->wide4_ok() && t->node_format == RT_NODES_WIDE4)  ? RT_NODES_WIDE4
                      : t->node_format == RT_NODES_AUTO                      ? RT_NODES_AUTO
                                                                             : RT_NODES_FULL;
     s->graph_mode = t->graph != 0;
