@@ -766,6 +766,7 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
     if (device < 0 || device >= ndev) return bail(fail(s, RT_ERR_INVALID, "device index out of range"));
     s->device = device;
     s->S.node_format = RT_NODES_AUTO;
+    s->S.noise_medium = -1;
     if (cudaSetDevice(device) != cudaSuccess) return bail(fail(s, RT_ERR_CUDA, "cudaSetDevice failed"));
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, device);
@@ -1446,8 +1447,8 @@ int32_t rt_scene_create(const RtSceneDesc* d, int32_t device, RtScene** out) {
         }
         if ((rc = upload(s, dm.data(), dm.size(), &s->S.media))) return bail(rc);
         s->S.n_media = d->n_media;
-    s->S.noise_medium = -1;
-    for (int32_t i = d->n_media - 1; i >= 0; i--) if (d->media[i].type == RT_MEDIUM_NOISE) s->S.noise_medium = i;
+        for (int32_t i = d->n_media - 1; i >= 0; i--)
+            if (d->media[i].type == RT_MEDIUM_NOISE) s->S.noise_medium = i;
     }
 
     std::call_once(g_elut_once, build_elut);
@@ -1964,9 +1965,9 @@ static int run_wavefront(RtScene* s, const WaveBufs& W, const RtCamera* cam, con
     };
     // launches per iteration: extend, classify, shadow, retire (two halves when they overlap), one shading
     // kernel per class the scene's materials produce (the medium class counted
-    // with the media pair), the guide pair and the photon gather's two
+    // with the media's two), the guide pair and the photon gather's two
     const int64_t per_it = (overlap ? 5 : 4) + __builtin_popcount(s->S.class_mask & ~(1u << CLS_MEDIUM)) +
-                           (R.guide.mode != 0 ? 2 : 0) + (s->S.n_media > 0 ? 2 : 0) + (R.photons ? 2 : 0);
+                           (R.guide.mode != 0 ? 2 : 0) + (s->S.n_media > 0 ? 3 : 0) + (R.photons ? 2 : 0);
     auto prologue = [&]() {
         CK(cudaMemsetAsync(W.counters, 0, sizeof(uint32_t) * RT_CTR_WORDS, s->stream));
         mark(0);
