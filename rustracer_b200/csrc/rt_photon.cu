@@ -1281,18 +1281,26 @@ rtph::Map PhotonMapDev::view() const {
 
 namespace rth {
 
-// grow a device array to at least `n` elements of `bytes` (contents not kept)
+// grow a device array to at least `n` elements of `bytes` (contents not kept).  Where
+// several arrays share one capacity it is 0 while they grow: if one of them cannot,
+// the next, smaller request must not find the capacity of arrays that are gone.
 template <class T>
 static cudaError_t grow(T*& p, size_t n, size_t bytes) {
     if (p) cudaFree(p);
     p = nullptr;
-    return cudaMalloc((void**)&p, std::max<size_t>(n, 1) * bytes);
+    cudaError_t e = cudaMalloc((void**)&p, std::max<size_t>(n, 1) * bytes);
+    if (e) {
+        p = nullptr;
+        cudaGetLastError();
+    }
+    return e;
 }
 
 // map arrays (emission-order copy, Morton-ordered copy, sort keys) for n photons
 static cudaError_t ensure_map(PhotonMapDev& map, size_t n) {
-    if (n <= map.cap_map && map.pos) return cudaSuccess;
+    if (n <= map.cap_map) return cudaSuccess;
     size_t c = std::max<size_t>(n, map.cap_map * 5 / 4);
+    map.cap_map = 0;
     cudaError_t e;
     float4** f4[] = {&map.pos, &map.pow, &map.nor, &map.exp_pos, &map.exp_pow, &map.exp_nor, &map.fpos, &map.fpow, &map.fnor};
     for (float4** q : f4) if ((e = grow(*q, c, sizeof(float4)))) return e;
@@ -1368,8 +1376,9 @@ static cudaError_t build_tree(PhotonMapDev& map, uint32_t n, cudaStream_t st) {
     uint32_t nleaf = (n + PH_LEAF - 1) / PH_LEAF, p2 = 1;
     while (p2 < nleaf) p2 <<= 1;
     map.nleaf_pow2 = p2;
-    if ((size_t)(2 * p2 - 1) > map.cap_heap || !map.blo) {
+    if ((size_t)(2 * p2 - 1) > map.cap_heap) {
         size_t c = 2 * (size_t)p2 - 1;
+        map.cap_heap = 0;
         if ((e = grow(map.blo, c, sizeof(float4))) || (e = grow(map.bhi, c, sizeof(float4)))) return e;
         map.cap_heap = c;
     }
@@ -1427,8 +1436,9 @@ cudaError_t photon_build(const DevScene& S, PhotonMapDev& map, const PathState& 
     }
     const uint32_t total = count;          // photons traced by this build (slots 0 .. total − 1)
     cudaError_t e;
-    if (total > map.cap_work || !map.flags) {
+    if (total > map.cap_work) {
         size_t c = std::max<size_t>(total, map.cap_work * 5 / 4);
+        map.cap_work = 0;
         if ((e = grow(map.flags, c, 1)) || (e = grow(map.st_pos, c, sizeof(float4))) ||
             (e = grow(map.st_pow, c, sizeof(float4))) || (e = grow(map.st_nor, c, sizeof(float4))) ||
             (e = grow(map.fl32, c, sizeof(uint32_t))) || (e = grow(map.scan, c, sizeof(uint32_t))))
