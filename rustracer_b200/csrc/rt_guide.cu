@@ -421,8 +421,8 @@ uint64_t splitmix(uint64_t& s) {
 
 namespace rtgh {
 
-constexpr int DL_WORKERS = 8;
-constexpr size_t DL_CHUNK = 2u << 20;
+constexpr int DL_WORKERS = 8, DL_FEWEST = 4;
+constexpr size_t DL_CHUNK = 512u << 10;
 
 struct Guide {
     RtGuideParams prm{};
@@ -582,19 +582,24 @@ int ensure_paths(Guide* g, uint32_t cap) {
 // A device array of tens of megabytes into the caller's pageable memory.  A
 // plain copy goes through the driver's one staging thread and takes a fresh
 // array's page faults one after the other (67 MB gradient: 3.2 ms into memory
-// touched before, 14 ms into a new array; the link alone 1.2 ms).  Here
-// DL_WORKERS threads each copy every eighth chunk through a pinned slot of their
-// own, so the faults and the host copies run beside one another and beside the
-// link (2.5 ms into a new array).  16 MB of pinned memory per guide, released
-// with it.  Pinned or managed destinations, and a host short of pinned memory
-// or threads, take the plain copy.
+// touched before, 14-29 ms into a new array, by the host; the link alone 1.2 ms).
+// Here up to DL_WORKERS threads, no more than the CPUs the process may use, each
+// copy their share of the chunks through a pinned slot of their own, so the faults
+// and the host copies run beside one another and beside the link (16 CPUs, where a
+// plain copy takes 29 ms into a new array and 3.7 into a touched one: 2 threads
+// 13.8 and 4.2 ms, 4 threads 7.9 and 3.0, 8 threads 4.9 and 2.9; chunks of 2 MB 4.8
+// and 2.3).  The slots are pinned at a guide's first download, which a user pays
+// for: 4 MB take 1.6-3.4 ms, the 16 MB of the larger chunks 7-11.  Released with the
+// guide.  Pinned or managed destinations, fewer than DL_FEWEST CPUs, and a host
+// short of pinned memory take the plain copy.
 static cudaError_t download(Guide* g, void* host, const void* dev, size_t bytes, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
     int device = 0;
-    bool ready = pageable && bytes > DL_CHUNK && cudaGetDevice(&device) == cudaSuccess;
+    const int workers = rth::usable_threads(DL_WORKERS);
+    bool ready = pageable && bytes > DL_CHUNK && workers >= DL_FEWEST && cudaGetDevice(&device) == cudaSuccess;
     if (ready && !g->pin) {
         if (cudaHostAlloc((void**)&g->pin, DL_WORKERS * DL_CHUNK, cudaHostAllocDefault) != cudaSuccess) g->pin = nullptr;
         for (auto& ev : g->dl_ev)
@@ -610,7 +615,7 @@ static cudaError_t download(Guide* g, void* host, const void* dev, size_t bytes,
     auto work = [=](int w) -> cudaError_t {
         cudaError_t r = cudaSetDevice(device);
         char* slot = g->pin + w * DL_CHUNK;
-        for (size_t c = w; c < chunks && r == cudaSuccess; c += DL_WORKERS) {
+        for (size_t c = w; c < chunks && r == cudaSuccess; c += workers) {
             const size_t at0 = c * DL_CHUNK, len = std::min(DL_CHUNK, bytes - at0);
             if ((r = cudaMemcpyAsync(slot, (const char*)dev + at0, len, cudaMemcpyDeviceToHost, st))) break;
             if ((r = cudaEventRecord(g->dl_ev[w], st))) break;
@@ -619,8 +624,8 @@ static cudaError_t download(Guide* g, void* host, const void* dev, size_t bytes,
         }
         return r;
     };
-    cudaError_t got[DL_WORKERS];
-    rth::on_threads(DL_WORKERS, [&](int w) { got[w] = work(w); });
+    cudaError_t got[DL_WORKERS] = {};
+    rth::on_threads(workers, [&](int w) { got[w] = work(w); });
     for (cudaError_t r : got) if (e == cudaSuccess) e = r;
     return e;
 }

@@ -3055,8 +3055,8 @@ int guide_api(RtScene* s, const float* q, const float* dirs, const float* u, int
 int stage_samples(RtScene* s, const float* smp, int64_t n, Tmp& t, const float4** d) {
     std::vector<float4> h((size_t)n * 3);
     // two transcendental functions a row: 50 ns, so 65,536 rows took 3.3 ms of a
-    // call whose kernels take 0.4 ms; 8 threads from 2048 rows on
-    const int workers = n < 2048 ? 1 : 8;
+    // call whose kernels take 0.4 ms; up to 8 threads from 2048 rows on
+    const int workers = n < 2048 ? 1 : rth::usable_threads(8);
     rth::on_threads(workers, [&](int w) {
         for (int64_t i = n * w / workers; i < n * (w + 1) / workers; i++) {
             const float* r = smp + i * 13;

@@ -320,9 +320,17 @@ void launch_develop(const float* lin, const float* sum, const uint32_t* cnt, uin
 }  // namespace rth
 
 // host state of the path-guiding network (rt_guide.cu)
+#include <sched.h>
 #include <future>
 #include <string>
 namespace rth {
+// threads worth starting at once: at most `most`, and the CPUs this process may use
+inline int usable_threads(int most) {
+    cpu_set_t set;
+    CPU_ZERO(&set);
+    if (sched_getaffinity(0, sizeof(set), &set) != 0) return 1;
+    return std::max(1, std::min(most, CPU_COUNT(&set)));
+}
 // f(0) … f(n − 1), n ≤ 16, each on a thread of its own where one can be had
 template <typename F>
 void on_threads(int n, F&& f) {
