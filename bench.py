@@ -15,12 +15,13 @@ value    : path samples/s with the scene resident in HBM, device time of each
 e2e      : the same metric through the C ABI with HOST output buffers (the
            accumulated image is read back every step), wall time per step.
 roofline : the closest-hit traversal kernel (extend).  Algorithmic bytes per
-           launch = Σ over that launch's rays of 224 B × 8-wide nodes visited
-           + 36 B × triangle tests + 16 B × sphere tests + 64 B × quad tests, as
-           counted by the CPU oracle's restatement of the reference traversal
-           on rays captured from the GPU's own queues (a subsample per bounce,
-           scaled by the bounce's ray count); divided by the kernel's CUDA-event
-           time; peak = measured HBM copy bandwidth.
+           launch = Σ over that launch's rays of the layout's bytes × 8-wide
+           nodes visited (NODE_BYTES) + 48 B × primitive tests (the leaf record)
+           + 16 B × sphere tests + 64 B × quad tests, as counted by the CPU
+           oracle's restatement of the reference traversal on rays captured from
+           the GPU's own queues (a subsample per bounce, scaled by the bounce's
+           ray count); divided by the kernel's CUDA-event time; peak = measured
+           HBM copy bandwidth.
 cpu_baseline: the CPU oracle (restatement of the reference's CPU path) on a
            bounded sample of the same frame (bands of 32 rows, 1 spp each,
            ~12 s on all host cores).
@@ -52,6 +53,10 @@ DEPTH = 12
 HERO = 4
 METRIC = "path samples/s (1920x1080 icosphere workload)"
 UNIT = "path samples/s"
+# what a visit of one 8-wide node reads, by rt_set_tuning's node_format: full, quantised,
+# 4-wide (two levels of one node each at least); the library's own choice is one of the
+# first two and counted as the smaller
+NODE_BYTES = {0: 208.0, 1: 80.0, 2: 224.0, "auto": 80.0}
 REF_BANDS = 320         # bands of 32 rows per reference-arm step (~2.5 s on 16 cores: 5 steps ≥ 10 s)
 
 
@@ -350,9 +355,9 @@ def roofline(scene, sb, cam, w=W, h=H, spp=SPP, depth=DEPTH, hero=HERO, seed=2, 
     """Roofline of the extend (closest-hit) kernel; see the module docstring.
     The kernel is not HBM-bound: its node and primitive fetches are served
     mostly by L1 and L2, so `frac` (algorithmic bytes per second over the HBM
-    copy peak) measures how fast the cache hierarchy delivers the reference
-    layout's bytes, and `dram_frac` beside it is the DRAM traffic ncu measured
-    for the kernel over the same time."""
+    copy peak) measures how fast the cache hierarchy delivers the layout's
+    bytes, and `dram_frac` beside it is the DRAM traffic ncu measured for the
+    kernel over the same time."""
     from oracle import oracle as O
     from rustracer_b200.renderer import pass_params
     peak, peak_kind = measured_peak()
@@ -364,6 +369,8 @@ def roofline(scene, sb, cam, w=W, h=H, spp=SPP, depth=DEPTH, hero=HERO, seed=2, 
     kt = scene.kernel_times()
     ext_rays = scene.last_stats()["ext_rays"]
     scene.set_profiling(False)
+    tuning = scene.get_tuning()
+    node_bytes = NODE_BYTES["auto" if tuning["node_auto"] else tuning["node_format"]]
     o = O.OracleScene(sb)
     rng = np.random.default_rng(0)
     total_bytes_pass = 0.0
@@ -374,7 +381,8 @@ def roofline(scene, sb, cam, w=W, h=H, spp=SPP, depth=DEPTH, hero=HERO, seed=2, 
             break
         sub = r[rng.choice(len(r), size=min(len(r), 20000), replace=False)]
         stt = o.trace_stats(sub)
-        bpr = (224.0 * stt[:, 0] + 36.0 * stt[:, 1] + 16.0 * stt[:, 2] + 64.0 * stt[:, 3]).mean()
+        # columns: nodes, triangles, spheres, quads
+        bpr = (node_bytes * stt[:, 0] + 48.0 * stt[:, 1:4].sum(1) + 16.0 * stt[:, 2] + 64.0 * stt[:, 3]).mean()
         total_bytes_pass += bpr * len(r)
         per_depth.append((d, len(r), float(bpr), float(stt[:, 0].mean()), float(stt[:, 1].mean())))
     ext_ms, ext_launches = kt["extend"]
@@ -393,7 +401,9 @@ def roofline(scene, sb, cam, w=W, h=H, spp=SPP, depth=DEPTH, hero=HERO, seed=2, 
     launch_s = ext_ms / 1000.0 / max(1, ext_launches)
     dram_gbs = traffic / launch_s / 1e9 if (traffic and launch_s > 0) else None
     return {"kernel": "k_extend (8-wide BVH closest hit)", "bound": "hbm",
-            "limiter": "L1/TEX throughput and load latency (node fetches hit L1/L2), not DRAM bandwidth",
+            "limiter": "issue slots at 13-16 active lanes of 32 and the latency of node fetches (L1/L2), "
+                       "not DRAM bandwidth",
+            "node_bytes": node_bytes,
             "achieved": achieved, "peak": peak,
             "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak if achieved else None,
             "traffic": traffic, "traffic_source": traffic_source, "dram_gbs": dram_gbs,

@@ -792,14 +792,16 @@ __global__ void k_fix_leaf_refs(float4* nodes, int64_t n_nodes, const int32_t* _
     }
 }
 // ── packed nodes: what the traversal reads (rt_trace.cu) ────────────────────
-// From a tree in the reference layout (preorder, child references): every
-// child gets a slot by octant (bit 0, 1, 2 of the slot: the upper side of x, y,
-// z), so a ray finds its children roughly front to back as slot XOR octant
-// without keeping distances; the inner children of a node become neighbours in
-// slot order, so a node index, a slot mask and a population count name a child
-// (a header instead of 8 references), and a visit's pending children are one
-// 8-byte stack entry.  The leaves of a node are neighbours too, in their own
-// copy of the triangle records (for other primitives only the reference), so a
+// From a tree in the reference layout (preorder, child references).  The scheme is
+// that of Ylitie, Karras and Laine 2017 (octant slots, a base index and masks in
+// place of child references); the slot choice, the header and the leaf records are
+// this file's.  Every child gets a slot by octant (bit 0, 1, 2 of the slot: the
+// upper side of x, y, z), so a ray finds its children roughly front to back as
+// slot XOR octant without keeping distances; the inner children of a node become
+// neighbours in slot order, so a node index, a slot mask and a population count
+// name a child (a header instead of 8 references), and a visit's pending children
+// are one 8-byte stack entry.  The leaves of a node are neighbours too, in their
+// own copy of the triangle records (for other primitives only the reference), so a
 // leaf's triangle is found from the header without a reference in between; the
 // leaves' float boxes are a second array.
 //

@@ -132,9 +132,10 @@ struct PendTargets {
 
 namespace rtph { struct Map; }
 
-// Uniform cell grid over the photons' box: cubic cells of at least twice the
-// gather radius (so a gather ball meets at most 2 cells per axis), at most
-// 1024 per axis and RT_PH_GRID_MAX_CELLS in all.
+// Uniform cell grid over the photons' box: cubic cells, at most 1024 per axis and
+// RT_PH_GRID_MAX_CELLS in all.  The query grid's cells are at least twice the gather
+// radius (a gather ball meets at most 2 per axis), the render path's at least the
+// radius (3 per axis).
 #define RT_PH_GRID_MAX_CELLS (1u << 22)
 struct PhotonGrid {
     float lo[3];
@@ -145,7 +146,8 @@ struct PhotonGrid {
 
 // Device photon map: photons sorted by (grid cell, Morton code) — every cell a
 // contiguous run — with the [start, end) table of the cells, a box heap over
-// 32-photon leaves of the same order, and an emission-order copy.  Its arrays
+// 32-photon leaves of the same order, an emission-order copy, and the render
+// path's copy by cell of its finer grid.  Its arrays
 // and the build's work buffers grow on demand and are kept across builds, so a
 // rebuild of a map no larger than before allocates and frees nothing
 // (release() only drops the map).

@@ -2,7 +2,8 @@
 //
 // Compiled with --fmad=false: the reference (Rust) never fuses a*b+c, and the
 // hit ids / t values must be bit-identical to that arithmetic, so no FFMA may
-// appear in the primitive tests.  The slab test is FSUB+FMUL+FMNMX only.
+// appear in the primitive tests and the leaf-box test.  The node tests, which only
+// have to be conservative, use explicit FMAs: one per plane.
 //
 // Traversal (replaces BvhTree::hit_index, src/bvh.rs:229-288, and the AVX2
 // slab test :326-364): one ray per lane in persistent warps; lanes that finish
@@ -11,10 +12,12 @@
 // Per visited node the thread tests all 8 child boxes, intersects the hit leaves
 // at once (closest t, ties → smaller canonical id) and is left with a mask of
 // hit inner children.  The children of a node are neighbours in memory and sit
-// in slots by octant (pack_slots in rt_build.cu), so that mask and the index of
+// in slots by octant (octant_slots in rt_build.cu), so that mask and the index of
 // the first child are the whole to-do list of the visit (a "group", 8 bytes):
 // the next child is the slot nearest along the ray's octant, no distances are
-// kept or sorted, and a visit pushes at most one stack entry.
+// kept or sorted, and a visit pushes at most one stack entry (octant slots and
+// stack entries of a first child and its pending slots: Ylitie, Karras and Laine,
+// Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs, 2017).
 #include <algorithm>
 
 #include <cub/block/block_scan.cuh>
@@ -206,11 +209,11 @@ RT_D uint32_t node_test(const DevScene& S, uint32_t ni, const RayC& R, float tmi
 // its unit 2^8 above the last mantissa bit), with 2^15·S taken off A rounded the
 // same way: that loses at most 2^-8 steps (2^23 + q would lose a whole one), so
 // q·S + A stays on the conservative side but for the last FMA's own rounding,
-// which the widened exit covers: the hits are the brute-force ones.  The kernel
-// is bound by issue here (73 % of the slots, ALU pipe 56 %), so the decode is
-// what counts; packed two-wide FMAs save 14 % of the instructions and lose it
-// again to the register pairs their constants need (spills; icosphere extend
-// 50.2 against 49.7 ms).
+// which the widened exit covers.  The kernel issues in 63 % of the cycles on the
+// first bounce and 54 % later, at 13 to 16 lanes of 32 and 4 long-scoreboard stalls
+// per issue: half instructions, half the wait for the next node.  Packed two-wide
+// FMAs save 14 % of the instructions and lose it again to the register pairs their
+// constants need (spills; icosphere extend 50.2 against 49.7 ms).
 RT_D float qbyte(uint32_t w, uint32_t sel) { return __uint_as_float(__byte_perm(w, 0x47000000u, sel)); }
 
 __device__ __noinline__ uint32_t qnode_test_general(const float4* N, float3 o, float3 inv, float tmin, float tmax);
